@@ -5,72 +5,330 @@
 // C core scalar semantics (rbg_math.c.in:30-121).  (+) is associative and commutative, so the
 // accumulation order does not change C; an OverflowError is raised when any product signals one.
 //
-// One tiled kernel with the full scalar semantics per term (identities, parity filters, wrap,
-// overflow events), 64 x 64 outputs per CTA staged through shared memory.
+// One kernel, 128 x 128 outputs per CTA, the reduction staged through shared memory in chunks of
+// 32 steps.  Operands in the clean regime run on 32-bit lanes (avos.cuh): a product is one
+// multiply-add x * 2^msb(y) + (y - 2^msb(y)), a sum one unsigned min.  Two things are kept out of
+// the inner loop:
+//   - steps of a chunk whose column of A or row of B (within the tile) is all zero are skipped,
+//     as are the steps at which a warp's rows of A are zero (closures are sparse);
+//   - the identities.  A -1 on the left is staged as a lane value that yields the right operand;
+//     1 and -1 on the right (parity filters) are staged as zeros and folded in by a pass of their
+//     own over the chunk's steps that hold one.
+// With dense operands the issue slots bound it (64 multiply-adds and mins per 5 vector loads from
+// shared memory); with a closure times its pedigree most steps are skipped and a chunk's staging
+// latency does: one CTA of 512 threads per SM (the accumulators and the next chunk's values, in
+// flight during a chunk's products, take its registers), one barrier per chunk.  n = 2048, W (x) A
+// of a pedigree: 7.32 ms with the full scalar semantics per product (64 x 64 tiles), 0.36 ms now.
+// A tile in which some product may reach the storage type's top bit, or which holds a negative
+// value other than -1, is redone by the same CTA with the full scalar semantics (wrap, overflow
+// events).
 #include <cuda_runtime.h>
+#include <cooperative_groups.h>
 #include <string.h>
 #include <algorithm>
 #include "rbg_internal.cuh"
 
 namespace rbg {
 
-constexpr int MM_T = 64;        // output tile edge
-constexpr int MM_K = 32;        // reduction chunk
-constexpr int MM_THREADS = 256; // 16 x 16 threads, 4 x 4 outputs each
+namespace cg = cooperative_groups;
+
+constexpr int MM_T = 128;        // output tile edge
+constexpr int MM_K = 32;         // reduction steps per chunk (one per lane of a warp)
+constexpr int MM_THREADS = 512;  // 32 x 16 threads, 4 x 8 outputs each
+constexpr int MM_SPLIT = 8;      // CTAs of a cluster that share one tile's reduction, at most
+constexpr uint32_t MM_NONE = 0xffffffffu;      // lane: zero operand / no product yet
+constexpr uint32_t MM_RED_LEFT = 0x80000001u;  // lane: -1 as the left operand (times 2^s, s >= 1, is 2^s)
+
+struct MmSmem {
+    uint32_t as[2][MM_K][MM_T];   // A's chunk, transposed; 4-row groups swizzled by the step (mm_as)
+    uint32_t bm[2][MM_K][MM_T];   // 2^msb of B's values (0: zero or an identity)
+    uint32_t bl[2][MM_K][MM_T];   // value - 2^msb (MM_NONE with bm 0)
+    uint32_t ident[2][2][MM_K][4];// columns 4 l + c whose value is 1 / -1: bit l of word c
+    uint32_t or_b[2][MM_K];       // OR of the step's values in B (identities as 1)
+    // written by atomics, so three slots in turn: one read, one being written, one cleared
+    uint32_t or_a[3][MM_K];       // OR of the step's values in A
+    uint32_t id_any[3];           // steps that hold an identity in B
+};
+
+// position of row i of step j in MmSmem::as: the transposing stores of a warp (8 steps apart by
+// 4, 4 rows) hit 32 banks, and four consecutive rows stay one 16-byte vector
+__device__ __forceinline__ int mm_as(int j, int i) { return ((((i >> 2) ^ ((j >> 2) & 7)) << 2) | (i & 3)); }
 
 __device__ __forceinline__ void mm_flush_flags(unsigned *dflags, unsigned f) {
     for (int o = 16; o > 0; o >>= 1) f |= __shfl_xor_sync(0xffffffffu, f, o);
     if ((threadIdx.x & 31) == 0 && f) atomicOr(dflags, f);
 }
 
-// Exact kernel: any storage type, full scalar semantics.
+// column of a thread's output c within the tile
+__device__ __forceinline__ int mm_col(int tx, int c) { return (c < 4 ? 0 : 60) + 4 * tx + c; }
+
+constexpr size_t align_up_c(size_t x) { return (x + 15) / 16 * 16; }
+
+// the sum as a minimum: the red one first, "no path" last
+template <typename U> __device__ __forceinline__ U mm_enc(U v) { return v == 0 ? (U)~(U)0 : v == (U)~(U)0 ? (U)0 : v; }
+
+// Four consecutive values of a row from column c (`cols` valid columns); `vec`: the row starts
+// and the leading dimension are aligned for vector loads.
+template <typename T> struct alignas(sizeof(T) * 4 > 16 ? 16 : sizeof(T) * 4) MmVec { T v[4]; };
 template <typename T>
-__global__ void __launch_bounds__(MM_THREADS)
-mm_exact_kernel(int64_t m, int64_t q, int64_t p, const T *__restrict__ A, int64_t lda,
-                const T *__restrict__ B, int64_t ldb, T *__restrict__ C, int64_t ldc,
-                unsigned *dflags) {
-    __shared__ T As[MM_T][MM_K + 1];
-    __shared__ T Bs[MM_K][MM_T + 1];
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    const int64_t i0 = (int64_t)blockIdx.y * MM_T, k0 = (int64_t)blockIdx.x * MM_T;
-    T acc[4][4];
+__device__ __forceinline__ void mm_load4(const T *__restrict__ row, bool live, int64_t c, int64_t cols, bool vec,
+                                         T (&x)[4]) {
+    if (live && vec && c + 4 <= cols) {
+        const MmVec<T> t = *reinterpret_cast<const MmVec<T> *>(row + c);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) x[k] = t.v[k];
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) x[k] = (live && c + k < cols) ? row[c + k] : (T)0;
+    }
+}
+
+// Full scalar semantics for one tile, steps [j0, j1): the outputs of each thread (as in mm_kernel)
+// into `tile`, in the encoding of mm_enc.  Every thread of the CTA calls it; `tile` may overlap
+// the staging buffers.
+template <typename T>
+__device__ __noinline__ void mm_exact_tile(int64_t m, int64_t p, int64_t i0, int64_t k0, int64_t j0, int64_t j1,
+                                           const T *__restrict__ A, int64_t lda, const T *__restrict__ B, int64_t ldb,
+                                           unsigned char *smem, unsigned *dflags) {
+    typedef typename utype<T>::type U;
+    T(*as)[MM_K + 1] = reinterpret_cast<T(*)[MM_K + 1]>(smem);
+    T(*bs)[MM_T + 1] = reinterpret_cast<T(*)[MM_T + 1]>(smem + align_up_c(sizeof(T) * MM_T * (MM_K + 1)));
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    unsigned ev = 0;
+    T acc[4][8];
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][c] = 0;
-    unsigned ev = 0;
-    for (int64_t j0 = 0; j0 < q; j0 += MM_K) {
-        for (int e = threadIdx.x; e < MM_T * MM_K; e += MM_THREADS) {
-            int r = e / MM_K, c = e % MM_K;
-            int64_t gi = i0 + r, gj = j0 + c;
-            As[r][c] = (gi < m && gj < q) ? A[gi * lda + gj] : (T)0;
-            int rr = e / MM_T, cc = e % MM_T;
-            int64_t bj = j0 + rr, bk = k0 + cc;
-            Bs[rr][cc] = (bj < q && bk < p) ? B[bj * ldb + bk] : (T)0;
+        for (int c = 0; c < 8; ++c) acc[r][c] = 0;
+    for (int64_t j = j0; j < j1; j += MM_K) {
+        __syncthreads();
+        for (int e = tid; e < MM_T * MM_K; e += MM_THREADS) {
+            const int r = e / MM_K, c = e % MM_K, rr = e / MM_T, cc = e % MM_T;
+            as[r][c] = (i0 + r < m && j + c < j1) ? A[(i0 + r) * lda + j + c] : (T)0;
+            bs[rr][cc] = (j + rr < j1 && k0 + cc < p) ? B[(j + rr) * ldb + k0 + cc] : (T)0;
         }
         __syncthreads();
-        for (int jj = 0; jj < MM_K; ++jj) {
-            T a[4], b[4];
+        for (int t = 0; t < MM_K; ++t) {
+            T a[4], b[8];
 #pragma unroll
-            for (int r = 0; r < 4; ++r) a[r] = As[ty + 16 * r][jj];
+            for (int r = 0; r < 4; ++r) a[r] = as[4 * ty + r][t];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) b[c] = Bs[jj][tx + 16 * c];
+            for (int c = 0; c < 8; ++c) b[c] = bs[t][mm_col(tx, c)];
 #pragma unroll
             for (int r = 0; r < 4; ++r)
 #pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    acc[r][c] = avos_sum<T>(acc[r][c], (T)avos_product<T>(a[r], b[c], ev));
+                for (int c = 0; c < 8; ++c) acc[r][c] = avos_sum<T>(acc[r][c], (T)avos_product<T>(a[r], b[c], ev));
         }
-        __syncthreads();
     }
+    __syncthreads();
+    U *tile = reinterpret_cast<U *>(smem);
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            int64_t gi = i0 + ty + 16 * r, gk = k0 + tx + 16 * c;
-            if (gi < m && gk < p) C[gi * ldc + gk] = acc[r][c];
-        }
+        for (int c = 0; c < 8; ++c) tile[(4 * ty + r) * MM_T + mm_col(tx, c)] = mm_enc<U>((U)acc[r][c]);
     mm_flush_flags(dflags, ev);
+}
+
+// One 128 x 128 tile of C per cluster of `split` CTAs (1, 2, 4 or 8), each taking an equal part of
+// the reduction's chunks; the parts meet through distributed shared memory.
+template <typename T>
+__global__ void __launch_bounds__(MM_THREADS, 1)
+mm_kernel(int64_t m, int64_t q, int64_t p, const T *__restrict__ A, int64_t lda, const T *__restrict__ B, int64_t ldb,
+          T *__restrict__ C, int64_t ldc, int split, bool vec_a, bool vec_b, bool vec_c, unsigned *dflags) {
+    typedef typename utype<T>::type U;
+    constexpr int LBITS = sizeof(T) >= 4 ? 32 : (int)sizeof(T) * 8;   // a clean product's MSB stays below LBITS - 1
+    extern __shared__ __align__(16) unsigned char mm_smem[];
+    MmSmem &S = *reinterpret_cast<MmSmem *>(mm_smem);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tx = tid & 15, ty = tid >> 4;
+    const int part = (int)(blockIdx.x % split);
+    const int64_t k0 = (int64_t)(blockIdx.x / split) * MM_T, i0 = (int64_t)blockIdx.y * MM_T;
+    const int64_t chunks = (q + MM_K - 1) / MM_K;
+    const int64_t c0 = chunks * part / split, c1 = chunks * (part + 1) / split;
+
+    uint32_t acc[4][8];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 8; ++c) acc[r][c] = MM_NONE;
+    if (tid < 3 * MM_K) (&S.or_a[0][0])[tid] = 0;
+    if (tid < 3) S.id_any[tid] = 0;
+
+    // a thread's part of a chunk: 4 steps of rows ar and ar + 64 of A, 4 columns of steps warp and
+    // warp + 16 of B
+    const int ar = tid >> 3, aj = (tid & 7) * 4;
+    T xa[2][4], xb[2][4];
+    auto fetch = [&](int64_t ch) {
+        const int64_t j = ch * MM_K;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int64_t i = i0 + ar + 64 * h;
+            mm_load4<T>(A + i * lda, i < m, j + aj, q, vec_a, xa[h]);
+            const int64_t jb = j + warp + 16 * h;
+            mm_load4<T>(B + jb * ldb, jb < q, k0 + 4 * lane, p, vec_b, xb[h]);
+        }
+    };
+    if (c0 < c1) fetch(c0);
+    bool dirty = false;
+    int s3 = 0;                              // or_a's slot: chunk number modulo 3
+    __syncthreads();
+    for (int64_t ch = c0; ch < c1; ++ch) {
+        const int buf = (int)((ch - c0) & 1);
+        bool bad = false;                    // a value the lanes cannot hold
+        uint32_t oa[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const T v = xa[h][k];
+                const bool red = v == (T)-1;
+                bad |= !red && ((U)v >> (LBITS - 1)) != 0;
+                oa[k] |= red ? 1u : (uint32_t)(U)v;
+                S.as[buf][aj + k][mm_as(aj + k, ar + 64 * h)] =
+                    red ? MM_RED_LEFT : v == 0 ? MM_NONE : (uint32_t)(U)v;
+            }
+            const int jb = warp + 16 * h;
+            uint32_t ob = 0, mv[4], lv[4];
+            bool some_id = false;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const T v = xb[h][k];
+                const bool id = v == (T)-1 || v == (T)1;
+                some_id |= id;
+                bad |= !id && ((U)v >> (LBITS - 1)) != 0;
+                ob |= id ? 1u : (uint32_t)(U)v;
+                const bool plain = !id && v != 0;
+                mv[k] = plain ? 0x80000000u >> __clz((int)(uint32_t)(U)v) : 0u;
+                lv[k] = plain ? (uint32_t)(U)v ^ mv[k] : MM_NONE;
+            }
+            *reinterpret_cast<uint4 *>(&S.bm[buf][jb][4 * lane]) = make_uint4(mv[0], mv[1], mv[2], mv[3]);
+            *reinterpret_cast<uint4 *>(&S.bl[buf][jb][4 * lane]) = make_uint4(lv[0], lv[1], lv[2], lv[3]);
+            ob = __reduce_or_sync(0xffffffffu, ob);
+            if (lane == 0) S.or_b[buf][jb] = ob;
+            if (__any_sync(0xffffffffu, some_id)) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const unsigned one = __ballot_sync(0xffffffffu, xb[h][k] == (T)1);
+                    const unsigned red = __ballot_sync(0xffffffffu, xb[h][k] == (T)-1);
+                    if (lane == 0) {
+                        S.ident[buf][0][jb][k] = one;
+                        S.ident[buf][1][jb][k] = red;
+                    }
+                }
+                if (lane == 0) atomicOr(&S.id_any[s3], 1u << jb);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {        // lanes l, l + 8, l + 16, l + 24 hold the same steps
+            oa[k] |= __shfl_xor_sync(0xffffffffu, oa[k], 8);
+            oa[k] |= __shfl_xor_sync(0xffffffffu, oa[k], 16);
+            if (lane < 8 && oa[k]) atomicOr(&S.or_a[s3][aj + k], oa[k]);
+        }
+        if (__syncthreads_or(bad)) { dirty = true; break; }
+        if (ch + 1 < c1) fetch(ch + 1);      // in flight during this chunk's products
+        const uint32_t va = S.or_a[s3][lane], vb = S.or_b[buf][lane];
+        const uint32_t idm = S.id_any[s3];
+        // the previous chunk's slots: read before this chunk's barrier, written after the next one
+        if (warp == 0) {
+            const int old = s3 == 0 ? 2 : s3 - 1;
+            S.or_a[old][lane] = 0;
+            if (lane == 0) S.id_any[old] = 0;
+        }
+        const bool live = va != 0 && vb != 0;
+        uint32_t act = __ballot_sync(0xffffffffu, live);
+        const bool risk = live && (31 - __clz((int)va)) + (31 - __clz((int)vb)) >= LBITS - 1;
+        if (__any_sync(0xffffffffu, risk)) { dirty = true; break; }   // the same vote in every warp
+        uint32_t ids = idm & act;
+        while (act) {
+            const int j = __ffs((int)act) - 1;
+            act &= act - 1;
+            const uint4 x4 = *reinterpret_cast<const uint4 *>(&S.as[buf][j][mm_as(j, 4 * ty)]);
+            const uint32_t x[4] = {x4.x, x4.y, x4.z, x4.w};
+            if (!__any_sync(0xffffffffu, (x[0] & x[1] & x[2] & x[3]) != MM_NONE)) continue;
+            const uint4 m0 = *reinterpret_cast<const uint4 *>(&S.bm[buf][j][4 * tx]);
+            const uint4 m1 = *reinterpret_cast<const uint4 *>(&S.bm[buf][j][64 + 4 * tx]);
+            const uint4 l0 = *reinterpret_cast<const uint4 *>(&S.bl[buf][j][4 * tx]);
+            const uint4 l1 = *reinterpret_cast<const uint4 *>(&S.bl[buf][j][64 + 4 * tx]);
+            const uint32_t mm[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+            const uint32_t ll[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int c = 0; c < 8; ++c) acc[r][c] = min(acc[r][c], x[r] * mm[c] + ll[c]);
+        }
+        // identities on the right: 1 keeps an odd left value (and 1), -1 an even one; -1 (x) -1 is
+        // the red one (0 in the encoding, which absorbs)
+        while (ids) {
+            const int j = __ffs((int)ids) - 1;
+            ids &= ids - 1;
+            const uint4 x4 = *reinterpret_cast<const uint4 *>(&S.as[buf][j][mm_as(j, 4 * ty)]);
+            const uint32_t x[4] = {x4.x, x4.y, x4.z, x4.w};
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                const int bit = c < 4 ? tx : 16 + tx;
+                const bool one = (S.ident[buf][0][j][c & 3] >> bit) & 1u, red = (S.ident[buf][1][j][c & 3] >> bit) & 1u;
+                if (!(one || red)) continue;
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    uint32_t v = MM_NONE;
+                    if (x[r] == MM_RED_LEFT) v = red ? 0u : MM_NONE;
+                    else if (x[r] != MM_NONE && (x[r] & 1u) == (one ? 1u : 0u)) v = x[r];
+                    acc[r][c] = min(acc[r][c], v);
+                }
+            }
+        }
+        s3 = s3 == 2 ? 0 : s3 + 1;
+    }
+    // outputs: straight from the registers, or through the tile in shared memory when it was redone
+    // or is shared by a cluster
+    U *tile = reinterpret_cast<U *>(mm_smem);
+    auto dec = [](U e) -> T { return (T)mm_enc<U>(e); };   // the encoding is its own inverse
+    auto lane_enc = [](uint32_t v) -> U { return (v >> 31) ? (U)~(U)0 : (U)v; };
+    if (dirty) {
+        mm_exact_tile<T>(m, p, i0, k0, c0 * MM_K, c1 * MM_K < q ? c1 * MM_K : q, A, lda, B, ldb, mm_smem, dflags);
+    } else if (split > 1) {
+        __syncthreads();                     // the last chunk's reads of the staging buffers
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int c = 0; c < 8; ++c) tile[(4 * ty + r) * MM_T + mm_col(tx, c)] = lane_enc(acc[r][c]);
+    } else {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int64_t gi = i0 + 4 * ty + r;
+            if (gi >= m) break;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int64_t gk = k0 + 64 * h + 4 * tx;
+                MmVec<T> o;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) o.v[c] = dec(lane_enc(acc[r][4 * h + c]));
+                if (vec_c && gk + 4 <= p) {
+                    *reinterpret_cast<MmVec<T> *>(C + gi * ldc + gk) = o;
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        if (gk + c < p) C[gi * ldc + gk + c] = o.v[c];
+                }
+            }
+        }
+        return;
+    }
+    if (split > 1) cg::this_cluster().sync();
+    else __syncthreads();
+    const int rows = MM_T / split;
+    for (int e = tid; e < rows * MM_T; e += MM_THREADS) {
+        const int at = part * rows * MM_T + e;
+        U v = (U)~(U)0;
+        if (split > 1) {
+            for (int s = 0; s < split; ++s) v = min(v, cg::this_cluster().map_shared_rank(tile, s)[at]);
+        } else {
+            v = tile[at];
+        }
+        const int64_t gi = i0 + at / MM_T, gk = k0 + at % MM_T;
+        if (gi < m && gk < p) C[gi * ldc + gk] = dec(v);
+    }
+    if (split > 1) cg::this_cluster().sync();   // no CTA leaves while its tile is read
 }
 
 template <typename T>
@@ -81,10 +339,35 @@ static int matmul_t(int64_t m, int64_t q, int64_t p, const T *A, int64_t lda, co
         RBG_CUDA_TRY(cudaMemset2DAsync(C, ldc * sizeof(T), 0, p * sizeof(T), m, s));
         return RBG_OK;
     }
-    dim3 grid((unsigned)((p + MM_T - 1) / MM_T), (unsigned)((m + MM_T - 1) / MM_T));
+    constexpr size_t smem = std::max(sizeof(MmSmem), sizeof(T) * MM_T * MM_T);
+    static PerDeviceOnce once;               // per storage type, for every device
+    const int configured = once.run([] {
+        RBG_CUDA_TRY(cudaFuncSetAttribute(mm_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        return (int)RBG_OK;
+    });
+    if (configured) return configured;
+    const int64_t tx = (p + MM_T - 1) / MM_T, ty = (m + MM_T - 1) / MM_T, chunks = (q + MM_K - 1) / MM_K;
+    // too few tiles for the SMs: clusters share a tile's reduction, down to two chunks per CTA
+    // (135 x 655 x 17: 564 us with one CTA per 64 x 64 tile, 68 us; 300 x 310 x 290: 307 us, 94 us)
+    int split = 1;
+    while (split < MM_SPLIT && tx * ty * split * 2 <= sm_count() && chunks >= 4 * split) split *= 2;
+    auto vec = [](const void *ptr, int64_t ld) {
+        return (uintptr_t)ptr % alignof(MmVec<T>) == 0 && (ld * (int64_t)sizeof(T)) % (int64_t)alignof(MmVec<T>) == 0;
+    };
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(tx * split), (unsigned)ty);
+    cfg.blockDim = dim3(MM_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)split;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
     note_launches(1);
-    mm_exact_kernel<T><<<grid, MM_THREADS, 0, s>>>(m, q, p, A, lda, B, ldb, C, ldc, dflags);
-    RBG_CUDA_TRY(cudaGetLastError());
+    RBG_CUDA_TRY(cudaLaunchKernelEx(&cfg, mm_kernel<T>, m, q, p, A, lda, B, ldb, C, ldc, split, vec(A, lda),
+                                    vec(B, ldb), vec(C, ldc), dflags));
     return RBG_OK;
 }
 

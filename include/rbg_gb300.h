@@ -117,7 +117,7 @@ int32_t rbg_profile_end(double *ms, int64_t *launches);
 
 /* rbg_profile_end for the first `slots` (1..9) timer slots: 0-3 as above, then the DAG path of
  * rbg_fw_batch / rbg_fw_dense: 4 scan, 5 closure by levels (with its CSR), 6 statistics, 7 write,
- * 8 the replay of matrices in any numbering (pattern, triples, replay). */
+ * 8 the searches of matrices in any numbering. */
 int32_t rbg_profile_end_slots(double *ms, int64_t *launches, int32_t slots);
 
 /* Scratch bytes rbg_fw_dense needs for an n x n matrix of `dtype` under `mode`. */
@@ -186,12 +186,12 @@ int32_t rbg_fw_batch(int32_t dtype, int64_t count, const int64_t *sizes, const i
  * off-diagonal entry below, or every one above, the diagonal) the sequential loop's step k only
  * pushes row k into the rows of k's children (below) or pulls k's parents into the rows that
  * reach k (above), so the values are the DAG recurrence's and the diameter comes from each
- * cell's first product in step order.  In any other numbering the loop is replayed on the
- * closure's pattern (the triples (i, k, j) of each step with both cells in the pattern), which
- * gives the same diameter and overflow decision.  A matrix whose loop computes a product
+ * cell's first product in step order.  In any other numbering two searches from
+ * every vertex k, through the vertices below k, give the products of the loop's step k, hence the
+ * same diameter and overflow decision.  A matrix whose loop computes a product
  * reaching bit 31 continues without the 32-bit lanes: on 64-bit lanes (int64) or on the exact
  * kernel (int32).  The path's scratch (row slots, the candidates' CSR, the closure's row pool,
- * the replay's pattern and triples) is carved from `workspace`; a closure that does not fit
+ * the searches' cells) is carved from `workspace`; a closure that does not fit
  * leaves its matrices to the blocked kernels.  Every accept / reject decision is made on the
  * device and the results are read back once per call.
  */

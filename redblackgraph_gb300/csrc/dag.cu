@@ -1028,11 +1028,12 @@ size_t dag_workspace_for(int64_t n, int64_t nnz_bound) { return dag_layout(n, nn
 
 int dag_enqueue(const rbg_csr_t *A, int64_t nnz_bound, void *workspace, int32_t *pool_cols, int32_t *pool_vals,
                 int64_t pool_capacity, int64_t *row_off, int32_t *row_len, cudaStream_t s, bool captured,
-                DagCounters **counters, int64_t *launches) {
+                DagCounters **counters, DagChildren *kids, int64_t *launches) {
     const int64_t n = A->n_rows;
     DagWs w;
     dag_layout(n, nnz_bound, reinterpret_cast<unsigned char *>(workspace), &w);
     *counters = w.cnt;
+    if (kids) *kids = DagChildren{w.coff, w.children};
     int rc = dag_configure();
     if (rc) return rc;
     const DagArgs a = dag_args(n, A, w, pool_cols, pool_vals, pool_capacity, row_off, row_len);
@@ -1073,7 +1074,7 @@ extern "C" int32_t rbg_dag_closure(const rbg_csr_t *A, void *workspace, int64_t 
     DagCounters *dc = nullptr;
     int64_t launched = 0;
     int rc = dag_enqueue(A, annz, workspace, pool_cols, pool_vals, pool_capacity, row_off, row_len, s, false, &dc,
-                         &launched);
+                         nullptr, &launched);
     if (rc) return rc;
     DagCounters c;
     {

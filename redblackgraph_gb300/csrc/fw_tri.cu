@@ -25,15 +25,15 @@
 // (TRI_TOP_BIT): its caller skips the 32-bit lanes, which could only report that risk.
 //
 // A matrix with entries on both sides of the diagonal (an acyclic graph in any numbering) has the
-// same closure values, but which product reaches a cell first depends on the numbering: its
-// sequential loop is replayed on the closure's pattern (the triples (i, k, j) with (i, k) and
-// (k, j) in the pattern, step by step), which gives the exact product MSBs and first values.  A
+// same closure values, but which product reaches a cell first depends on the numbering: two searches
+// from every vertex k through the vertices below k give step k's products, hence the exact product
+// MSBs and first values.  A
 // vertex the closure by levels never places (a cycle, or below one) sends its matrix on.
 //
 // Pipeline (one call, every decision on the device): scan the dense rows (clean-regime test,
 // which side of the diagonal, up to TRI_CAP off-diagonal entries per row) -> CSR of the
 // candidate matrices with batch-global row numbers -> closure by levels -> for matrices in any
-// numbering, the transposed pattern, the steps' triples and the replay -> per-row statistics
+// numbering, the searches from every vertex -> per-row statistics
 // (largest product MSB, largest first-value MSB) -> the dense rows of the accepted matrices
 // written from the closure rows -> one result record per matrix, read back once.  Scratch is
 // carved from the caller's workspace; with RBG_MODE_GRAPH the sequence, level loop included (a
@@ -312,19 +312,33 @@ tri_stats_kernel(int64_t R, const int32_t *__restrict__ row_comp, const int32_t 
 
 
 // ------------------------------------------------------------------------------------------
-// Matrices in any numbering (entries on both sides of the diagonal): the sequential loop
-// replayed on the closure's pattern.
+// Matrices in any numbering (entries on both sides of the diagonal)
 // ------------------------------------------------------------------------------------------
-// Before step k of the loop, W(i, k) and W(k, j) hold the values of paths whose intermediate
-// vertices are all below k, and every cell the loop ever fills lies in the closure's pattern C
-// (in the clean regime a cell never returns to zero).  Step k therefore touches only the triples
-// (i, k, j) with (i, k) and (k, j) in C (the pattern holds no diagonal, and i != j in a DAG); a
-// triple performs a product when both cells are non-zero at that time.  No triple of a step
-// writes a cell another triple of the step reads ((i, j) = (i', k) would need j = k), so a step's
-// triples run in parallel and the steps in order.  The replay keeps each cell's current value
-// and the largest MSB of the products it performs (an overflow risk sends the matrix to the
-// blocked kernels) and of the first value each cell receives (the diameter); the values the
-// loop ends with are the closure's, which the closure by levels already holds.
+// Before step k of the loop, W(i, j) holds the smallest value of the paths from i to j whose
+// intermediate vertices are all below k.  In the clean regime msb(x (x) y) = msb(x) + msb(y) and
+// the sum is a minimum, so the MSB of W(i, j) is the shortest such path, the MSB of an edge being
+// its length.  Step k performs exactly the products (i, k, j) with i in In(k) and j in Out(k):
+// the vertices that reach k, and those k reaches, through intermediates below k.  Hence
+//   - the largest product MSB of step k is max over In(k) + max over Out(k) of those lengths;
+//   - a cell without an entry of A gets its first value at the smallest k with i in In(k) and j in
+//     Out(k), and that value's MSB is the two lengths' sum (the diameter's source);
+//   - the number of products is the sum over k of |In(k)| |Out(k)|.
+// Every k is searched on its own (no step waits for another), by the two searches from k along the
+// edges and against them; In(k) and Out(k) are disjoint in a DAG, so they share a table.
+//
+// A warp per k.  The vertices reached live in a table of TRI_TAB words in shared memory, (local
+// vertex << 8 | length), and in a list of table slots in the order of discovery, which is the
+// search's queue.  A vertex shortened after it was taken from the queue sends the list through
+// once more.  Searches that reach more vertices than the list holds go to a second launch (DENSE)
+// whose table has a word per vertex of the largest matrix.  Latency bound (a search is a few
+// dependent loads per length).  Replaying the loop in step order instead, one warp per matrix
+// walking its chain of non-empty steps, took 665 us of the 1,226 us of a renumbered n = 3001
+// pedigree's closure; with the searches the closure takes 541 us (n = 8191: 2,730 us to 656 us).
+constexpr int TRI_TAB = 512;                 // table words of a warp's search
+constexpr int TRI_LIST = 320;                // vertices it may reach before it goes to the dense one
+constexpr int TRI_SEARCH_WARPS = 8;          // warps per CTA (table searches)
+constexpr uint32_t TRI_EMPTY = 0xffffffffu;
+constexpr int TRI_FAR = 126;                 // lengths are capped (a product of MSB 31 is already a risk)
 
 // position of column c in the sorted closure row [o, o + len), or -1
 __device__ __forceinline__ int64_t tri_find_col(const int32_t *__restrict__ p_col, int64_t o, int len, int32_t c) {
@@ -339,17 +353,15 @@ __device__ __forceinline__ int64_t tri_find_col(const int32_t *__restrict__ p_co
     return -1;
 }
 
-__device__ __forceinline__ bool tri_gen_row(int ci, const int32_t *ckind, const unsigned *cbad, const DagCounters *dc,
-                                            const unsigned *gflags) {
-    return ckind[ci] == KIND_GENERAL && !cbad[ci] && tri_dag_ok(dc) && !*gflags;
-}
-
-// One warp per candidate row: a row never placed by the closure by levels (on or below a cycle)
-// marks its matrix; the general matrices' closure rows count their columns.
-__global__ void tri_gen_count_kernel(int64_t R, const int32_t *__restrict__ row_comp, const int32_t *__restrict__ ckind,
-                                     const int64_t *__restrict__ row_off, const int32_t *__restrict__ row_len,
-                                     const int32_t *__restrict__ p_col, const DagCounters *dc, const unsigned *any_gen,
-                                     unsigned *__restrict__ cbad, int64_t *__restrict__ ccnt) {
+// One warp per candidate row of a general matrix: a row never placed by the closure by levels (on
+// or below a cycle) marks its matrix; the cells of A's entries start with key 0 (their first value
+// is A's), the other cells empty.  Cell q of the row is cell[row_off + q].
+__global__ void tri_gen_init_kernel(int64_t R, const int32_t *__restrict__ row_comp, const int32_t *__restrict__ ckind,
+                                    const int64_t *__restrict__ indptr, const int32_t *__restrict__ a_col,
+                                    const int32_t *__restrict__ a_val, const int64_t *__restrict__ row_off,
+                                    const int32_t *__restrict__ row_len, const int32_t *__restrict__ p_col,
+                                    const DagCounters *dc, const unsigned *any_gen, unsigned *gflags,
+                                    unsigned *__restrict__ cbad, uint32_t *__restrict__ cell) {
     if (!tri_dag_ok(dc) || !*any_gen) return;
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -362,20 +374,204 @@ __global__ void tri_gen_count_kernel(int64_t R, const int32_t *__restrict__ row_
             continue;
         }
         const int64_t o = row_off[g];
-        for (int q = lane; q < len; q += 32)
-            atomicAdd(reinterpret_cast<unsigned long long *>(ccnt + p_col[o + q]), 1ull);
+        for (int q = lane; q < len; q += 32) cell[o + q] = TRI_EMPTY;
+        __syncwarp();
+        for (int64_t e = indptr[g] + lane; e < indptr[g + 1]; e += 32) {
+            const int64_t q = tri_find_col(p_col, o, len, a_col[e]);
+            if (q < 0) atomicOr(gflags, 2u);
+            else cell[q] = (uint32_t)msb_u32((uint32_t)a_val[e]);   // a clean value: 2 <= v < 2^31
+        }
     }
 }
 
-// The general matrices' closure pattern transposed: per column, the rows holding it and the pool
-// position of each entry (in any order).
-__global__ void tri_gen_csc_kernel(int64_t R, const int32_t *__restrict__ row_comp, const int32_t *__restrict__ ckind,
-                                   const unsigned *__restrict__ cbad, const int64_t *__restrict__ row_off,
-                                   const int32_t *__restrict__ row_len, const int32_t *__restrict__ p_col,
-                                   const DagCounters *dc, const unsigned *any_gen, const int64_t *__restrict__ cptr,
-                                   int32_t *__restrict__ ccur, int32_t *__restrict__ csc_row,
-                                   int32_t *__restrict__ csc_pos, int64_t cap, unsigned *gflags) {
-    if (!tri_dag_ok(dc) || !*any_gen) return;
+struct TriGraphView {                        // the candidates' graph, rows and columns batch-global
+    const int64_t *indptr;
+    const int32_t *a_col, *a_val;
+    const int64_t *coff;                     // children of a vertex (any order): edges child -> vertex
+    const int32_t *children;
+};
+
+// The table of a warp's search.  put() lowers vertex v's length to d and tells whether v is new
+// (`at`: where) or was shortened; the list holds `at`s.
+template <bool DENSE> struct TriTable {
+    uint32_t *word;
+    __device__ __forceinline__ int vertex(int at) const { return DENSE ? at : (int)(word[at] >> 8); }
+    __device__ __forceinline__ int length(int at) const { return (int)(word[at] & 0xffu); }
+    __device__ __forceinline__ int put(int v, int d, int &at) {   // 1: new, 2: shortened, 0: neither
+        const uint32_t w = ((uint32_t)v << 8) | (uint32_t)d;
+        if (DENSE) {
+            at = v;
+            const uint32_t old = atomicMin(&word[v], w);
+            return old == TRI_EMPTY ? 1 : old > w ? 2 : 0;
+        }
+        int h = (int)(((uint32_t)v * 2654435761u) >> 16) & (TRI_TAB - 1);
+        while (true) {                       // the list is shorter than the table: a slot is free
+            uint32_t cur = *(volatile uint32_t *)&word[h];
+            if (cur == TRI_EMPTY) {
+                cur = atomicCAS(&word[h], TRI_EMPTY, w);
+                if (cur == TRI_EMPTY) { at = h; return 1; }
+            }
+            if ((int)(cur >> 8) == v) {
+                at = h;
+                return atomicMin(&word[h], w) > w ? 2 : 0;
+            }
+            h = (h + 1) & (TRI_TAB - 1);
+        }
+    }
+};
+
+// One search from vertex k (local number) through intermediates below k, along the edges (FWD) or
+// against them; the vertices reached are list[n0, n1).  Returns n1, or -1 when the list is full.
+template <bool DENSE, bool FWD>
+__device__ __forceinline__ int tri_search(const TriGraphView &G, TriTable<DENSE> &T, volatile uint16_t *list, int cap,
+                                          int n0, int k, int64_t base, int lane) {
+    int n1 = n0, h = n0 - 1;                 // position n0 - 1 stands for k itself
+    bool again = false;
+    while (true) {
+        if (h >= n1) {                       // the end of the list: done, or once more from its start
+            if (!again) return n1;
+            again = false;
+            h = n0;
+        }
+        // up to 32 vertices of the queue, their edges flattened over the warp
+        const int left = h < n0 ? 1 : min(32, n1 - h);
+        int x = -1, dx = 0, cnt = 0;
+        int64_t e0 = 0;
+        if (lane < left) {
+            if (h < n0) {
+                x = k;
+            } else {
+                const int at = list[h + lane];
+                const int v = T.vertex(at);
+                dx = T.length(at);
+                x = v < k ? v : -1;          // a vertex above k is an end, never an intermediate
+            }
+            if (x >= 0) {
+                const int64_t *ptr = FWD ? G.indptr : G.coff;
+                e0 = ptr[base + x];
+                cnt = (int)(ptr[base + x + 1] - e0);
+            }
+        }
+        h += left;
+        int incl = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+        }
+        const int excl = incl - cnt;
+        const int total = __shfl_sync(0xffffffffu, incl, 31);
+        for (int b = 0; b < total; b += 32) {
+            const int idx = b + lane;
+            int lo = 0;
+#pragma unroll
+            for (int st = 16; st > 0; st >>= 1) {
+                const int v = __shfl_sync(0xffffffffu, excl, lo + st);
+                if (v <= idx) lo += st;
+            }
+            const int64_t eq = __shfl_sync(0xffffffffu, e0, lo) + (idx - __shfl_sync(0xffffffffu, excl, lo));
+            const int xq = __shfl_sync(0xffffffffu, x, lo), dq = __shfl_sync(0xffffffffu, dx, lo);
+            // a full list would leave no free slot in the table: stop before it can
+            if (n1 + 32 > cap) return -1;    // warp-uniform
+            int got = 0, at = 0;
+            if (idx < total) {
+                int y, len = 0;
+                if (FWD) {
+                    y = G.a_col[eq] - (int)base;
+                    len = msb_u32((uint32_t)G.a_val[eq]);
+                } else {
+                    const int32_t c = G.children[eq];
+                    y = c - (int)base;
+                    const int32_t want = (int32_t)(base + xq);   // the edge's value, in the child's row
+                    for (int64_t e = G.indptr[c]; e < G.indptr[c + 1]; ++e)
+                        if (G.a_col[e] == want) len = msb_u32((uint32_t)G.a_val[e]);
+                }
+                got = T.put(y, min(dq + len, TRI_FAR), at);
+            }
+            const unsigned fresh = __ballot_sync(0xffffffffu, got == 1);
+            if (got == 1) list[n1 + __popc(fresh & ((1u << lane) - 1u))] = (uint16_t)at;
+            n1 += __popc(fresh);
+            again |= __any_sync(0xffffffffu, got == 2);
+            __syncwarp();
+        }
+    }
+}
+
+// The searches of every vertex k of the general matrices, the statistics of step k, and the key
+// (k + 1, product MSB) offered to each cell (i, j) of In(k) x Out(k): a cell keeps its smallest.
+// The table searches walk all rows and leave the ones that outgrow the list to `ovf`, which the
+// dense ones then walk (tables of `words` words and lists per warp in dynamic shared memory).
+template <bool DENSE>
+__global__ void __launch_bounds__(DENSE ? 32 : 32 * TRI_SEARCH_WARPS)
+tri_gen_search_kernel(int64_t R, const int32_t *__restrict__ row_comp, const int32_t *__restrict__ ckind,
+                      const unsigned *__restrict__ cbad, const TriComp *__restrict__ comps, TriGraphView G,
+                      const int64_t *__restrict__ row_off, const int32_t *__restrict__ row_len,
+                      const int32_t *__restrict__ p_col, const DagCounters *dc, const unsigned *any_gen,
+                      unsigned *gflags, uint32_t *__restrict__ cell, int32_t *__restrict__ ovf, int words,
+                      int *__restrict__ cam, unsigned long long *__restrict__ cprod) {
+    if (!tri_dag_ok(dc) || !*any_gen || *gflags) return;
+    extern __shared__ __align__(16) unsigned char tri_search_smem[];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int tab = DENSE ? words : TRI_TAB, cap = DENSE ? words + 32 : TRI_LIST;
+    unsigned char *mine = tri_search_smem + (size_t)w * ((size_t)tab * 4 + (size_t)cap * 2);
+    TriTable<DENSE> T{reinterpret_cast<uint32_t *>(mine)};
+    volatile uint16_t *list = reinterpret_cast<uint16_t *>(mine + (size_t)tab * 4);
+    for (int q = lane; q < tab; q += 32) T.word[q] = TRI_EMPTY;
+    __syncwarp();
+    const int64_t todo = DENSE ? (int64_t)ovf[0] : R;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    for (int64_t t = (int64_t)blockIdx.x * (blockDim.x >> 5) + w; t < todo; t += warps) {
+        const int64_t g = DENSE ? (int64_t)ovf[1 + t] : t;
+        const int ci = row_comp[g];
+        if (ckind[ci] != KIND_GENERAL || cbad[ci]) continue;   // warp-uniform
+        const int64_t base = comps[ci].row_base;
+        const int k = (int)(g - base);
+        // a vertex without parents or without children is on no product
+        if (G.indptr[g + 1] == G.indptr[g] || G.coff[g + 1] == G.coff[g]) continue;
+        const int no = tri_search<DENSE, true>(G, T, list, cap, 0, k, base, lane);
+        const int used = no < 0 ? no : tri_search<DENSE, false>(G, T, list, cap, no, k, base, lane);
+        const int ni = used - no;
+        if (used < 0) {                        // (a dense list holds every vertex)
+            if (lane == 0) {
+                if (DENSE) atomicOr(gflags, 2u);
+                else ovf[1 + atomicAdd(ovf, 1)] = (int32_t)g;
+            }
+        } else {                             // both are non-empty
+            int mo = 0, mi = 0;
+            for (int q = lane; q < no; q += 32) mo = max(mo, T.length(list[q]));
+            for (int q = lane; q < ni; q += 32) mi = max(mi, T.length(list[no + q]));
+            mo = __reduce_max_sync(0xffffffffu, mo);
+            mi = __reduce_max_sync(0xffffffffu, mi);
+            const int64_t pairs = (int64_t)no * ni;
+            if (lane == 0) {
+                atomicMax(cam + ci, mo + mi);
+                atomicAdd(cprod + ci, (unsigned long long)pairs);
+            }
+            for (int64_t q = lane; q < pairs; q += 32) {
+                const int a = (int)(q / no), b = (int)(q - (int64_t)a * no);
+                const int ai = list[no + a], bj = list[b];
+                const int64_t i = base + T.vertex(ai);
+                const int64_t at = tri_find_col(p_col, row_off[i], row_len[i], (int32_t)(base + T.vertex(bj)));
+                if (at < 0) atomicOr(gflags, 2u);
+                else atomicMin(cell + at, ((uint32_t)(k + 1) << 8) | (uint32_t)(T.length(ai) + T.length(bj)));
+            }
+        }
+        __syncwarp();
+        if (used < 0) {                      // the list lacks some of the slots in use
+            for (int q = lane; q < tab; q += 32) T.word[q] = TRI_EMPTY;
+        } else {
+            for (int q = lane; q < used; q += 32) T.word[list[q]] = TRI_EMPTY;
+        }
+        __syncwarp();
+    }
+}
+
+// The largest first value of each general matrix, over its cells.
+__global__ void tri_gen_first_kernel(int64_t R, const int32_t *__restrict__ row_comp, const int32_t *__restrict__ ckind,
+                                     const unsigned *__restrict__ cbad, const int64_t *__restrict__ row_off,
+                                     const int32_t *__restrict__ row_len, const DagCounters *dc, const unsigned *any_gen,
+                                     unsigned *gflags, const uint32_t *__restrict__ cell, int *__restrict__ cfm) {
+    if (!tri_dag_ok(dc) || !*any_gen || *gflags) return;
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
     for (int64_t g = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); g < R; g += warps) {
@@ -383,240 +579,32 @@ __global__ void tri_gen_csc_kernel(int64_t R, const int32_t *__restrict__ row_co
         if (ckind[ci] != KIND_GENERAL || cbad[ci]) continue;   // warp-uniform
         const int64_t o = row_off[g];
         const int len = row_len[g];
-        for (int q = lane; q < len; q += 32) {
-            const int32_t c = p_col[o + q];
-            const int64_t at = cptr[c] + atomicAdd(ccur + c, 1);
-            if (at < cap) {
-                csc_row[at] = (int32_t)g;
-                csc_pos[at] = (int32_t)(o + q);
-            } else {
-                atomicOr(gflags, 1u);
-            }
-        }
-    }
-}
-
-// Triples of step k (batch-global vertex g): column g's entries times row g's entries.
-// Also the pattern length of every general row (lcnt), whose exclusive scan lays each general
-// matrix's current values out contiguously, row after row.
-__global__ void tri_gen_tcount_kernel(int64_t R, const int32_t *__restrict__ row_comp, const int32_t *__restrict__ ckind,
-                                      const unsigned *__restrict__ cbad, const int32_t *__restrict__ row_len,
-                                      const int64_t *__restrict__ cptr, const DagCounters *dc, const unsigned *any_gen,
-                                      const unsigned *gflags, int64_t *__restrict__ tcnt, int64_t *__restrict__ lcnt) {
-    const bool on = tri_dag_ok(dc) && *any_gen && !*gflags;
-    for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g <= R; g += (int64_t)gridDim.x * blockDim.x) {
-        int64_t c = 0, l = 0;
-        if (on && g < R) {
-            const int ci = row_comp[g];
-            if (ckind[ci] == KIND_GENERAL && !cbad[ci]) {
-                c = (cptr[g + 1] - cptr[g]) * (int64_t)row_len[g];
-                l = row_len[g];
-            }
-        }
-        tcnt[g] = c;
-        lcnt[g] = l;
-    }
-}
-
-// One warp per vertex k of a general matrix: its step's triples, as positions of (i, k), (k, j)
-// and (i, j) among the matrix's current values (row g's entry q at lpos[g] - lpos[first row] + q).
-__global__ void tri_gen_fill_kernel(int64_t R, const int32_t *__restrict__ row_comp, const int32_t *__restrict__ ckind,
-                                    const unsigned *__restrict__ cbad, const TriComp *__restrict__ comps,
-                                    const int64_t *__restrict__ row_off, const int32_t *__restrict__ row_len,
-                                    const int32_t *__restrict__ p_col, const int64_t *__restrict__ cptr,
-                                    const int32_t *__restrict__ csc_row, const int32_t *__restrict__ csc_pos,
-                                    const int64_t *__restrict__ tpos, const int64_t *__restrict__ lpos,
-                                    const DagCounters *dc, const unsigned *any_gen, int4 *__restrict__ trip,
-                                    int64_t cap, unsigned *gflags) {
-    if (!tri_dag_ok(dc) || !*any_gen || *gflags) return;
-    const int lane = threadIdx.x & 31;
-    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t k = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); k < R; k += warps) {
-        const int ci = row_comp[k];
-        if (ckind[ci] != KIND_GENERAL || cbad[ci]) continue;   // warp-uniform
-        const int64_t m0 = lpos[comps[ci].row_base];
-        const int64_t c0 = cptr[k], r0 = row_off[k], base = tpos[k], lk = lpos[k] - m0;
-        const int cn = (int)(cptr[k + 1] - c0), rn = row_len[k];
-        const int64_t total = (int64_t)cn * rn;
-        if (base + total > cap) {
-            if (lane == 0 && total) atomicOr(gflags, 1u);
-            continue;
-        }
-        for (int64_t t = lane; t < total; t += 32) {
-            const int a = (int)(t / rn), b = (int)(t - (int64_t)a * rn);
-            const int32_t i = csc_row[c0 + a];
-            const int64_t oi = row_off[i], li = lpos[i] - m0;
-            const int64_t qc = tri_find_col(p_col, oi, row_len[i], p_col[r0 + b]);
-            if (qc < 0) {
-                atomicOr(gflags, 2u);
-                continue;
-            }
-            trip[base + t] = make_int4((int32_t)(li + (csc_pos[c0 + a] - oi)), (int32_t)(lk + b),
-                                       (int32_t)(li + (qc - oi)), (int32_t)k);
-        }
-    }
-}
-
-// One warp per row of a general matrix: the current MSBs (row g's at lpos[g]) start as those of
-// A's entries, zero (no value) elsewhere in the pattern; A's largest MSB starts the first-value
-// maximum.
-__global__ void tri_gen_init_kernel(int64_t R, const int32_t *__restrict__ row_comp, const int32_t *__restrict__ ckind,
-                                    const unsigned *__restrict__ cbad, const int64_t *__restrict__ indptr,
-                                    const int32_t *__restrict__ a_col, const int32_t *__restrict__ a_val,
-                                    const int64_t *__restrict__ row_off, const int32_t *__restrict__ row_len,
-                                    const int32_t *__restrict__ p_col, const int64_t *__restrict__ lpos,
-                                    const DagCounters *dc, const unsigned *any_gen, unsigned *gflags,
-                                    uint8_t *__restrict__ cur, int *__restrict__ cfm) {
-    if (!tri_dag_ok(dc) || !*any_gen || *gflags) return;
-    const int lane = threadIdx.x & 31;
-    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t g = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); g < R; g += warps) {
-        const int ci = row_comp[g];
-        if (ckind[ci] != KIND_GENERAL || cbad[ci]) continue;   // warp-uniform
-        const int64_t o = row_off[g], l = lpos[g];
-        const int len = row_len[g];
-        for (int q = lane; q < len; q += 32) cur[l + q] = 0;
-        __syncwarp();
         int fm = -1;
-        for (int64_t e = indptr[g] + lane; e < indptr[g + 1]; e += 32) {
-            const int64_t q = tri_find_col(p_col, o, len, a_col[e]);
-            if (q < 0) {
-                atomicOr(gflags, 2u);
-                continue;
-            }
-            cur[l + (q - o)] = (uint8_t)msb_u32((uint32_t)a_val[e]);   // a clean value: 2 <= v < 2^31
-            fm = max(fm, dag_row_msb(a_val[e]));
+        for (int q = lane; q < len; q += 32) {
+            const uint32_t c = cell[o + q];
+            if (c == TRI_EMPTY) atomicOr(gflags, 2u);          // a cell no step reaches: inconsistent
+            else fm = max(fm, (int)(c & 0xffu));
         }
         fm = __reduce_max_sync(0xffffffffu, fm);
         if (lane == 0 && fm >= 0) atomicMax(cfm + ci, fm);
     }
 }
 
-// One warp per general matrix: its triples (ordered by step) streamed in chunks of TRI_CHUNK,
-// each chunk loaded TRI_PREFETCH chunks ahead so that no step waits for its triples; within a
-// chunk the lanes take the chunk's steps in order (a warp barrier after each), so one step's
-// stores come before the next step's loads.  A cell is tracked by the MSB of its current value alone
-// (0: no value yet): msb(x (x) y) = msb(x) + msb(y) in the clean regime and msb(min(a, b)) =
-// min(msb(a), msb(b)), so the products' MSBs and each cell's first value, all the replay decides
-// from, come out exactly.  The matrix's P MSBs, one byte each, lie contiguously at
-// curg + lpos[first row].  SMEM: one CTA of one warp per matrix with P <= TRI_SMEM_CELLS copies
-// them into shared memory first (a step then costs a shared-memory round trip, not one to L2);
-// otherwise a warp per matrix with P > TRI_SMEM_CELLS works on them in place.  The chain of steps
-// of the largest matrices (~2,300 non-empty steps) sets the kernel's length.
-constexpr int TRI_PER_LANE = 4;              // triples of a chunk per lane
-constexpr int TRI_CHUNK = 32 * TRI_PER_LANE;
-constexpr int TRI_PREFETCH = 4;              // chunks in flight
-constexpr int64_t TRI_SMEM_CELLS = 57344;    // 56 KB of shared memory: four one-warp CTAs per SM
-
-template <bool SMEM>
-__global__ void __launch_bounds__(SMEM ? 32 : 256)
-tri_gen_replay_kernel(int count, const TriComp *__restrict__ comps, const int32_t *__restrict__ ckind,
-                      const unsigned *__restrict__ cbad, const int64_t *__restrict__ tpos,
-                      const int64_t *__restrict__ lpos, const int4 *__restrict__ trip, const DagCounters *dc,
-                      const unsigned *any_gen, const unsigned *gflags, uint8_t *curg, int *__restrict__ cam,
-                      int *__restrict__ cfm, unsigned long long *__restrict__ cprod) {
-    if (!tri_dag_ok(dc) || !*any_gen) return;
-    extern __shared__ __align__(16) uint8_t tri_cells[];
-    const int lane = threadIdx.x & 31;
-    const int warps = SMEM ? gridDim.x : gridDim.x * (blockDim.x >> 5);
-    const int first_ci = SMEM ? blockIdx.x : blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    for (int ci = first_ci; ci < count; ci += warps) {
-        if (!tri_gen_row(ci, ckind, cbad, dc, gflags)) continue;   // warp-uniform
-        const int64_t base = comps[ci].row_base, rows = comps[ci].n;
-        const int64_t m0 = lpos[base], P = lpos[base + rows] - m0;
-        if (SMEM ? P > TRI_SMEM_CELLS : P <= TRI_SMEM_CELLS) continue;
-        uint8_t *val = curg + m0;
-        if (SMEM) {
-            for (int64_t q = lane; q < P; q += 32) tri_cells[q] = val[q];
-            __syncwarp();
-            val = tri_cells;
-        }
-        const int64_t T0 = tpos[base], T1 = tpos[base + rows];
-        // chunks of TRI_CHUNK triples, triple j of a lane at chunk position 32 j + lane (coalesced
-        // loads; a lane's triples ascend by step); a ring of TRI_PREFETCH chunks in flight, slot d
-        // holding chunk c0 + d and refilled with chunk c0 + d + TRI_PREFETCH once taken (slots are
-        // compile-time indices, so no register awaiting its load is read early)
-        auto fetch = [&](int64_t c, int j) -> int4 {
-            const int64_t t = T0 + c * TRI_CHUNK + 32 * j + lane;
-            return t < T1 ? trip[t] : make_int4(0, 0, 0, INT_MAX);
-        };
-        int4 q[TRI_PREFETCH][TRI_PER_LANE];
-#pragma unroll
-        for (int d = 0; d < TRI_PREFETCH; ++d)
-#pragma unroll
-            for (int j = 0; j < TRI_PER_LANE; ++j) q[d][j] = fetch(d, j);
-        int top = -1, first = -1;
-        unsigned long long prods = 0;
-        const int64_t chunks = (T1 - T0 + TRI_CHUNK - 1) / TRI_CHUNK;
-        for (int64_t c0 = 0; c0 < chunks; c0 += TRI_PREFETCH)
-#pragma unroll
-        for (int d = 0; d < TRI_PREFETCH; ++d) {
-            const int64_t c = c0 + d;
-            if (c >= chunks) break;                                   // warp-uniform
-            int4 tr[TRI_PER_LANE];
-#pragma unroll
-            for (int j = 0; j < TRI_PER_LANE; ++j) {
-                tr[j] = q[d][j];
-                q[d][j] = fetch(c + TRI_PREFETCH, j);
-            }
-            // the chunk's steps in order: each lane does all its triples of the step at once
-            // (a step's triples are independent), then a warp barrier
-            int next = 0;                                             // the lane's first pending triple
-            while (true) {
-                int mine = INT_MAX;
-#pragma unroll
-                for (int j = 0; j < TRI_PER_LANE; ++j)
-                    if (j == next) mine = tr[j].w;
-                const int k = __reduce_min_sync(0xffffffffu, next < TRI_PER_LANE ? mine : INT_MAX);
-                if (k == INT_MAX) break;                              // warp-uniform
-#pragma unroll
-                for (int j = 0; j < TRI_PER_LANE; ++j) {
-                    if (j < next || tr[j].w != k) continue;
-                    ++next;
-                    if ((uint64_t)(uint32_t)tr[j].x >= (uint64_t)P || (uint64_t)(uint32_t)tr[j].y >= (uint64_t)P ||
-                        (uint64_t)(uint32_t)tr[j].z >= (uint64_t)P) {
-                        atomicOr(const_cast<int *>(&dc->flags), TRI_BAD_ROW);
-                        continue;
-                    }
-                    // the three cells are read together: one round trip per step
-                    const int mx = val[tr[j].x], my = val[tr[j].y], old = val[tr[j].z];
-                    if (mx != 0 && my != 0) {
-                        const int pm = mx + my;              // the product's MSB
-                        top = max(top, pm);
-                        ++prods;
-                        if (old == 0) {
-                            first = max(first, pm);
-                            val[tr[j].z] = (uint8_t)pm;
-                        } else if (pm < old) {
-                            val[tr[j].z] = (uint8_t)pm;
-                        }
-                    }
-                }
-                __syncwarp();
-            }
-        }
-        top = __reduce_max_sync(0xffffffffu, top);
-        first = __reduce_max_sync(0xffffffffu, first);
-        for (int o = 16; o > 0; o >>= 1) prods += __shfl_xor_sync(0xffffffffu, prods, o);
-        if (lane == 0) {
-            if (top >= 0) atomicMax(cam + ci, top);
-            if (first >= 0) atomicMax(cfm + ci, first);
-            cprod[ci] += prods;
-        }
-    }
-}
+// shared memory of a dense search over matrices of up to n rows, and of a CTA of table searches
+constexpr size_t tri_dense_smem(int n) { return (size_t)n * 4 + (size_t)(n + 32) * 2; }
+constexpr size_t TRI_TAB_SMEM = (size_t)TRI_SEARCH_WARPS * (TRI_TAB * 4 + TRI_LIST * 2);
 
 PerDeviceOnce g_tri_configured;
 int tri_configure() {
     return g_tri_configured.run([] {
-        RBG_CUDA_TRY(cudaFuncSetAttribute(tri_gen_replay_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)TRI_SMEM_CELLS));
+        RBG_CUDA_TRY(cudaFuncSetAttribute(tri_gen_search_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)tri_dense_smem((int)TRI_MAX_N)));
         return (int)RBG_OK;
     });
 }
 
-// Recorded graphs: the IF node around the replay opens only when the closure by levels went
-// through and some matrix needs the replay; the decision is also kept for the launch count.
+// Recorded graphs: the IF node around the searches opens only when the closure by levels went
+// through and some matrix needs them; the decision is also kept for the launch count.
 __global__ void tri_gen_gate_kernel(const DagCounters *dc, const unsigned *any_gen, unsigned *ran,
                                     cudaGraphConditionalHandle h) {
     if (threadIdx.x != 0) return;
@@ -660,7 +648,7 @@ int tri_captured_if(cudaStream_t s, Gate gate, Body body) {
     return RBG_OK;
 }
 
-constexpr int TRI_GEN_LAUNCHES = 10;         // launches of the replay block
+constexpr int TRI_GEN_LAUNCHES = 4;          // launches of the any-numbering block
 
 __device__ __forceinline__ bool tri_accepted(int ci, const int32_t *ckind, const int *cam, const unsigned *cbad,
                                              const DagCounters *dc, const unsigned *gflags) {
@@ -839,19 +827,18 @@ struct Carve {
 // row index, and the row pool in whatever remains.
 struct TriLayout {
     TriComp *dc;
-    int64_t *dpre, *indptr, *row_off, *ccnt, *cptr, *tcnt, *tpos, *lpos;
+    int64_t *dpre, *indptr, *row_off;
     unsigned *cflags, *cbad, *gflags;        // gflags[0]: the general path's scratch overflowed; [1]: any general;
-                                             // [2]: the replay ran (recorded graphs: its IF node's decision)
+                                             // [2]: the any-numbering block ran (its IF node's decision)
     int32_t *ckind, *row_cnt, *row_comp, *slot_col, *slot_val, *a_col, *a_val, *row_len, *p_col, *p_val;
-    int32_t *ccur, *csc_row, *csc_pos;
-    uint8_t *cur;                            // the replay's current MSB per pattern entry
-    int4 *trip;                              // (pool positions of (i, k), (k, j), (i, j); step k)
+    int32_t *ovf;                            // any numbering: count and rows of the searches the table is too small for
+    uint32_t *cell;                          // any numbering: per pool entry, the key of the cell's first value
     int *cam, *cfm;
     unsigned long long *cprod;
     TriOut *res;
     void *tmp, *dag_ws;
     size_t scan_tmp;
-    int64_t pool, csc_cap, trip_cap;
+    int64_t pool;
     size_t fixed;                            // bytes before the pool
 };
 
@@ -880,32 +867,22 @@ void tri_layout(unsigned char *base, size_t ws_bytes, size_t C, size_t NR, TriLa
     L.dag_ws = cv.take<unsigned char>(dag_workspace_for((int64_t)NR, (int64_t)(NR * TRI_CAP)));
     L.row_off = cv.take<int64_t>(NR);
     L.row_len = cv.take<int32_t>(NR);
-    L.ccnt = cv.take<int64_t>(NR + 1);
-    L.cptr = cv.take<int64_t>(NR + 1);
-    L.ccur = cv.take<int32_t>(NR);
-    L.tcnt = cv.take<int64_t>(NR + 1);
-    L.tpos = cv.take<int64_t>(NR + 1);
-    L.lpos = cv.take<int64_t>(NR + 1);
+    L.ovf = cv.take<int32_t>(NR + 1);
     L.fixed = align_up(cv.off, 256);
-    // the rest: 40% for the row pool (column, value and the replay's current MSB per entry),
-    // 15% for the transposed pattern, 45% for the replay's triples
-    const size_t rest = ws_bytes > L.fixed + 2048 ? ws_bytes - L.fixed - 2048 : 0;
-    L.pool = std::min<int64_t>((int64_t)(rest / 10 * 4 / 9 / 64 * 64), (int64_t)INT32_MAX / 64 * 64);
-    L.csc_cap = (int64_t)(rest / 100 * 15 / 8);
-    L.trip_cap = (int64_t)(rest / 100 * 45 / 16);
+    // the rest: the row pool, 12 bytes an entry (column, value, first-value key)
+    const size_t rest = ws_bytes > L.fixed + 1024 ? ws_bytes - L.fixed - 1024 : 0;
+    L.pool = std::min<int64_t>((int64_t)(rest / 12 / 64 * 64), (int64_t)INT32_MAX / 64 * 64);
     Carve tail{base};
     tail.off = L.fixed;
     L.p_col = tail.take<int32_t>((size_t)L.pool);
     L.p_val = tail.take<int32_t>((size_t)L.pool);
-    L.cur = tail.take<uint8_t>((size_t)L.pool);
-    L.csc_row = tail.take<int32_t>((size_t)L.csc_cap);
-    L.csc_pos = tail.take<int32_t>((size_t)L.csc_cap);
-    L.trip = tail.take<int4>((size_t)L.trip_cap);
+    L.cell = tail.take<uint32_t>((size_t)L.pool);
 }
 
 struct TriShape {
     int64_t count, R, ctas;
     int64_t ld_in, ld_out;
+    int max_n;                               // rows of the largest matrix on the path
 };
 
 // Every launch of the DAG path, in stream order, with no host synchronisation when `captured`
@@ -940,45 +917,31 @@ int tri_enqueue(const TriShape &sh, const TriLayout &L, const T *in, T *out, cud
     *launches += 5;
     rbg_csr_t A{R, R, L.indptr, L.a_col, L.a_val};
     RBG_CUDA_TRY(cudaMemsetAsync(L.row_len, 0xff, (size_t)R * 4, s));   // -1: never placed
+    DagChildren kids;
     int rc = dag_enqueue(&A, R * TRI_CAP, L.dag_ws, L.p_col, L.p_val, L.pool, L.row_off, L.row_len, s, captured,
-                         dcount, launches);
+                         dcount, &kids, launches);
     if (rc) return rc;
     timer_end(5, tdag, s);
-    // 2b. matrices in any numbering: the loop replayed on the closure's pattern (every kernel
-    // returns at once when the batch holds none; a recorded graph skips the block by an IF node)
+    // 2b. matrices in any numbering: the searches from every vertex (every kernel returns at once
+    // when the batch holds none; a recorded graph skips the block by an IF node)
     {
         cudaEvent_t tg = timer_begin(8, s);
         const DagCounters *dcn = *dcount;
         const unsigned *any = L.gflags + 1;
-        const int gw = grid_for(R * 32, 256);
-        RBG_CUDA_TRY(cudaMemsetAsync(L.ccnt, 0, (size_t)(R + 1) * 8, s));
-        RBG_CUDA_TRY(cudaMemsetAsync(L.ccur, 0, (size_t)R * 4, s));
+        RBG_CUDA_TRY(cudaMemsetAsync(L.ovf, 0, 4, s));
         auto body = [&](cudaStream_t b) -> int {
-            tri_gen_count_kernel<<<gw, 256, 0, b>>>(R, L.row_comp, L.ckind, L.row_off, L.row_len, L.p_col, dcn, any,
-                                                    L.cbad, L.ccnt);
-            size_t tb2 = L.scan_tmp;
-            RBG_CUDA_TRY(cub::DeviceScan::ExclusiveSum(L.tmp, tb2, L.ccnt, L.cptr, (int)(R + 1), b));
-            tri_gen_csc_kernel<<<gw, 256, 0, b>>>(R, L.row_comp, L.ckind, L.cbad, L.row_off, L.row_len, L.p_col, dcn,
-                                                  any, L.cptr, L.ccur, L.csc_row, L.csc_pos, L.csc_cap, L.gflags);
-            // (the column counts are scanned already: ccnt now takes the rows' pattern lengths)
-            tri_gen_tcount_kernel<<<grid_for(R + 1, 256), 256, 0, b>>>(R, L.row_comp, L.ckind, L.cbad, L.row_len,
-                                                                      L.cptr, dcn, any, L.gflags, L.tcnt, L.ccnt);
-            tb2 = L.scan_tmp;
-            RBG_CUDA_TRY(cub::DeviceScan::ExclusiveSum(L.tmp, tb2, L.tcnt, L.tpos, (int)(R + 1), b));
-            tb2 = L.scan_tmp;
-            RBG_CUDA_TRY(cub::DeviceScan::ExclusiveSum(L.tmp, tb2, L.ccnt, L.lpos, (int)(R + 1), b));
-            tri_gen_fill_kernel<<<gw, 256, 0, b>>>(R, L.row_comp, L.ckind, L.cbad, L.dc, L.row_off, L.row_len,
-                                                   L.p_col, L.cptr, L.csc_row, L.csc_pos, L.tpos, L.lpos, dcn, any,
-                                                   L.trip, L.trip_cap, L.gflags);
-            tri_gen_init_kernel<<<gw, 256, 0, b>>>(R, L.row_comp, L.ckind, L.cbad, L.indptr, L.a_col, L.a_val,
-                                                   L.row_off, L.row_len, L.p_col, L.lpos, dcn, any, L.gflags, L.cur,
-                                                   L.cfm);
-            tri_gen_replay_kernel<true><<<(unsigned)count, 32, (size_t)TRI_SMEM_CELLS, b>>>(
-                count, L.dc, L.ckind, L.cbad, L.tpos, L.lpos, L.trip, dcn, any, L.gflags, L.cur, L.cam, L.cfm,
-                L.cprod);
-            tri_gen_replay_kernel<false><<<grid_for((int64_t)count * 32, 256), 256, 0, b>>>(
-                count, L.dc, L.ckind, L.cbad, L.tpos, L.lpos, L.trip, dcn, any, L.gflags, L.cur, L.cam, L.cfm,
-                L.cprod);
+            const int gw = grid_for(R * 32, 256);
+            const TriGraphView G{L.indptr, L.a_col, L.a_val, kids.coff, kids.children};
+            tri_gen_init_kernel<<<gw, 256, 0, b>>>(R, L.row_comp, L.ckind, L.indptr, L.a_col, L.a_val, L.row_off,
+                                                   L.row_len, L.p_col, dcn, any, L.gflags, L.cbad, L.cell);
+            tri_gen_search_kernel<false><<<grid_for(R * 32, 32 * TRI_SEARCH_WARPS), 32 * TRI_SEARCH_WARPS, TRI_TAB_SMEM,
+                                           b>>>(R, L.row_comp, L.ckind, L.cbad, L.dc, G, L.row_off, L.row_len, L.p_col,
+                                                dcn, any, L.gflags, L.cell, L.ovf, TRI_TAB, L.cam, L.cprod);
+            tri_gen_search_kernel<true><<<4 * sm_count(), 32, tri_dense_smem(sh.max_n), b>>>(
+                R, L.row_comp, L.ckind, L.cbad, L.dc, G, L.row_off, L.row_len, L.p_col, dcn, any, L.gflags, L.cell,
+                L.ovf, sh.max_n, L.cam, L.cprod);
+            tri_gen_first_kernel<<<gw, 256, 0, b>>>(R, L.row_comp, L.ckind, L.cbad, L.row_off, L.row_len, dcn, any,
+                                                    L.gflags, L.cell, L.cfm);
             RBG_CUDA_TRY(cudaGetLastError());
             return (int)RBG_OK;
         };
@@ -1092,11 +1055,12 @@ int tri_batch(int64_t count, const int64_t *sizes, const int64_t *in_off, const 
     }
     std::vector<TriComp> hc((size_t)count);
     std::vector<int64_t> pre((size_t)count + 1, 0);
-    int64_t R = 0;
+    int64_t R = 0, max_n = 0;
     for (int64_t i = 0; i < count; ++i) {
         const int64_t n = (sizes[i] > 0 && sizes[i] <= TRI_MAX_N) ? sizes[i] : 0;
         hc[(size_t)i] = TriComp{n, in_off[i], out_off[i], R};
         R += n;
+        max_n = std::max(max_n, n);
         pre[(size_t)i + 1] = pre[(size_t)i] + (n + TRI_ROWS - 1) / TRI_ROWS;
     }
     if (R == 0 || R * TRI_CAP > INT32_MAX) return RBG_OK;
@@ -1105,7 +1069,7 @@ int tri_batch(int64_t count, const int64_t *sizes, const int64_t *in_off, const 
     tri_layout(nullptr, ws_bytes, C, NR, L);
     if (L.pool < 4 * R) return RBG_OK;       // no room for a closure: the other paths decide
     tri_layout(ws, ws_bytes, C, NR, L);
-    const TriShape sh{count, R, pre[C], ld_in, ld_out};
+    const TriShape sh{count, R, pre[C], ld_in, ld_out, (int)max_n};
     {
         HostStaging hs(s, C * sizeof(TriComp) + (C + 1) * 8 + C * sizeof(TriOut) + sizeof(DagCounters) + 256);
         int rc = hs.up(L.dc, hc.data(), C * sizeof(TriComp));

@@ -101,8 +101,8 @@ void launch_recording(bool on);
 // Benchmark timer (rbg_profile_begin / rbg_profile_end_slots): CUDA events around the kernels
 // of each slot, recorded on the launching stream while the timer is on.  Slots: 0 phase-3
 // tiles, 1 panels, 2 diagonal tiles, 3 convert + finalize, 4 DAG path scan, 5 DAG path
-// closure by levels (with its CSR), 6 DAG path statistics, 7 DAG path write, 8 DAG path replay
-// of matrices in any numbering (pattern, triples, replay).
+// closure by levels (with its CSR), 6 DAG path statistics, 7 DAG path write, 8 DAG path
+// searches of matrices in any numbering.
 constexpr int TIMER_SLOTS = 9;
 cudaEvent_t timer_begin(int slot, cudaStream_t s);
 void timer_end(int slot, cudaEvent_t start, cudaStream_t s);
@@ -137,16 +137,20 @@ struct DagCounters {
     unsigned long long reserved, max_abs, total;
     long long level;                         // the graph loop's level counter
 };
+struct DagChildren {         // children lists of the levels' graph, kept in the workspace
+    const int64_t *coff;
+    const int32_t *children;
+};
 size_t dag_workspace_for(int64_t n, int64_t nnz_bound);
 int dag_enqueue(const rbg_csr_t *A, int64_t nnz_bound, void *workspace, int32_t *pool_cols, int32_t *pool_vals,
                 int64_t pool_capacity, int64_t *row_off, int32_t *row_len, cudaStream_t s, bool captured,
-                DagCounters **counters, int64_t *launches);
+                DagCounters **counters, DagChildren *kids, int64_t *launches);
 constexpr int DAG_GRAPH_CHUNK = 4;           // levels per iteration of the graph's while node
 
 // fw_tri.cu: the components of an int32 or int64 batch that are acyclic and in the clean regime
 // (at most 16 off-diagonal entries per row, at most 8192 rows), closed through the DAG closure by
-// levels (in any numbering: off the topological order the loop is replayed on the closure's
-// pattern for the diameter and the overflow decision); sets closed[i] = TRI_CLOSED and results[i] for each
+// levels (in any numbering: off the topological order, searches from every vertex give
+// the diameter and the overflow decision); sets closed[i] = TRI_CLOSED and results[i] for each
 // of them and leaves every other component untouched.  closed[i] = TRI_TOP_BIT marks a component
 // the closure went through completely whose loop computes a product reaching bit 31: 32-bit
 // lanes would only report that risk, so the caller goes on with 64-bit lanes (int64) or the

@@ -58,15 +58,19 @@ constexpr int TRI_BM_WORDS = (int)(TRI_MAX_N / 32);
 constexpr unsigned TF_UNCLEAN = 1u, TF_BELOW = 2u, TF_ABOVE = 4u, TF_WIDE = 8u;
 constexpr int KIND_NONE = DAG_KIND_NONE, KIND_BELOW = DAG_KIND_BELOW, KIND_ABOVE = DAG_KIND_ABOVE;
 constexpr int KIND_GENERAL = DAG_KIND_GENERAL;
+constexpr int KIND_PENDING = -1;             // short closures: any numbering, left to the levels
 constexpr int TRI_TOP = DAG_TOP_MSB;         // products reaching bit 31 leave the path
 
 struct TriComp {
     int64_t n, in_off, out_off, row_base;    // row_base: first batch-global row
+    int64_t orig;                            // index in the caller's batch (row statistics)
 };
+
+constexpr int32_t TRI_PENDING = 3;           // closed by the levels in a second pass of the call
 
 // Result of one matrix, written on the device and read back once per call.
 struct TriOut {
-    int32_t verdict, diameter;               // verdict: TRI_OPEN, TRI_CLOSED or TRI_TOP_BIT
+    int32_t verdict, diameter;               // verdict: TRI_OPEN, TRI_CLOSED, TRI_TOP_BIT or TRI_PENDING
     unsigned long long executed;
 };
 
@@ -147,7 +151,7 @@ __global__ void __launch_bounds__(TRI_THREADS, 5)
 tri_scan_kernel(const T *__restrict__ in, int64_t ld_in, const TriComp *__restrict__ comps,
                 const int64_t *__restrict__ pre, int count, int32_t *__restrict__ slot_col,
                 int32_t *__restrict__ slot_val, int32_t *__restrict__ row_cnt, int32_t *__restrict__ row_comp,
-                unsigned *__restrict__ cflags) {
+                unsigned *__restrict__ cflags, unsigned long long *__restrict__ state) {
     constexpr int E = TriVec<T>::E;
     const int ci = tri_find(pre, count, blockIdx.x);
     const TriComp c = comps[ci];
@@ -198,6 +202,7 @@ tri_scan_kernel(const T *__restrict__ in, int64_t ld_in, const TriComp *__restri
     if (lane == 0) {
         row_cnt[g] = cnt;
         row_comp[g] = ci;
+        if (state) state[g] = 0;             // short closures: not closed yet
         if (flags) atomicOr(cflags + ci, flags);
     }
 }
@@ -249,7 +254,9 @@ __global__ void tri_csr_fill_kernel(int64_t R, const int32_t *__restrict__ row_c
 // The closure by levels kept every row in the pool (no pool overflow); otherwise nothing of this
 // call's DAG path is used.  A matrix with a row never placed (a cycle: only matrices with entries
 // on both sides of the diagonal can hold one) is marked in cbad.
-__device__ __forceinline__ bool tri_dag_ok(const DagCounters *dc) { return !(dc->flags & 7); }
+constexpr int TRI_DAG_BAD = 15;              // DagCounters::flags that reject the call's DAG path
+constexpr int TRI_GAVE_UP = 8;               // a bounded wait of the short closure ran out
+__device__ __forceinline__ bool tri_dag_ok(const DagCounters *dc) { return !(dc->flags & TRI_DAG_BAD); }
 
 // A closure row entry outside its matrix (which a consistent closure never holds): the access is
 // skipped and the call's DAG path rejected (flag 4), so the blocked kernels decide.
@@ -590,6 +597,244 @@ __global__ void tri_gen_first_kernel(int64_t R, const int32_t *__restrict__ row_
     }
 }
 
+// ------------------------------------------------------------------------------------------
+// Short closures: matrices in a topological order, few rows in all
+// ------------------------------------------------------------------------------------------
+// With few rows the closure by levels is launches and their latency (three kernels a level, the
+// children lists and row orders before them).  Here every row is one warp that waits for its
+// parents itself: the warp takes the next row in the order of a ticket (a matrix with entries
+// below the diagonal from its first row, one with entries above from its last), so a row's parents
+// have smaller tickets, held by warps that run already, and every wait ends (it is bounded all the
+// same).  A finished row is published as one 64-bit word, its pool position and length, stored
+// after a fence and read with an acquire.
+//
+// The row itself: the columns of its entries and of its parents' rows are marked in a bitmap (a
+// word per 32 columns), whose prefix counts give every column its place in the row; the values
+// meet there by atomic minima.  The bitmap also tells a product that reaches a cell first, the
+// statistics of dag_rows.cuh: below the diagonal while the parents are folded in (ascending, the
+// loop's step order), above it in a second walk after the row is published.
+//
+// Latency bound: about 2 us per generation.  One n = 512 pedigree in 12 generations takes 81 us,
+// 389 us by levels; n = 8192, int64: 313 us, 835 us by levels.
+constexpr int TRI_PULL_WARPS = 8;            // warps (rows) per CTA
+constexpr int TRI_PULL_CTAS = 4;             // CTAs per SM
+constexpr int64_t TRI_PULL_ROWS = 16384;     // rows of a call on this path
+constexpr int TRI_PULL_VALS = 512;           // columns of a row kept in shared memory
+constexpr int TRI_PULL_TRIES = 1 << 22;      // polls of a parent before the call's DAG path is given up
+constexpr int TRI_STATE_LEN_BITS = 24;
+
+struct TriPullWarp {
+    unsigned bm[TRI_BM_WORDS];
+    unsigned short pre[TRI_BM_WORDS];        // columns before the word
+    int col[TRI_PULL_VALS], val[TRI_PULL_VALS];
+};
+
+__device__ __forceinline__ unsigned long long tri_acquire(const unsigned long long *p) {
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void tri_release(unsigned long long *p, unsigned long long v) {
+    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+__global__ void __launch_bounds__(32 * TRI_PULL_WARPS, TRI_PULL_CTAS)
+tri_pull_kernel(int64_t R, const int32_t *__restrict__ row_comp, const TriComp *__restrict__ comps,
+                const unsigned *__restrict__ cflags, const int32_t *__restrict__ slot_col,
+                const int32_t *__restrict__ slot_val, const int32_t *__restrict__ row_cnt,
+                unsigned long long *state, int64_t *__restrict__ row_off, int32_t *__restrict__ row_len,
+                int32_t *p_col, int32_t *p_val, int64_t capacity, DagCounters *dc, int *ticket,
+                int32_t *__restrict__ ckind, int *__restrict__ cam, int *__restrict__ cfm,
+                unsigned long long *__restrict__ cprod) {
+    __shared__ TriPullWarp warps[TRI_PULL_WARPS];
+    TriPullWarp &S = warps[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    while (true) {
+        int t = 0;
+        if (lane == 0) t = atomicAdd(ticket, 1);
+        t = __shfl_sync(0xffffffffu, t, 0);
+        if (t >= R) return;
+        const int ci = row_comp[t];
+        const unsigned f = cflags[ci];
+        const TriComp c = comps[ci];
+        const int n = (int)c.n, words = (n + 31) >> 5;
+        const int kind = (f & (TF_UNCLEAN | TF_WIDE)) ? KIND_NONE
+                         : ((f & TF_BELOW) && (f & TF_ABOVE)) ? KIND_PENDING
+                         : (f & TF_ABOVE) ? KIND_ABOVE : KIND_BELOW;
+        if (t == c.row_base && lane == 0) ckind[ci] = kind;
+        if (kind <= KIND_NONE) continue;     // warp-uniform
+        // a matrix with entries above the diagonal goes from its last row to its first
+        const int64_t g = kind == KIND_ABOVE ? 2 * c.row_base + n - 1 - t : t;
+        const int cnt = row_cnt[g];          // at most TRI_CAP
+        int w = -1, v = 0, len = 0;
+        int64_t off = 0;
+        if (lane < cnt) {
+            w = slot_col[g * TRI_CAP + lane];
+            v = slot_val[g * TRI_CAP + lane];
+        }
+        for (int q = lane; q < words; q += 32) S.bm[q] = 0;
+        __syncwarp();
+        if (lane < cnt) atomicOr(&S.bm[w >> 5], 1u << (w & 31));
+        // the parents' rows, as soon as they are published
+        bool late = false;
+        if (lane < cnt) {
+            unsigned long long st = 0;
+            int tries = 0;
+            while ((st = tri_acquire(state + c.row_base + w)) == 0 && ++tries < TRI_PULL_TRIES) {}
+            late = st == 0;
+            if (st) {
+                off = (int64_t)(st >> TRI_STATE_LEN_BITS) - 1;
+                len = (int)(st & ((1u << TRI_STATE_LEN_BITS) - 1u));
+            }
+        }
+        __syncwarp();
+        int incl = len;                      // the parents' entries, flattened over the warp
+#pragma unroll
+        for (int o = 1; o < TRI_CAP; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += x;
+        }
+        const int excl = incl - len;
+        const int total = __shfl_sync(0xffffffffu, incl, TRI_CAP - 1);
+        // pool room for the row's bound, asked for while the parents' rows are read
+        unsigned long long at = 0;
+        if (lane == 0) at = atomicAdd(&dc->reserved, (unsigned long long)(total + cnt));
+        int am = -1, fm = lane < cnt ? dag_row_msb(v) : -1;
+        // candidate idx of the flattened rows: its column and product (0 beyond the end)
+        auto candidate = [&](int idx, int &col, int &pm) -> int {
+            int lo = 0;
+#pragma unroll
+            for (int sft = TRI_CAP / 2; sft > 0; sft >>= 1) {
+                const int x = __shfl_sync(0xffffffffu, excl, lo + sft);
+                if (lo + sft < cnt && x <= idx) lo += sft;
+            }
+            const int vq = __shfl_sync(0xffffffffu, v, lo), xq = __shfl_sync(0xffffffffu, excl, lo);
+            const int64_t oq = __shfl_sync(0xffffffffu, off, lo);
+            col = -1 - lane;                 // no column, each lane its own
+            pm = -1;
+            if (idx >= total) return 0;
+            col = __ldcg(p_col + oq + (idx - xq)) - (int)c.row_base;
+            const int y = __ldcg(p_val + oq + (idx - xq));
+            pm = dag_row_msb(vq) + dag_row_msb(y);
+            return cy_product(vq, y);
+        };
+        // the first 128 candidates stay in registers
+        int kc[4], kv[4];
+        for (int b = 0; b < total; b += 128) {
+            int km[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (b + 32 * u < total) {
+                    int cc, pp;
+                    const int vv = candidate(b + 32 * u + lane, cc, pp);
+                    km[u] = pp;
+                    if (b == 0) { kc[u] = cc; kv[u] = vv; }
+                    am = max(am, pp);
+                    // the lowest lane of a column not yet marked performs the cell's first product
+                    const unsigned same = __match_any_sync(0xffffffffu, cc);
+                    if (cc >= 0 && !(same & below) && !((S.bm[cc >> 5] >> (cc & 31)) & 1u)) {
+                        if (kind == KIND_BELOW) fm = max(fm, km[u]);
+                        atomicOr(&S.bm[cc >> 5], 1u << (cc & 31));
+                    }
+                    __syncwarp();
+                }
+        }
+        // places of the columns: words [lane * wl, lane * wl + wl) per lane
+        const int wl = (words + 31) >> 5;
+        int mine = 0;
+        for (int q = lane * wl; q < min(words, (lane + 1) * wl); ++q) mine += __popc(S.bm[q]);
+        int run = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, run, o);
+            if (lane >= o) run += x;
+        }
+        const int nd = __shfl_sync(0xffffffffu, run, 31);
+        run -= mine;
+        for (int q = lane * wl; q < min(words, (lane + 1) * wl); ++q) {
+            S.pre[q] = (unsigned short)run;
+            run += __popc(S.bm[q]);
+        }
+        at = __shfl_sync(0xffffffffu, at, 0);
+        const bool room = (int64_t)at + total + cnt <= capacity;
+        const bool wide = nd > TRI_PULL_VALS;    // the values meet in the pool instead
+        int32_t *oc = wide ? p_col + at : S.col, *ov = wide ? p_val + at : S.val;
+        if (room) {
+            for (int q = lane; q < nd; q += 32) ov[q] = INT_MAX;
+            if (wide) __threadfence();
+            __syncwarp();
+            auto put = [&](int col, int val) {
+                const int r = S.pre[col >> 5] + __popc(S.bm[col >> 5] & ((1u << (col & 31)) - 1u));
+                oc[r] = (int)c.row_base + col;
+                if (val != 0) atomicMin(ov + r, val);
+            };
+            if (lane < cnt) put(w, v);
+            for (int b = 0; b < total; b += 128) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (b + 32 * u < total) {
+                        int cc = kc[u], pp, vv = kv[u];
+                        if (b > 0) vv = candidate(b + 32 * u + lane, cc, pp);
+                        if (cc >= 0) put(cc, vv);
+                    }
+            }
+            __syncwarp();
+            if (!wide)
+                for (int q = lane; q < nd; q += 32) {
+                    p_col[at + q] = S.col[q];
+                    p_val[at + q] = S.val[q];
+                }
+        }
+        late = __any_sync(0xffffffffu, late);
+        if (lane == 0) {
+            if (!room) atomicOr(&dc->flags, 1);
+            if (late) atomicOr(&dc->flags, TRI_GAVE_UP);
+            row_off[g] = (int64_t)at;
+            row_len[g] = room ? nd : 0;
+            __threadfence();
+            tri_release(state + g, ((at + 1) << TRI_STATE_LEN_BITS) | (unsigned long long)(room ? nd : 0));
+        }
+        __syncwarp();
+        unsigned long long prods = (unsigned long long)total;
+        if (kind == KIND_ABOVE) {
+            // steps k over the row ascending, each adding C(i, k) (x) A(k, .), two steps at a time
+            prods = 0;
+            for (int q = lane; q < words; q += 32) S.bm[q] = 0;
+            __syncwarp();
+            if (lane < cnt) atomicOr(&S.bm[w >> 5], 1u << (w & 31));
+            __syncwarp();
+            const int e = lane & (TRI_CAP - 1), half = lane / TRI_CAP;
+            for (int q = 0; room && q < nd; q += 32 / TRI_CAP) {
+                int j = -1 - lane, pm = -1;
+                if (q + half < nd) {
+                    const int64_t k = wide ? (int64_t)__ldcg(p_col + at + q + half) : (int64_t)S.col[q + half];
+                    const int kvv = wide ? __ldcg(p_val + at + q + half) : S.val[q + half];
+                    if (e < row_cnt[k]) {
+                        j = slot_col[k * TRI_CAP + e];
+                        pm = dag_row_msb(kvv) + dag_row_msb(slot_val[k * TRI_CAP + e]);
+                    }
+                }
+                am = max(am, pm);
+                prods += __popc(__ballot_sync(0xffffffffu, j >= 0));
+                const unsigned same = __match_any_sync(0xffffffffu, j);
+                if (j >= 0 && !(same & below) && !((S.bm[j >> 5] >> (j & 31)) & 1u)) {
+                    fm = max(fm, pm);
+                    atomicOr(&S.bm[j >> 5], 1u << (j & 31));
+                }
+                __syncwarp();
+            }
+        }
+        am = __reduce_max_sync(0xffffffffu, am);
+        fm = __reduce_max_sync(0xffffffffu, fm);
+        if (lane == 0) {
+            if (am >= 0) atomicMax(cam + ci, am);
+            if (fm >= 0) atomicMax(cfm + ci, fm);
+            if (prods) atomicAdd(cprod + ci, prods);
+        }
+    }
+}
+
 // shared memory of a dense search over matrices of up to n rows, and of a CTA of table searches
 constexpr size_t tri_dense_smem(int n) { return (size_t)n * 4 + (size_t)(n + 32) * 2; }
 constexpr size_t TRI_TAB_SMEM = (size_t)TRI_SEARCH_WARPS * (TRI_TAB * 4 + TRI_LIST * 2);
@@ -653,7 +898,7 @@ constexpr int TRI_GEN_LAUNCHES = 4;          // launches of the any-numbering bl
 __device__ __forceinline__ bool tri_accepted(int ci, const int32_t *ckind, const int *cam, const unsigned *cbad,
                                              const DagCounters *dc, const unsigned *gflags) {
     const int k = ckind[ci];
-    return k != KIND_NONE && cam[ci] < TRI_TOP && !cbad[ci] && tri_dag_ok(dc) && !(k == KIND_GENERAL && *gflags);
+    return k > KIND_NONE && cam[ci] < TRI_TOP && !cbad[ci] && tri_dag_ok(dc) && !(k == KIND_GENERAL && *gflags);
 }
 
 // The statistics are complete and some product of the loop reaches bit 31 (the first such
@@ -661,14 +906,15 @@ __device__ __forceinline__ bool tri_accepted(int ci, const int32_t *ckind, const
 __device__ __forceinline__ bool tri_top_bit(int ci, const int32_t *ckind, const int *cam, const unsigned *cbad,
                                             const DagCounters *dc, const unsigned *gflags) {
     const int k = ckind[ci];
-    return k != KIND_NONE && cam[ci] >= TRI_TOP && !cbad[ci] && tri_dag_ok(dc) && !(k == KIND_GENERAL && *gflags);
+    return k > KIND_NONE && cam[ci] >= TRI_TOP && !cbad[ci] && tri_dag_ok(dc) && !(k == KIND_GENERAL && *gflags);
 }
 
 // One warp per row of an accepted matrix.  Out of place, the whole dense row is written in
 // segments of SEG columns (2 KB) built in shared memory (zeros, the closure row's entries, the
 // diagonal) and stored as full 16-byte vectors on the row's 16-byte grid, so no DRAM line is
 // written partially; in place, only the closure's entries (the other cells already hold the
-// result).  The row statistics are recorded when asked for (32-bit storage).
+// result).  The row statistics are recorded when asked for (32-bit storage).  The first CTA of a
+// matrix writes its result record.
 template <typename T>
 __global__ void __launch_bounds__(TRI_THREADS)
 tri_write_kernel(const T *__restrict__ in, int64_t ld_in, T *__restrict__ out, int64_t ld_out,
@@ -676,12 +922,22 @@ tri_write_kernel(const T *__restrict__ in, int64_t ld_in, T *__restrict__ out, i
                  const int32_t *__restrict__ ckind, const int *__restrict__ cam, const unsigned *__restrict__ cbad,
                  const DagCounters *dc, const unsigned *gflags,
                  const int64_t *__restrict__ row_off, const int32_t *__restrict__ row_len,
-                 const int32_t *__restrict__ p_col, const int32_t *__restrict__ p_val, RowStats rs) {
+                 const int32_t *__restrict__ p_col, const int32_t *__restrict__ p_val, RowStats rs,
+                 const int *__restrict__ cfm, const unsigned long long *__restrict__ cprod, TriOut *__restrict__ res) {
     constexpr int SEG = 2048 / (int)sizeof(T);
     constexpr int E = TriVec<T>::E;
     __shared__ __align__(16) T seg_all[TRI_ROWS][SEG];
     const int ci = tri_find(pre, count, blockIdx.x);
-    if (!tri_accepted(ci, ckind, cam, cbad, dc, gflags)) return;   // block-uniform
+    const bool accepted = tri_accepted(ci, ckind, cam, cbad, dc, gflags);   // block-uniform
+    if ((int64_t)blockIdx.x == pre[ci] && threadIdx.x == 0) {
+        TriOut o;
+        o.verdict = accepted ? TRI_CLOSED : tri_top_bit(ci, ckind, cam, cbad, dc, gflags) ? TRI_TOP_BIT
+                    : ckind[ci] == KIND_PENDING ? TRI_PENDING : TRI_OPEN;
+        o.diameter = cfm[ci] > 0 ? cfm[ci] : 0;
+        o.executed = cprod[ci];
+        res[ci] = o;
+    }
+    if (!accepted) return;
     const TriComp c = comps[ci];
     const int i = (int)(((int64_t)blockIdx.x - pre[ci]) * TRI_ROWS) + (threadIdx.x >> 5);
     if (i >= c.n) return;                    // warp-uniform
@@ -781,33 +1037,19 @@ tri_write_kernel(const T *__restrict__ in, int64_t ld_in, T *__restrict__ out, i
             const unsigned long long wd[4] = {orw(w0), orw(w1), orw(w2), orw(w3)};
             mx = __reduce_max_sync(0xffffffffu, mx);
             if (lane == 0) {
-                const int64_t at = rs.row_base[ci] + i;
+                const int64_t at = rs.row_base[c.orig] + i;
                 rs.row_count[rs.row_id ? (int64_t)rs.row_id[at] : at] = clen + (diag != 0 ? 1 : 0);
                 if (rs.chunk_mask) {
                     const int64_t words = (n + 2047) / 2048;
-                    unsigned long long *mrow = rs.chunk_mask + (c.in_off + 2047) / 2048 + rs.row_base[ci] + ci +
+                    unsigned long long *mrow = rs.chunk_mask + (c.in_off + 2047) / 2048 + rs.row_base[c.orig] + c.orig +
                                                (int64_t)i * words;
 #pragma unroll
                     for (int t = 0; t < 4; ++t)
                         if (t < words) mrow[t] = wd[t];
                 }
-                if (rs.comp_max && mx > 0) atomicMax(rs.comp_max + ci, mx);
+                if (rs.comp_max && mx > 0) atomicMax(rs.comp_max + c.orig, mx);
             }
         }
-    }
-}
-
-__global__ void tri_result_kernel(int count, const int32_t *__restrict__ ckind, const int *__restrict__ cam,
-                                  const int *__restrict__ cfm, const unsigned long long *__restrict__ cprod,
-                                  const unsigned *__restrict__ cbad, const DagCounters *dc, const unsigned *gflags,
-                                  TriOut *__restrict__ res) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-        TriOut o;
-        o.verdict = tri_accepted(i, ckind, cam, cbad, dc, gflags) ? TRI_CLOSED
-                    : tri_top_bit(i, ckind, cam, cbad, dc, gflags) ? TRI_TOP_BIT : TRI_OPEN;
-        o.diameter = cfm[i] > 0 ? cfm[i] : 0;
-        o.executed = cprod[i];
-        res[i] = o;
     }
 }
 
@@ -823,12 +1065,14 @@ struct Carve {
 };
 
 // The scratch of one call, carved from the caller's workspace: the matrix table, per-matrix
-// flags and statistics, the scan's row slots, the candidates' CSR, the closure's workspace and
-// row index, and the row pool in whatever remains.
+// flags, statistics and results with the call's counters (`head`, uploaded whole at the start of a
+// call in its starting state), the scan's row slots, then either the candidates' CSR, the closure's
+// workspace and row index (levels) or the rows' states (short closures), and the row pool in
+// whatever remains.
 struct TriLayout {
     TriComp *dc;
     int64_t *dpre, *indptr, *row_off;
-    unsigned *cflags, *cbad, *gflags;        // gflags[0]: the general path's scratch overflowed; [1]: any general;
+    unsigned *cflags, *cbad, *gflags;        // gflags[0]: the searches' scratch is inconsistent; [1]: any general;
                                              // [2]: the any-numbering block ran (its IF node's decision)
     int32_t *ckind, *row_cnt, *row_comp, *slot_col, *slot_val, *a_col, *a_val, *row_len, *p_col, *p_val;
     int32_t *ovf;                            // any numbering: count and rows of the searches the table is too small for
@@ -836,16 +1080,18 @@ struct TriLayout {
     int *cam, *cfm;
     unsigned long long *cprod;
     TriOut *res;
+    DagCounters *counters;                   // short closures: the call's counters, beside the results
+    int *ticket;
+    unsigned long long *state;               // short closures: per row 0, or (pool position + 1) << 24 | length
     void *tmp, *dag_ws;
     size_t scan_tmp;
     int64_t pool;
+    size_t head;                             // bytes uploaded at the start of a call
     size_t fixed;                            // bytes before the pool
 };
 
-void tri_layout(unsigned char *base, size_t ws_bytes, size_t C, size_t NR, TriLayout &L) {
+void tri_layout(unsigned char *base, size_t ws_bytes, size_t C, size_t NR, bool is_short, TriLayout &L) {
     Carve cv{base};
-    L.scan_tmp = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, L.scan_tmp, (int64_t *)nullptr, (int64_t *)nullptr, (int)(NR + 1));
     L.dc = cv.take<TriComp>(C);
     L.dpre = cv.take<int64_t>(C + 1);
     L.cflags = cv.take<unsigned>(C);
@@ -855,19 +1101,28 @@ void tri_layout(unsigned char *base, size_t ws_bytes, size_t C, size_t NR, TriLa
     L.cprod = cv.take<unsigned long long>(C);
     L.cbad = cv.take<unsigned>(C);
     L.gflags = cv.take<unsigned>(3);
+    L.ticket = cv.take<int>(1);
+    L.counters = cv.take<DagCounters>(1);
     L.res = cv.take<TriOut>(C);
+    L.head = cv.off;
     L.row_cnt = cv.take<int32_t>(NR);
     L.row_comp = cv.take<int32_t>(NR);
     L.slot_col = cv.take<int32_t>(NR * TRI_CAP);
     L.slot_val = cv.take<int32_t>(NR * TRI_CAP);
-    L.indptr = cv.take<int64_t>(NR + 1);
-    L.tmp = cv.take<unsigned char>(L.scan_tmp);
-    L.a_col = cv.take<int32_t>(NR * TRI_CAP);
-    L.a_val = cv.take<int32_t>(NR * TRI_CAP);
-    L.dag_ws = cv.take<unsigned char>(dag_workspace_for((int64_t)NR, (int64_t)(NR * TRI_CAP)));
     L.row_off = cv.take<int64_t>(NR);
     L.row_len = cv.take<int32_t>(NR);
-    L.ovf = cv.take<int32_t>(NR + 1);
+    if (is_short) {
+        L.state = cv.take<unsigned long long>(NR);
+    } else {
+        L.scan_tmp = 0;
+        cub::DeviceScan::ExclusiveSum(nullptr, L.scan_tmp, (int64_t *)nullptr, (int64_t *)nullptr, (int)(NR + 1));
+        L.indptr = cv.take<int64_t>(NR + 1);
+        L.tmp = cv.take<unsigned char>(L.scan_tmp);
+        L.a_col = cv.take<int32_t>(NR * TRI_CAP);
+        L.a_val = cv.take<int32_t>(NR * TRI_CAP);
+        L.dag_ws = cv.take<unsigned char>(dag_workspace_for((int64_t)NR, (int64_t)(NR * TRI_CAP)));
+        L.ovf = cv.take<int32_t>(NR + 1);
+    }
     L.fixed = align_up(cv.off, 256);
     // the rest: the row pool, 12 bytes an entry (column, value, first-value key)
     const size_t rest = ws_bytes > L.fixed + 1024 ? ws_bytes - L.fixed - 1024 : 0;
@@ -892,14 +1147,13 @@ int tri_enqueue(const TriShape &sh, const TriLayout &L, const T *in, T *out, cud
                 const RowStats &rs, DagCounters **dcount, int64_t *launches) {
     const int64_t R = sh.R;
     const int count = (int)sh.count;
-    RBG_CUDA_TRY(cudaMemsetAsync(L.cflags, 0, (size_t)count * 4, s));
-    RBG_CUDA_TRY(cudaMemsetAsync(L.gflags, 0, 12, s));
     // 1. scan
     {
         cudaEvent_t t = timer_begin(4, s);
         note_launches(1);
         tri_scan_kernel<T><<<(unsigned)sh.ctas, TRI_THREADS, 0, s>>>(in, sh.ld_in, L.dc, L.dpre, count, L.slot_col,
-                                                                     L.slot_val, L.row_cnt, L.row_comp, L.cflags);
+                                                                     L.slot_val, L.row_cnt, L.row_comp, L.cflags,
+                                                                     nullptr);
         RBG_CUDA_TRY(cudaGetLastError());
         timer_end(4, t, s);
     }
@@ -974,17 +1228,15 @@ int tri_enqueue(const TriShape &sh, const TriLayout &L, const T *in, T *out, cud
     // 4. dense rows of the accepted matrices (decided on the device from the statistics)
     {
         cudaEvent_t t = timer_begin(7, s);
-        note_launches(2);
+        note_launches(1);
         tri_write_kernel<T><<<(unsigned)sh.ctas, TRI_THREADS, 0, s>>>(in, sh.ld_in, out, sh.ld_out, L.dc, L.dpre,
                                                                       count, L.ckind, L.cam, L.cbad, *dcount,
                                                                       L.gflags, L.row_off, L.row_len, L.p_col,
-                                                                      L.p_val, rs);
-        tri_result_kernel<<<(unsigned)std::min<int64_t>((count + 255) / 256, 1024), 256, 0, s>>>(
-            count, L.ckind, L.cam, L.cfm, L.cprod, L.cbad, *dcount, L.gflags, L.res);
+                                                                      L.p_val, rs, L.cfm, L.cprod, L.res);
         RBG_CUDA_TRY(cudaGetLastError());
         timer_end(7, t, s);
     }
-    *launches += 3;
+    *launches += 2;
     return RBG_OK;
 }
 
@@ -1044,47 +1296,88 @@ int tri_record(const TriShape &sh, const TriLayout &L, const T *in, T *out, cons
 
 }  // namespace
 
-template <typename T>
-int tri_batch(int64_t count, const int64_t *sizes, const int64_t *in_off, const int64_t *out_off, int64_t ld_in,
-              int64_t ld_out, const T *in, T *out, rbg_result_t *results, char *closed, unsigned char *ws,
-              size_t ws_bytes, uint32_t mode, cudaStream_t s, const RowStats &rs) {
-    if (count <= 0 || count > INT32_MAX || !ws) return RBG_OK;
-    {
-        const int rc = tri_configure();     // before any capture: kernel attributes per device
-        if (rc) return rc;
-    }
-    std::vector<TriComp> hc((size_t)count);
-    std::vector<int64_t> pre((size_t)count + 1, 0);
-    int64_t R = 0, max_n = 0;
-    for (int64_t i = 0; i < count; ++i) {
-        const int64_t n = (sizes[i] > 0 && sizes[i] <= TRI_MAX_N) ? sizes[i] : 0;
-        hc[(size_t)i] = TriComp{n, in_off[i], out_off[i], R};
-        R += n;
-        max_n = std::max(max_n, n);
-        pre[(size_t)i + 1] = pre[(size_t)i] + (n + TRI_ROWS - 1) / TRI_ROWS;
-    }
-    if (R == 0 || R * TRI_CAP > INT32_MAX) return RBG_OK;
-    const size_t C = (size_t)count, NR = (size_t)R;
-    TriLayout L;
-    tri_layout(nullptr, ws_bytes, C, NR, L);
-    if (L.pool < 4 * R) return RBG_OK;       // no room for a closure: the other paths decide
-    tri_layout(ws, ws_bytes, C, NR, L);
-    const TriShape sh{count, R, pre[C], ld_in, ld_out, (int)max_n};
-    {
-        HostStaging hs(s, C * sizeof(TriComp) + (C + 1) * 8 + C * sizeof(TriOut) + sizeof(DagCounters) + 256);
-        int rc = hs.up(L.dc, hc.data(), C * sizeof(TriComp));
-        if (!rc) rc = hs.up(L.dpre, pre.data(), (C + 1) * 8);
-        if (rc) return rc;
-    }
+namespace {
 
+// The host's part of one call over `count` matrices: the tables, the layout and the results.
+template <typename T> struct TriCall {
+    int64_t count;
+    const int64_t *sizes, *in_off, *out_off;
+    int64_t ld_in, ld_out;
+    const T *in;
+    T *out;
+    unsigned char *ws;
+    size_t ws_bytes;
+    uint32_t mode;
+    cudaStream_t s;
+    const RowStats &rs;
+    const int64_t *orig;                     // the matrices' numbers in the caller's batch (null: as they are)
+    TriShape sh;
+    TriLayout L;
+    std::vector<unsigned char> head;         // the head of the layout in its starting state
+    std::vector<TriOut> res;
+    DagCounters hd;
+
+    // rows and CTAs of the call; false: no matrix is within the path's sizes
+    bool shape() {
+        sh = TriShape{count, 0, 0, ld_in, ld_out, 0};
+        for (int64_t i = 0; i < count; ++i) {
+            const int64_t n = rows(i);
+            sh.R += n;
+            sh.ctas += (n + TRI_ROWS - 1) / TRI_ROWS;
+            sh.max_n = std::max<int>(sh.max_n, (int)n);
+        }
+        return sh.R > 0 && sh.R * TRI_CAP <= INT32_MAX;
+    }
+    int64_t rows(int64_t i) const { return (sizes[i] > 0 && sizes[i] <= TRI_MAX_N) ? sizes[i] : 0; }
+    // carve the workspace; false: no room for a closure (the other paths decide)
+    bool layout(bool is_short) {
+        tri_layout(nullptr, ws_bytes, (size_t)count, (size_t)sh.R, is_short, L);
+        if (L.pool < 4 * sh.R) return false;
+        TriLayout H;                         // the same offsets over the host's copy of the head
+        head.assign(L.head, 0);
+        tri_layout(head.data(), ws_bytes, (size_t)count, (size_t)sh.R, is_short, H);
+        tri_layout(ws, ws_bytes, (size_t)count, (size_t)sh.R, is_short, L);
+        int64_t row = 0, cta = 0;
+        for (int64_t i = 0; i < count; ++i) {
+            const int64_t n = rows(i);
+            H.dc[i] = TriComp{n, in_off[i], out_off[i], row, orig ? orig[i] : i};
+            H.dpre[i] = cta;
+            H.cam[i] = H.cfm[i] = -1;
+            row += n;
+            cta += (n + TRI_ROWS - 1) / TRI_ROWS;
+        }
+        H.dpre[count] = cta;
+        return true;
+    }
+    int upload() {
+        HostStaging hs(s, head.size() + (size_t)count * sizeof(TriOut) + sizeof(DagCounters) + 512);
+        return hs.up(ws, head.data(), head.size());
+    }
+    int read(const DagCounters *dcount, unsigned *gate_ran) {
+        res.resize((size_t)count);
+        HostStaging hs(s, (size_t)count * sizeof(TriOut) + sizeof(DagCounters) + 128);
+        int rc = hs.down(res.data(), L.res, (size_t)count * sizeof(TriOut));
+        if (!rc) rc = hs.down(&hd, dcount, sizeof(hd));
+        if (!rc && gate_ran) rc = hs.down(gate_ran, L.gflags + 2, 4);
+        if (!rc) rc = hs.finish();
+        return rc;
+    }
+};
+
+template <typename T> int tri_levels(TriCall<T> &c) {
+    if (!c.layout(false)) return RBG_OK;
+    int rc = c.upload();
+    if (rc) return rc;
     DagCounters *dcount = nullptr;
     int64_t fixed_launches = -1;             // >= 0: a graph ran; its level loop is counted below
-    if ((mode & RBG_MODE_GRAPH) && !timer_on()) {
+    if ((c.mode & RBG_MODE_GRAPH) && !timer_on()) {
         int dev = 0;
         RBG_CUDA_TRY(cudaGetDevice(&dev));
-        TriGraphKey key{dev, (int)sizeof(T), in, out, ws, ws_bytes, ld_in, ld_out,
-                        std::vector<int64_t>(sizes, sizes + count), std::vector<int64_t>(in_off, in_off + count),
-                        std::vector<int64_t>(out_off, out_off + count), rs};
+        const int64_t count = c.count;
+        TriGraphKey key{dev, (int)sizeof(T), c.in, c.out, c.ws, c.ws_bytes, c.ld_in, c.ld_out,
+                        std::vector<int64_t>(c.sizes, c.sizes + count),
+                        std::vector<int64_t>(c.in_off, c.in_off + count),
+                        std::vector<int64_t>(c.out_off, c.out_off + count), c.rs};
         std::lock_guard<std::mutex> lk(g_tri_graph_mu);
         TriGraph *hit = nullptr;
         for (auto &e : g_tri_graphs)
@@ -1092,7 +1385,7 @@ int tri_batch(int64_t count, const int64_t *sizes, const int64_t *in_off, const 
         if (!hit) {
             TriGraph g;
             g.key = std::move(key);
-            const int rc = tri_record<T>(sh, L, in, out, rs, g);
+            rc = tri_record<T>(c.sh, c.L, c.in, c.out, c.rs, g);
             if (rc) return rc;
             if (g_tri_graphs.size() >= TRI_GRAPH_CACHE) {
                 size_t old = 0;
@@ -1106,41 +1399,114 @@ int tri_batch(int64_t count, const int64_t *sizes, const int64_t *in_off, const 
             hit = &g_tri_graphs.back();
         }
         hit->stamp = ++g_tri_clock;
-        RBG_CUDA_TRY(cudaGraphLaunch(hit->exec, s));
+        RBG_CUDA_TRY(cudaGraphLaunch(hit->exec, c.s));
         dcount = hit->dcount;
         fixed_launches = hit->launches;
     } else {
         int64_t launches = 0;
-        const int rc = tri_enqueue<T>(sh, L, in, out, s, false, rs, &dcount, &launches);
+        rc = tri_enqueue<T>(c.sh, c.L, c.in, c.out, c.s, false, c.rs, &dcount, &launches);
         if (rc) return rc;
     }
-    std::vector<TriOut> h(C);
-    DagCounters hd;
     unsigned gate_ran = 0;
-    {
-        HostStaging hs(s, C * sizeof(TriOut) + sizeof(DagCounters) + 128);
-        int rc = hs.down(h.data(), L.res, C * sizeof(TriOut));
-        if (!rc) rc = hs.down(&hd, dcount, sizeof(hd));
-        if (!rc && fixed_launches >= 0) rc = hs.down(&gate_ran, L.gflags + 2, 4);
-        if (!rc) rc = hs.finish();
-        if (rc) return rc;
-    }
+    rc = c.read(dcount, fixed_launches >= 0 ? &gate_ran : nullptr);
+    if (rc) return rc;
     if (fixed_launches >= 0) {
-        const int64_t iters = std::max<int64_t>(1, (hd.nlevels + DAG_GRAPH_CHUNK - 1) / DAG_GRAPH_CHUNK);
+        const int64_t iters = std::max<int64_t>(1, (c.hd.nlevels + DAG_GRAPH_CHUNK - 1) / DAG_GRAPH_CHUNK);
         note_launches(fixed_launches + iters * (3 * DAG_GRAPH_CHUNK + 1) + (gate_ran ? TRI_GEN_LAUNCHES : 0));
     }
-    for (size_t i = 0; i < C; ++i) {
-        closed[i] = (char)h[i].verdict;
-        if (h[i].verdict != TRI_CLOSED) continue;
-        rbg_result_t &r = results[i];
+    return RBG_OK;
+}
+
+// Short closures: scan, one closure kernel, write.
+template <typename T> int tri_short(TriCall<T> &c) {
+    if (!c.layout(true)) return RBG_OK;
+    int rc = c.upload();
+    if (rc) return rc;
+    const TriLayout &L = c.L;
+    const int count = (int)c.count;
+    note_launches(3);
+    {
+        cudaEvent_t t = timer_begin(4, c.s);
+        tri_scan_kernel<T><<<(unsigned)c.sh.ctas, TRI_THREADS, 0, c.s>>>(c.in, c.ld_in, L.dc, L.dpre, count, L.slot_col,
+                                                                        L.slot_val, L.row_cnt, L.row_comp, L.cflags,
+                                                                        L.state);
+        timer_end(4, t, c.s);
+    }
+    {
+        cudaEvent_t t = timer_begin(5, c.s);
+        const int64_t need = (c.sh.R + TRI_PULL_WARPS - 1) / TRI_PULL_WARPS, most = (int64_t)TRI_PULL_CTAS * sm_count();
+        tri_pull_kernel<<<(unsigned)std::min<int64_t>(need, most), 32 * TRI_PULL_WARPS, 0, c.s>>>(
+            c.sh.R, L.row_comp, L.dc, L.cflags, L.slot_col, L.slot_val, L.row_cnt, L.state, L.row_off, L.row_len, L.p_col,
+            L.p_val, L.pool, L.counters, L.ticket, L.ckind, L.cam, L.cfm, L.cprod);
+        timer_end(5, t, c.s);
+    }
+    {
+        cudaEvent_t t = timer_begin(7, c.s);
+        tri_write_kernel<T><<<(unsigned)c.sh.ctas, TRI_THREADS, 0, c.s>>>(c.in, c.ld_in, c.out, c.ld_out, L.dc, L.dpre,
+                                                                         count, L.ckind, L.cam, L.cbad, L.counters,
+                                                                         L.gflags, L.row_off, L.row_len, L.p_col,
+                                                                         L.p_val, c.rs, L.cfm, L.cprod, L.res);
+        timer_end(7, t, c.s);
+    }
+    RBG_CUDA_TRY(cudaGetLastError());
+    return c.read(L.counters, nullptr);
+}
+
+template <typename T> void tri_take_results(const TriCall<T> &c, const int64_t *idx, rbg_result_t *results, char *closed) {
+    if (c.res.empty() || (c.hd.flags & TRI_DAG_BAD)) return;     // nothing of the DAG path is used
+    for (int64_t i = 0; i < c.count; ++i) {
+        const int64_t o = idx ? idx[i] : i;
+        const TriOut &h = c.res[(size_t)i];
+        closed[o] = (char)h.verdict;
+        if (h.verdict != TRI_CLOSED) continue;
+        rbg_result_t &r = results[o];
         r.status = RBG_OK;
         r.flags = 0;
-        r.diameter = h[i].diameter;
+        r.diameter = h.diameter;
         r.k = r.i = r.j = -1;
         r.path = RBG_PATH_DAG;
-        r.executed = (int64_t)h[i].executed;
+        r.executed = (int64_t)h.executed;
     }
-    return RBG_OK;
+}
+
+}  // namespace
+
+template <typename T>
+int tri_batch(int64_t count, const int64_t *sizes, const int64_t *in_off, const int64_t *out_off, int64_t ld_in,
+              int64_t ld_out, const T *in, T *out, rbg_result_t *results, char *closed, unsigned char *ws,
+              size_t ws_bytes, uint32_t mode, cudaStream_t s, const RowStats &rs) {
+    if (count <= 0 || count > INT32_MAX || !ws) return RBG_OK;
+    {
+        const int rc = tri_configure();     // before any capture: kernel attributes per device
+        if (rc) return rc;
+    }
+    TriCall<T> c{count, sizes, in_off, out_off, ld_in, ld_out, in, out, ws, ws_bytes, mode, s, rs, nullptr};
+    if (!c.shape()) return RBG_OK;
+    if (c.sh.R > TRI_PULL_ROWS) {
+        const int rc = tri_levels(c);
+        if (!rc) tri_take_results(c, nullptr, results, closed);
+        return rc;
+    }
+    int rc = tri_short(c);
+    if (rc) return rc;
+    tri_take_results(c, nullptr, results, closed);
+    // the matrices in any numbering, or all of them when the short closure gave up, by levels
+    std::vector<int64_t> idx, sz, io, oo;
+    for (int64_t i = 0; i < count; ++i) {
+        if (c.res.empty() || (c.hd.flags & TRI_DAG_BAD) || closed[i] != (char)TRI_PENDING) continue;
+        closed[i] = TRI_OPEN;
+        idx.push_back(i);
+        sz.push_back(sizes[i]);
+        io.push_back(in_off[i]);
+        oo.push_back(out_off[i]);
+    }
+    if (idx.empty()) return RBG_OK;
+    TriCall<T> g{(int64_t)idx.size(), sz.data(), io.data(), oo.data(), ld_in, ld_out, in, out, ws, ws_bytes, mode, s, rs,
+                 idx.data()};
+    if (!g.shape()) return RBG_OK;
+    rc = tri_levels(g);
+    if (!rc) tri_take_results(g, idx.data(), results, closed);
+    return rc;
 }
 
 template int tri_batch<int32_t>(int64_t, const int64_t *, const int64_t *, const int64_t *, int64_t, int64_t,

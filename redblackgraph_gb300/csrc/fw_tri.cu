@@ -63,7 +63,6 @@ constexpr int TRI_TOP = DAG_TOP_MSB;         // products reaching bit 31 leave t
 
 struct TriComp {
     int64_t n, in_off, out_off, row_base;    // row_base: first batch-global row
-    int64_t orig;                            // index in the caller's batch (row statistics)
 };
 
 constexpr int32_t TRI_PENDING = 3;           // closed by the levels in a second pass of the call
@@ -347,6 +346,34 @@ constexpr int TRI_SEARCH_WARPS = 8;          // warps per CTA (table searches)
 constexpr uint32_t TRI_EMPTY = 0xffffffffu;
 constexpr int TRI_FAR = 126;                 // lengths are capped (a product of MSB 31 is already a risk)
 
+// The candidates' graph for the searches, vertices batch-global: rows in CSR (columns batch-global)
+// or, with row_cnt, in TRI_CAP slots each (columns local); children of a vertex in any order.
+struct TriGraphView {
+    const int64_t *indptr;
+    const int32_t *row_cnt;
+    const int32_t *a_col, *a_val;
+    const int64_t *coff;
+    const int32_t *kid_cnt;                  // null: coff[v + 1] ends vertex v's list
+    const int32_t *children;
+    __device__ __forceinline__ int64_t row(int64_t g, int &cnt) const {
+        if (row_cnt) {
+            cnt = row_cnt[g];
+            return g * TRI_CAP;
+        }
+        const int64_t e = indptr[g];
+        cnt = (int)(indptr[g + 1] - e);
+        return e;
+    }
+    __device__ __forceinline__ int local(int64_t e, int64_t base) const {
+        return row_cnt ? a_col[e] : a_col[e] - (int)base;
+    }
+    __device__ __forceinline__ int64_t kids(int64_t g, int &cnt) const {
+        const int64_t e = coff[g];
+        cnt = kid_cnt ? kid_cnt[g] : (int)(coff[g + 1] - e);
+        return e;
+    }
+};
+
 // position of column c in the sorted closure row [o, o + len), or -1
 __device__ __forceinline__ int64_t tri_find_col(const int32_t *__restrict__ p_col, int64_t o, int len, int32_t c) {
     int lo = 0, hi = len - 1;
@@ -364,8 +391,8 @@ __device__ __forceinline__ int64_t tri_find_col(const int32_t *__restrict__ p_co
 // or below a cycle) marks its matrix; the cells of A's entries start with key 0 (their first value
 // is A's), the other cells empty.  Cell q of the row is cell[row_off + q].
 __global__ void tri_gen_init_kernel(int64_t R, const int32_t *__restrict__ row_comp, const int32_t *__restrict__ ckind,
-                                    const int64_t *__restrict__ indptr, const int32_t *__restrict__ a_col,
-                                    const int32_t *__restrict__ a_val, const int64_t *__restrict__ row_off,
+                                    const TriComp *__restrict__ comps, TriGraphView G,
+                                    const int64_t *__restrict__ row_off,
                                     const int32_t *__restrict__ row_len, const int32_t *__restrict__ p_col,
                                     const DagCounters *dc, const unsigned *any_gen, unsigned *gflags,
                                     unsigned *__restrict__ cbad, uint32_t *__restrict__ cell) {
@@ -374,7 +401,7 @@ __global__ void tri_gen_init_kernel(int64_t R, const int32_t *__restrict__ row_c
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
     for (int64_t g = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); g < R; g += warps) {
         const int ci = row_comp[g];
-        if (ckind[ci] != KIND_GENERAL) continue;   // warp-uniform
+        if (ckind[ci] != KIND_GENERAL || cbad[ci]) continue;   // warp-uniform
         const int len = row_len[g];
         if (len < 0) {
             if (lane == 0) atomicOr(cbad + ci, 1u);
@@ -383,20 +410,16 @@ __global__ void tri_gen_init_kernel(int64_t R, const int32_t *__restrict__ row_c
         const int64_t o = row_off[g];
         for (int q = lane; q < len; q += 32) cell[o + q] = TRI_EMPTY;
         __syncwarp();
-        for (int64_t e = indptr[g] + lane; e < indptr[g + 1]; e += 32) {
-            const int64_t q = tri_find_col(p_col, o, len, a_col[e]);
+        const int64_t base = comps[ci].row_base;
+        int cnt;
+        const int64_t e0 = G.row(g, cnt);
+        for (int64_t e = e0 + lane; e < e0 + cnt; e += 32) {
+            const int64_t q = tri_find_col(p_col, o, len, (int32_t)(base + G.local(e, base)));
             if (q < 0) atomicOr(gflags, 2u);
-            else cell[q] = (uint32_t)msb_u32((uint32_t)a_val[e]);   // a clean value: 2 <= v < 2^31
+            else cell[q] = (uint32_t)msb_u32((uint32_t)G.a_val[e]);   // a clean value: 2 <= v < 2^31
         }
     }
 }
-
-struct TriGraphView {                        // the candidates' graph, rows and columns batch-global
-    const int64_t *indptr;
-    const int32_t *a_col, *a_val;
-    const int64_t *coff;                     // children of a vertex (any order): edges child -> vertex
-    const int32_t *children;
-};
 
 // The table of a warp's search.  put() lowers vertex v's length to d and tells whether v is new
 // (`at`: where) or was shortened; the list holds `at`s.
@@ -453,11 +476,7 @@ __device__ __forceinline__ int tri_search(const TriGraphView &G, TriTable<DENSE>
                 dx = T.length(at);
                 x = v < k ? v : -1;          // a vertex above k is an end, never an intermediate
             }
-            if (x >= 0) {
-                const int64_t *ptr = FWD ? G.indptr : G.coff;
-                e0 = ptr[base + x];
-                cnt = (int)(ptr[base + x + 1] - e0);
-            }
+            if (x >= 0) e0 = FWD ? G.row(base + x, cnt) : G.kids(base + x, cnt);
         }
         h += left;
         int incl = cnt;
@@ -484,14 +503,15 @@ __device__ __forceinline__ int tri_search(const TriGraphView &G, TriTable<DENSE>
             if (idx < total) {
                 int y, len = 0;
                 if (FWD) {
-                    y = G.a_col[eq] - (int)base;
+                    y = G.local(eq, base);
                     len = msb_u32((uint32_t)G.a_val[eq]);
                 } else {
                     const int32_t c = G.children[eq];
                     y = c - (int)base;
-                    const int32_t want = (int32_t)(base + xq);   // the edge's value, in the child's row
-                    for (int64_t e = G.indptr[c]; e < G.indptr[c + 1]; ++e)
-                        if (G.a_col[e] == want) len = msb_u32((uint32_t)G.a_val[e]);
+                    int rc;                  // the edge's value, in the child's row
+                    const int64_t r0 = G.row(c, rc);
+                    for (int64_t e = r0; e < r0 + rc; ++e)
+                        if (G.local(e, base) == xq) len = msb_u32((uint32_t)G.a_val[e]);
                 }
                 got = T.put(y, min(dq + len, TRI_FAR), at);
             }
@@ -534,7 +554,10 @@ tri_gen_search_kernel(int64_t R, const int32_t *__restrict__ row_comp, const int
         const int64_t base = comps[ci].row_base;
         const int k = (int)(g - base);
         // a vertex without parents or without children is on no product
-        if (G.indptr[g + 1] == G.indptr[g] || G.coff[g + 1] == G.coff[g]) continue;
+        int parents, kids;
+        G.row(g, parents);
+        G.kids(g, kids);
+        if (parents == 0 || kids == 0) continue;
         const int no = tri_search<DENSE, true>(G, T, list, cap, 0, k, base, lane);
         const int used = no < 0 ? no : tri_search<DENSE, false>(G, T, list, cap, no, k, base, lane);
         const int ni = used - no;
@@ -645,7 +668,8 @@ tri_pull_kernel(int64_t R, const int32_t *__restrict__ row_comp, const TriComp *
                 unsigned long long *state, int64_t *__restrict__ row_off, int32_t *__restrict__ row_len,
                 int32_t *p_col, int32_t *p_val, int64_t capacity, DagCounters *dc, int *ticket,
                 int32_t *__restrict__ ckind, int *__restrict__ cam, int *__restrict__ cfm,
-                unsigned long long *__restrict__ cprod) {
+                unsigned long long *__restrict__ cprod, const int32_t *__restrict__ order,
+                const unsigned *__restrict__ cbad) {
     __shared__ TriPullWarp warps[TRI_PULL_WARPS];
     TriPullWarp &S = warps[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
@@ -659,13 +683,21 @@ tri_pull_kernel(int64_t R, const int32_t *__restrict__ row_comp, const TriComp *
         const unsigned f = cflags[ci];
         const TriComp c = comps[ci];
         const int n = (int)c.n, words = (n + 31) >> 5;
-        const int kind = (f & (TF_UNCLEAN | TF_WIDE)) ? KIND_NONE
-                         : ((f & TF_BELOW) && (f & TF_ABOVE)) ? KIND_PENDING
-                         : (f & TF_ABOVE) ? KIND_ABOVE : KIND_BELOW;
-        if (t == c.row_base && lane == 0) ckind[ci] = kind;
-        if (kind <= KIND_NONE) continue;     // warp-uniform
-        // a matrix with entries above the diagonal goes from its last row to its first
-        const int64_t g = kind == KIND_ABOVE ? 2 * c.row_base + n - 1 - t : t;
+        int kind;                            // warp-uniform
+        int64_t g = t;
+        if (order) {                         // the matrices in any numbering (tri_order_kernel)
+            kind = cbad[ci] ? KIND_NONE : ckind[ci];
+            if (kind <= KIND_NONE) continue;
+            g = order[t];
+        } else {
+            kind = (f & (TF_UNCLEAN | TF_WIDE)) ? KIND_NONE
+                   : ((f & TF_BELOW) && (f & TF_ABOVE)) ? KIND_PENDING
+                   : (f & TF_ABOVE) ? KIND_ABOVE : KIND_BELOW;
+            if (t == c.row_base && lane == 0) ckind[ci] = kind;
+            if (kind <= KIND_NONE) continue;
+            // a matrix with entries above the diagonal goes from its last row to its first
+            if (kind == KIND_ABOVE) g = 2 * c.row_base + n - 1 - t;
+        }
         const int cnt = row_cnt[g];          // at most TRI_CAP
         int w = -1, v = 0, len = 0;
         int64_t off = 0;
@@ -825,6 +857,7 @@ tri_pull_kernel(int64_t R, const int32_t *__restrict__ row_comp, const TriComp *
                 __syncwarp();
             }
         }
+        if (kind == KIND_GENERAL) continue;  // the searches take its statistics
         am = __reduce_max_sync(0xffffffffu, am);
         fm = __reduce_max_sync(0xffffffffu, fm);
         if (lane == 0) {
@@ -833,6 +866,99 @@ tri_pull_kernel(int64_t R, const int32_t *__restrict__ row_comp, const TriComp *
             if (prods) atomicAdd(cprod + ci, prods);
         }
     }
+}
+
+// Second pass of a short closure, one CTA per matrix: a matrix in any numbering gets its children
+// lists and its rows in a topological order (Kahn's algorithm by levels, the counters and the
+// frontier in shared memory, so a level costs two barriers and one read of the frontier's children);
+// one with a cycle is marked in cbad, every other matrix is taken off the path (its result is read
+// already).
+constexpr int TRI_ORDER_THREADS = 1024;
+struct TriOrderSmem {
+    int end[TRI_MAX_N];                      // children of v: [end[v - 1], end[v]) of the matrix's list
+    int rem[TRI_MAX_N];                      // parents not placed yet
+    unsigned short list[TRI_MAX_N];          // placed vertices
+};
+
+__global__ void __launch_bounds__(TRI_ORDER_THREADS)
+tri_order_kernel(const TriComp *__restrict__ comps, int32_t *ckind, const int32_t *__restrict__ slot_col,
+                 const int32_t *__restrict__ row_cnt, int32_t *__restrict__ order, int64_t *__restrict__ coff,
+                 int32_t *__restrict__ kid_cnt, int32_t *__restrict__ children, unsigned *__restrict__ cbad,
+                 int *ticket, unsigned *any_gen) {
+    extern __shared__ __align__(16) unsigned char tri_order_smem[];
+    TriOrderSmem &S = *reinterpret_cast<TriOrderSmem *>(tri_order_smem);
+    __shared__ int s_sum[TRI_ORDER_THREADS / 32], s_tail;
+    const int ci = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    if (ci == 0 && tid == 0) *ticket = 0;
+    const int kind = ckind[ci];
+    __syncthreads();
+    if (kind != KIND_PENDING) {
+        if (tid == 0) ckind[ci] = KIND_NONE;
+        return;
+    }
+    if (tid == 0) {
+        ckind[ci] = KIND_GENERAL;
+        atomicOr(any_gen, 1u);
+        s_tail = 0;
+    }
+    const TriComp c = comps[ci];
+    const int n = (int)c.n;
+    const int64_t g0 = c.row_base;
+    int32_t *kids = children + g0 * TRI_CAP;
+    for (int v = tid; v < n; v += TRI_ORDER_THREADS) S.end[v] = 0;
+    __syncthreads();
+    for (int v = tid; v < n; v += TRI_ORDER_THREADS) {
+        const int m = row_cnt[g0 + v];
+        S.rem[v] = m;
+        for (int e = 0; e < m; ++e) atomicAdd(&S.end[slot_col[(g0 + v) * TRI_CAP + e]], 1);
+    }
+    __syncthreads();
+    // exclusive scan of the counts, a run of consecutive vertices per thread
+    const int run = (n + TRI_ORDER_THREADS - 1) / TRI_ORDER_THREADS;
+    int sum = 0;
+    for (int v = tid * run; v < min(n, (tid + 1) * run); ++v) sum += S.end[v];
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += x;
+    }
+    if (lane == 31) s_sum[w] = incl;
+    __syncthreads();
+    int at = incl - sum;
+    for (int q = 0; q < w; ++q) at += s_sum[q];
+    for (int v = tid * run; v < min(n, (tid + 1) * run); ++v) {
+        const int k = S.end[v];
+        coff[g0 + v] = g0 * TRI_CAP + at;
+        kid_cnt[g0 + v] = k;
+        S.end[v] = at;                       // a cursor that ends at the list's end
+        at += k;
+    }
+    __syncthreads();
+    for (int v = tid; v < n; v += TRI_ORDER_THREADS) {
+        const int m = S.rem[v];
+        for (int e = 0; e < m; ++e)
+            kids[atomicAdd(&S.end[slot_col[(g0 + v) * TRI_CAP + e]], 1)] = (int32_t)(g0 + v);
+        if (m == 0) S.list[atomicAdd(&s_tail, 1)] = (unsigned short)v;
+    }
+    __syncthreads();                         // (the lists' writes are visible to the CTA)
+    // levels: 8 lanes per frontier vertex
+    int h = 0, tail = s_tail;
+    while (h < tail) {                       // block-uniform
+        for (int q = h + (tid >> 3); q < tail; q += TRI_ORDER_THREADS / 8) {
+            const int v = S.list[q];
+            for (int e = (v ? S.end[v - 1] : 0) + (tid & 7); e < S.end[v]; e += 8) {
+                const int k = kids[e] - (int)g0;
+                if (atomicSub(&S.rem[k], 1) == 1) S.list[atomicAdd(&s_tail, 1)] = (unsigned short)k;
+            }
+        }
+        __syncthreads();
+        h = tail;
+        tail = s_tail;
+        __syncthreads();
+    }
+    for (int q = tid; q < tail; q += TRI_ORDER_THREADS) order[g0 + q] = (int32_t)(g0 + S.list[q]);
+    if (tid == 0 && tail < n) cbad[ci] = 1u; // on a cycle, or below one
 }
 
 // shared memory of a dense search over matrices of up to n rows, and of a CTA of table searches
@@ -844,6 +970,8 @@ int tri_configure() {
     return g_tri_configured.run([] {
         RBG_CUDA_TRY(cudaFuncSetAttribute(tri_gen_search_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)tri_dense_smem((int)TRI_MAX_N)));
+        RBG_CUDA_TRY(cudaFuncSetAttribute(tri_order_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)sizeof(TriOrderSmem)));
         return (int)RBG_OK;
     });
 }
@@ -1037,17 +1165,17 @@ tri_write_kernel(const T *__restrict__ in, int64_t ld_in, T *__restrict__ out, i
             const unsigned long long wd[4] = {orw(w0), orw(w1), orw(w2), orw(w3)};
             mx = __reduce_max_sync(0xffffffffu, mx);
             if (lane == 0) {
-                const int64_t at = rs.row_base[c.orig] + i;
+                const int64_t at = rs.row_base[ci] + i;
                 rs.row_count[rs.row_id ? (int64_t)rs.row_id[at] : at] = clen + (diag != 0 ? 1 : 0);
                 if (rs.chunk_mask) {
                     const int64_t words = (n + 2047) / 2048;
-                    unsigned long long *mrow = rs.chunk_mask + (c.in_off + 2047) / 2048 + rs.row_base[c.orig] + c.orig +
+                    unsigned long long *mrow = rs.chunk_mask + (c.in_off + 2047) / 2048 + rs.row_base[ci] + ci +
                                                (int64_t)i * words;
 #pragma unroll
                     for (int t = 0; t < 4; ++t)
                         if (t < words) mrow[t] = wd[t];
                 }
-                if (rs.comp_max && mx > 0) atomicMax(rs.comp_max + c.orig, mx);
+                if (rs.comp_max && mx > 0) atomicMax(rs.comp_max + ci, mx);
             }
         }
     }
@@ -1083,6 +1211,8 @@ struct TriLayout {
     DagCounters *counters;                   // short closures: the call's counters, beside the results
     int *ticket;
     unsigned long long *state;               // short closures: per row 0, or (pool position + 1) << 24 | length
+    int32_t *order, *kid_cnt, *children;     // short closures in any numbering: rows in a topological order and
+    int64_t *coff;                           // the children lists (tri_order_kernel)
     void *tmp, *dag_ws;
     size_t scan_tmp;
     int64_t pool;
@@ -1111,8 +1241,13 @@ void tri_layout(unsigned char *base, size_t ws_bytes, size_t C, size_t NR, bool 
     L.slot_val = cv.take<int32_t>(NR * TRI_CAP);
     L.row_off = cv.take<int64_t>(NR);
     L.row_len = cv.take<int32_t>(NR);
+    L.ovf = cv.take<int32_t>(NR + 1);
     if (is_short) {
         L.state = cv.take<unsigned long long>(NR);
+        L.order = cv.take<int32_t>(NR);
+        L.coff = cv.take<int64_t>(NR);
+        L.kid_cnt = cv.take<int32_t>(NR);
+        L.children = cv.take<int32_t>(NR * TRI_CAP);
     } else {
         L.scan_tmp = 0;
         cub::DeviceScan::ExclusiveSum(nullptr, L.scan_tmp, (int64_t *)nullptr, (int64_t *)nullptr, (int)(NR + 1));
@@ -1121,7 +1256,6 @@ void tri_layout(unsigned char *base, size_t ws_bytes, size_t C, size_t NR, bool 
         L.a_col = cv.take<int32_t>(NR * TRI_CAP);
         L.a_val = cv.take<int32_t>(NR * TRI_CAP);
         L.dag_ws = cv.take<unsigned char>(dag_workspace_for((int64_t)NR, (int64_t)(NR * TRI_CAP)));
-        L.ovf = cv.take<int32_t>(NR + 1);
     }
     L.fixed = align_up(cv.off, 256);
     // the rest: the row pool, 12 bytes an entry (column, value, first-value key)
@@ -1139,6 +1273,23 @@ struct TriShape {
     int64_t ld_in, ld_out;
     int max_n;                               // rows of the largest matrix on the path
 };
+
+// The any-numbering block: TRI_GEN_LAUNCHES launches.
+void tri_searches(const TriShape &sh, const TriLayout &L, const TriGraphView &G, const DagCounters *dc, cudaStream_t s) {
+    const int64_t R = sh.R;
+    const int gw = grid_for(R * 32, 256);
+    const unsigned *any = L.gflags + 1;
+    tri_gen_init_kernel<<<gw, 256, 0, s>>>(R, L.row_comp, L.ckind, L.dc, G, L.row_off, L.row_len, L.p_col, dc, any,
+                                           L.gflags, L.cbad, L.cell);
+    tri_gen_search_kernel<false><<<grid_for(R * 32, 32 * TRI_SEARCH_WARPS), 32 * TRI_SEARCH_WARPS, TRI_TAB_SMEM, s>>>(
+        R, L.row_comp, L.ckind, L.cbad, L.dc, G, L.row_off, L.row_len, L.p_col, dc, any, L.gflags, L.cell, L.ovf, TRI_TAB,
+        L.cam, L.cprod);
+    tri_gen_search_kernel<true><<<4 * sm_count(), 32, tri_dense_smem(sh.max_n), s>>>(
+        R, L.row_comp, L.ckind, L.cbad, L.dc, G, L.row_off, L.row_len, L.p_col, dc, any, L.gflags, L.cell, L.ovf,
+        sh.max_n, L.cam, L.cprod);
+    tri_gen_first_kernel<<<gw, 256, 0, s>>>(R, L.row_comp, L.ckind, L.cbad, L.row_off, L.row_len, dc, any, L.gflags,
+                                            L.cell, L.cfm);
+}
 
 // Every launch of the DAG path, in stream order, with no host synchronisation when `captured`
 // (the level loop then is a while node).  Returns the number of kernel launches issued.
@@ -1184,18 +1335,8 @@ int tri_enqueue(const TriShape &sh, const TriLayout &L, const T *in, T *out, cud
         const unsigned *any = L.gflags + 1;
         RBG_CUDA_TRY(cudaMemsetAsync(L.ovf, 0, 4, s));
         auto body = [&](cudaStream_t b) -> int {
-            const int gw = grid_for(R * 32, 256);
-            const TriGraphView G{L.indptr, L.a_col, L.a_val, kids.coff, kids.children};
-            tri_gen_init_kernel<<<gw, 256, 0, b>>>(R, L.row_comp, L.ckind, L.indptr, L.a_col, L.a_val, L.row_off,
-                                                   L.row_len, L.p_col, dcn, any, L.gflags, L.cbad, L.cell);
-            tri_gen_search_kernel<false><<<grid_for(R * 32, 32 * TRI_SEARCH_WARPS), 32 * TRI_SEARCH_WARPS, TRI_TAB_SMEM,
-                                           b>>>(R, L.row_comp, L.ckind, L.cbad, L.dc, G, L.row_off, L.row_len, L.p_col,
-                                                dcn, any, L.gflags, L.cell, L.ovf, TRI_TAB, L.cam, L.cprod);
-            tri_gen_search_kernel<true><<<4 * sm_count(), 32, tri_dense_smem(sh.max_n), b>>>(
-                R, L.row_comp, L.ckind, L.cbad, L.dc, G, L.row_off, L.row_len, L.p_col, dcn, any, L.gflags, L.cell,
-                L.ovf, sh.max_n, L.cam, L.cprod);
-            tri_gen_first_kernel<<<gw, 256, 0, b>>>(R, L.row_comp, L.ckind, L.cbad, L.row_off, L.row_len, dcn, any,
-                                                    L.gflags, L.cell, L.cfm);
+            const TriGraphView G{L.indptr, nullptr, L.a_col, L.a_val, kids.coff, nullptr, kids.children};
+            tri_searches(sh, L, G, dcn, b);
             RBG_CUDA_TRY(cudaGetLastError());
             return (int)RBG_OK;
         };
@@ -1310,7 +1451,6 @@ template <typename T> struct TriCall {
     uint32_t mode;
     cudaStream_t s;
     const RowStats &rs;
-    const int64_t *orig;                     // the matrices' numbers in the caller's batch (null: as they are)
     TriShape sh;
     TriLayout L;
     std::vector<unsigned char> head;         // the head of the layout in its starting state
@@ -1340,7 +1480,7 @@ template <typename T> struct TriCall {
         int64_t row = 0, cta = 0;
         for (int64_t i = 0; i < count; ++i) {
             const int64_t n = rows(i);
-            H.dc[i] = TriComp{n, in_off[i], out_off[i], row, orig ? orig[i] : i};
+            H.dc[i] = TriComp{n, in_off[i], out_off[i], row};
             H.dpre[i] = cta;
             H.cam[i] = H.cfm[i] = -1;
             row += n;
@@ -1417,49 +1557,69 @@ template <typename T> int tri_levels(TriCall<T> &c) {
     return RBG_OK;
 }
 
-// Short closures: scan, one closure kernel, write.
-template <typename T> int tri_short(TriCall<T> &c) {
-    if (!c.layout(true)) return RBG_OK;
-    int rc = c.upload();
-    if (rc) return rc;
+// Short closures, first pass: scan, closure kernel, write.  Second pass, over the same scratch, for
+// the matrices the first one left pending: their order, closure kernel, searches, write.
+template <typename T> int tri_short(TriCall<T> &c, bool second) {
+    if (!second) {
+        if (!c.layout(true)) return RBG_OK;
+        const int rc = c.upload();
+        if (rc) return rc;
+    }
     const TriLayout &L = c.L;
     const int count = (int)c.count;
-    note_launches(3);
-    {
-        cudaEvent_t t = timer_begin(4, c.s);
-        tri_scan_kernel<T><<<(unsigned)c.sh.ctas, TRI_THREADS, 0, c.s>>>(c.in, c.ld_in, L.dc, L.dpre, count, L.slot_col,
-                                                                        L.slot_val, L.row_cnt, L.row_comp, L.cflags,
-                                                                        L.state);
-        timer_end(4, t, c.s);
+    cudaStream_t s = c.s;
+    note_launches(second ? 3 + TRI_GEN_LAUNCHES : 3);
+    if (!second) {
+        cudaEvent_t t = timer_begin(4, s);
+        tri_scan_kernel<T><<<(unsigned)c.sh.ctas, TRI_THREADS, 0, s>>>(c.in, c.ld_in, L.dc, L.dpre, count, L.slot_col,
+                                                                      L.slot_val, L.row_cnt, L.row_comp, L.cflags,
+                                                                      L.state);
+        timer_end(4, t, s);
     }
     {
-        cudaEvent_t t = timer_begin(5, c.s);
+        cudaEvent_t t = timer_begin(5, s);
+        if (second)
+            tri_order_kernel<<<(unsigned)count, TRI_ORDER_THREADS, sizeof(TriOrderSmem), s>>>(
+                L.dc, L.ckind, L.slot_col, L.row_cnt, L.order, L.coff, L.kid_cnt, L.children, L.cbad, L.ticket,
+                L.gflags + 1);
         const int64_t need = (c.sh.R + TRI_PULL_WARPS - 1) / TRI_PULL_WARPS, most = (int64_t)TRI_PULL_CTAS * sm_count();
-        tri_pull_kernel<<<(unsigned)std::min<int64_t>(need, most), 32 * TRI_PULL_WARPS, 0, c.s>>>(
+        tri_pull_kernel<<<(unsigned)std::min<int64_t>(need, most), 32 * TRI_PULL_WARPS, 0, s>>>(
             c.sh.R, L.row_comp, L.dc, L.cflags, L.slot_col, L.slot_val, L.row_cnt, L.state, L.row_off, L.row_len, L.p_col,
-            L.p_val, L.pool, L.counters, L.ticket, L.ckind, L.cam, L.cfm, L.cprod);
-        timer_end(5, t, c.s);
+            L.p_val, L.pool, L.counters, L.ticket, L.ckind, L.cam, L.cfm, L.cprod, second ? L.order : nullptr, L.cbad);
+        timer_end(5, t, s);
+    }
+    if (second) {
+        cudaEvent_t t = timer_begin(8, s);
+        RBG_CUDA_TRY(cudaMemsetAsync(L.ovf, 0, 4, s));
+        const TriGraphView G{nullptr, L.row_cnt, L.slot_col, L.slot_val, L.coff, L.kid_cnt, L.children};
+        tri_searches(c.sh, L, G, L.counters, s);
+        timer_end(8, t, s);
     }
     {
-        cudaEvent_t t = timer_begin(7, c.s);
-        tri_write_kernel<T><<<(unsigned)c.sh.ctas, TRI_THREADS, 0, c.s>>>(c.in, c.ld_in, c.out, c.ld_out, L.dc, L.dpre,
-                                                                         count, L.ckind, L.cam, L.cbad, L.counters,
-                                                                         L.gflags, L.row_off, L.row_len, L.p_col,
-                                                                         L.p_val, c.rs, L.cfm, L.cprod, L.res);
-        timer_end(7, t, c.s);
+        cudaEvent_t t = timer_begin(7, s);
+        tri_write_kernel<T><<<(unsigned)c.sh.ctas, TRI_THREADS, 0, s>>>(c.in, c.ld_in, c.out, c.ld_out, L.dc, L.dpre,
+                                                                       count, L.ckind, L.cam, L.cbad, L.counters,
+                                                                       L.gflags, L.row_off, L.row_len, L.p_col,
+                                                                       L.p_val, c.rs, L.cfm, L.cprod, L.res);
+        timer_end(7, t, s);
     }
     RBG_CUDA_TRY(cudaGetLastError());
     return c.read(L.counters, nullptr);
 }
 
-template <typename T> void tri_take_results(const TriCall<T> &c, const int64_t *idx, rbg_result_t *results, char *closed) {
-    if (c.res.empty() || (c.hd.flags & TRI_DAG_BAD)) return;     // nothing of the DAG path is used
+// The call's results; `pending`: only of matrices marked so.  Returns how many stay pending.
+template <typename T>
+int64_t tri_take_results(const TriCall<T> &c, bool pending, rbg_result_t *results, char *closed) {
+    int64_t left = 0;
     for (int64_t i = 0; i < c.count; ++i) {
-        const int64_t o = idx ? idx[i] : i;
+        if (pending && closed[i] != (char)TRI_PENDING) continue;
+        closed[i] = TRI_OPEN;
+        if (c.res.empty() || (c.hd.flags & TRI_DAG_BAD)) continue;   // nothing of the DAG path is used
         const TriOut &h = c.res[(size_t)i];
-        closed[o] = (char)h.verdict;
+        closed[i] = (char)h.verdict;
+        left += h.verdict == TRI_PENDING;
         if (h.verdict != TRI_CLOSED) continue;
-        rbg_result_t &r = results[o];
+        rbg_result_t &r = results[i];
         r.status = RBG_OK;
         r.flags = 0;
         r.diameter = h.diameter;
@@ -1467,6 +1627,7 @@ template <typename T> void tri_take_results(const TriCall<T> &c, const int64_t *
         r.path = RBG_PATH_DAG;
         r.executed = (int64_t)h.executed;
     }
+    return left;
 }
 
 }  // namespace
@@ -1480,32 +1641,17 @@ int tri_batch(int64_t count, const int64_t *sizes, const int64_t *in_off, const 
         const int rc = tri_configure();     // before any capture: kernel attributes per device
         if (rc) return rc;
     }
-    TriCall<T> c{count, sizes, in_off, out_off, ld_in, ld_out, in, out, ws, ws_bytes, mode, s, rs, nullptr};
+    TriCall<T> c{count, sizes, in_off, out_off, ld_in, ld_out, in, out, ws, ws_bytes, mode, s, rs};
     if (!c.shape()) return RBG_OK;
-    if (c.sh.R > TRI_PULL_ROWS) {
-        const int rc = tri_levels(c);
-        if (!rc) tri_take_results(c, nullptr, results, closed);
-        return rc;
-    }
-    int rc = tri_short(c);
+    // up to TRI_PULL_ROWS rows the levels' launches cost more than the rows: warps that wait for
+    // their parents.  Beyond, waiting warps would fill the GPU (rows of one family are neighbours)
+    // and the levels, each as wide as the batch, are faster.
+    const bool is_short = c.sh.R <= TRI_PULL_ROWS;
+    int rc = is_short ? tri_short(c, false) : tri_levels(c);
     if (rc) return rc;
-    tri_take_results(c, nullptr, results, closed);
-    // the matrices in any numbering, or all of them when the short closure gave up, by levels
-    std::vector<int64_t> idx, sz, io, oo;
-    for (int64_t i = 0; i < count; ++i) {
-        if (c.res.empty() || (c.hd.flags & TRI_DAG_BAD) || closed[i] != (char)TRI_PENDING) continue;
-        closed[i] = TRI_OPEN;
-        idx.push_back(i);
-        sz.push_back(sizes[i]);
-        io.push_back(in_off[i]);
-        oo.push_back(out_off[i]);
-    }
-    if (idx.empty()) return RBG_OK;
-    TriCall<T> g{(int64_t)idx.size(), sz.data(), io.data(), oo.data(), ld_in, ld_out, in, out, ws, ws_bytes, mode, s, rs,
-                 idx.data()};
-    if (!g.shape()) return RBG_OK;
-    rc = tri_levels(g);
-    if (!rc) tri_take_results(g, idx.data(), results, closed);
+    if (tri_take_results(c, false, results, closed) == 0) return RBG_OK;
+    rc = tri_short(c, true);
+    if (!rc) tri_take_results(c, true, results, closed);
     return rc;
 }
 

@@ -5,58 +5,76 @@
 // order) minimising a[j] + b[j] over the j where both are non-zero; the host turns the two
 // values found there into the relationship name (lookup_relationship, :23-51).
 //
-// One warp per query: the lanes stride the two rows with coalesced loads, keep their best
-// (sum, j) pair, and a shuffle reduction picks the smallest sum, ties to the smallest j.  The
-// sum wraps in the matrix's own type, as numpy scalar arithmetic does on the reference's rows
-// (for unsigned types the red one, the type's maximum, plus y gives y - 1); the reduction
-// carries it widened to 128 bits, which keeps the type's order.
+// One CTA of 128 threads per query: the threads stride the two rows with 16-byte loads where both
+// rows allow it (a warp per query with 4-byte loads took 28 us for 256 queries on n = 4096
+// closures; LOOKUPTIME), keep the smallest (sum, j) and meet in a shuffle and shared-memory
+// reduction: the smallest sum, ties to the smallest j.  The sum wraps in the matrix's own type, as
+// numpy scalar arithmetic does on the reference's rows (for unsigned types the red one, the type's
+// maximum, plus y gives y - 1).  Types of up to 4 bytes pack (sum in the type's order, j) into one
+// 64-bit key; 8-byte types carry the two words.
 #include <cuda_runtime.h>
 #include <type_traits>
 #include "rbg_internal.cuh"
 
 namespace rbg {
 
-constexpr int RL_WARPS = 8;
+constexpr int RL_THREADS = 128;
+
+// the smallest (sum, j) seen: sum as an unsigned word in the type's order, j < 0 for none
+struct RlBest {
+    unsigned long long sum;
+    int64_t j;
+};
+__device__ __forceinline__ bool rl_less(const RlBest &a, const RlBest &b) {   // a before b; none is last
+    if (a.j < 0 || b.j < 0) return a.j >= 0 && b.j < 0;
+    return a.sum < b.sum || (a.sum == b.sum && a.j < b.j);
+}
 
 template <class T>
-__device__ __forceinline__ void rl_scan(const T *a, const T *b, int64_t n, int lane, __int128 &best,
-                                        int64_t &bj, int64_t &bx, int64_t &by) {
+__device__ __forceinline__ void rl_take(T x, T y, int64_t j, RlBest &best) {
     using UT = typename std::make_unsigned<T>::type;
-    for (int64_t j = lane; j < n; j += 32) {
-        const T x = a[j], y = b[j];
-        if (x != 0 && y != 0) {
-            const __int128 s = (__int128)(T)(UT)((UT)x + (UT)y);
-            if (bj < 0 || s < best) {   // lanes visit j in increasing order: first minimum kept
-                best = s;
-                bj = j;
-                bx = (int64_t)x;
-                by = (int64_t)y;
-            }
-        }
+    if (x == 0 || y == 0) return;
+    UT s = (UT)((UT)x + (UT)y);
+    if (std::is_signed<T>::value) s ^= (UT)1 << (sizeof(T) * 8 - 1);   // signed order as unsigned order
+    if (best.j < 0 || (unsigned long long)s < best.sum) {              // j ascends: the first minimum is kept
+        best.sum = (unsigned long long)s;
+        best.j = j;
     }
 }
 
-__device__ __forceinline__ __int128 shfl128(__int128 v, int src) {
-    const unsigned long long lo = (unsigned long long)v, hi = (unsigned long long)(v >> 64);
-    const unsigned long long l2 = __shfl_sync(0xffffffffu, lo, src);
-    const unsigned long long h2 = __shfl_sync(0xffffffffu, hi, src);
-    return (__int128)(((unsigned __int128)h2 << 64) | l2);
+template <class T>
+__device__ __forceinline__ RlBest rl_scan(const T *__restrict__ a, const T *__restrict__ b, int64_t n) {
+    constexpr int E = 16 / (int)sizeof(T);
+    RlBest best{0, -1};
+    int64_t done = 0;
+    if ((((uintptr_t)a | (uintptr_t)b) & 15) == 0) {
+        const int64_t nv = n / E;
+        for (int64_t q = threadIdx.x; q < nv; q += RL_THREADS) {
+            const uint4 x4 = reinterpret_cast<const uint4 *>(a)[q], y4 = reinterpret_cast<const uint4 *>(b)[q];
+            if ((x4.x | x4.y | x4.z | x4.w) == 0 || (y4.x | y4.y | y4.z | y4.w) == 0) continue;
+            const T *x = reinterpret_cast<const T *>(&x4), *y = reinterpret_cast<const T *>(&y4);
+#pragma unroll
+            for (int k = 0; k < E; ++k) rl_take<T>(x[k], y[k], q * E + k, best);
+        }
+        done = nv * E;
+    }
+    for (int64_t j = done + threadIdx.x; j < n; j += RL_THREADS) rl_take<T>(a[j], b[j], j, best);
+    return best;
 }
 
-__global__ void rl_kernel(int64_t count, const rbg_lookup_t *q, int64_t *out) {
-    const int lane = threadIdx.x & 31;
-    const int64_t warps = (int64_t)gridDim.x * RL_WARPS;
-    for (int64_t i = (int64_t)blockIdx.x * RL_WARPS + (threadIdx.x >> 5); i < count; i += warps) {
+__global__ void __launch_bounds__(RL_THREADS) rl_kernel(int64_t count, const rbg_lookup_t *q, int64_t *out) {
+    __shared__ RlBest s_best[RL_THREADS / 32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int64_t i = blockIdx.x; i < count; i += gridDim.x) {
         const rbg_lookup_t Q = q[i];
-        __int128 best = 0;
-        int64_t bj = -1, bx = 0, by = 0;
+        RlBest best{0, -1};
         const bool ok = Q.n > 0 && Q.u >= 0 && Q.u < Q.rows && Q.v >= 0 && Q.v < Q.rows && Q.ld >= Q.n;
-        if (ok) {
+        if (ok) {                            // block-uniform
             switch (Q.dtype) {
 #define RL_CASE(code, T)                                                                           \
     case code: {                                                                                   \
         const T *W = reinterpret_cast<const T *>(Q.W);                                             \
-        rl_scan<T>(W + Q.u * Q.ld, W + Q.v * Q.ld, Q.n, lane, best, bj, bx, by);                   \
+        best = rl_scan<T>(W + Q.u * Q.ld, W + Q.v * Q.ld, Q.n);                                    \
     } break;
                 RL_CASE(RBG_DTYPE_INT8, int8_t)
                 RL_CASE(RBG_DTYPE_UINT8, uint8_t)
@@ -70,20 +88,41 @@ __global__ void rl_kernel(int64_t count, const rbg_lookup_t *q, int64_t *out) {
                 default: break;
             }
         }
-        // reduce (best, j): smallest sum, then smallest j; lanes without a candidate have j < 0
         for (int o = 16; o > 0; o >>= 1) {
-            const __int128 ob = shfl128(best, lane ^ o);
-            const int64_t oj = __shfl_xor_sync(0xffffffffu, bj, o);
-            const int64_t ox = __shfl_xor_sync(0xffffffffu, bx, o);
-            const int64_t oy = __shfl_xor_sync(0xffffffffu, by, o);
-            const bool take = oj >= 0 && (bj < 0 || ob < best || (ob == best && oj < bj));
-            if (take) { best = ob; bj = oj; bx = ox; by = oy; }
+            const RlBest other{__shfl_xor_sync(0xffffffffu, best.sum, o), __shfl_xor_sync(0xffffffffu, best.j, o)};
+            if (rl_less(other, best)) best = other;
         }
-        if (lane == 0) {
-            out[3 * i] = ok ? bj : -2;
+        if (lane == 0) s_best[w] = best;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int k = 1; k < RL_THREADS / 32; ++k)
+                if (rl_less(s_best[k], best)) best = s_best[k];
+            int64_t bx = 0, by = 0;
+            if (best.j >= 0) {
+                switch (Q.dtype) {
+#define RL_CASE(code, T)                                                                           \
+    case code: {                                                                                   \
+        const T *W = reinterpret_cast<const T *>(Q.W);                                             \
+        bx = (int64_t)W[Q.u * Q.ld + best.j];                                                      \
+        by = (int64_t)W[Q.v * Q.ld + best.j];                                                      \
+    } break;
+                    RL_CASE(RBG_DTYPE_INT8, int8_t)
+                    RL_CASE(RBG_DTYPE_UINT8, uint8_t)
+                    RL_CASE(RBG_DTYPE_INT16, int16_t)
+                    RL_CASE(RBG_DTYPE_UINT16, uint16_t)
+                    RL_CASE(RBG_DTYPE_INT32, int32_t)
+                    RL_CASE(RBG_DTYPE_UINT32, uint32_t)
+                    RL_CASE(RBG_DTYPE_INT64, int64_t)
+                    RL_CASE(RBG_DTYPE_UINT64, uint64_t)
+#undef RL_CASE
+                    default: break;
+                }
+            }
+            out[3 * i] = ok ? best.j : -2;
             out[3 * i + 1] = bx;
             out[3 * i + 2] = by;
         }
+        __syncthreads();                     // s_best is written again for the next query
     }
 }
 
@@ -97,7 +136,7 @@ extern "C" int32_t rbg_relationship_lookup(int64_t count, const rbg_lookup_t *qu
     if (count == 0) return RBG_OK;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     note_launches(1);
-    rl_kernel<<<grid_for(count * 32, RL_WARPS * 32), RL_WARPS * 32, 0, s>>>(count, queries, out);
+    rl_kernel<<<grid_for(count, 1), RL_THREADS, 0, s>>>(count, queries, out);
     RBG_CUDA_TRY(cudaGetLastError());
     return RBG_OK;
 }

@@ -6,7 +6,7 @@ for two rows of a transitive closure the common ancestor is the first index mini
 comes from the generational distances MSB(a[j]) and MSB(b[j]) (lookup_relationship,
 :23-51).  The sums wrap in the rows' dtype, as the numpy scalars of the reference's rows do
 (the unsigned red one, the dtype's maximum, plus y gives y - 1).  The search runs in
-``rbg_relationship_lookup`` (one warp per query); ``lookup_many`` answers a whole batch of
+``rbg_relationship_lookup`` (one CTA per query); ``lookup_many`` answers a whole batch of
 (matrix, u, v) queries on resident device matrices in one launch.
 """
 from __future__ import annotations
@@ -62,17 +62,25 @@ def relationship_name(da: int, db: int) -> str:
 
 def decode(out: np.ndarray, dtypes) -> list[Relationship]:
     """Relationships from the raw (count, 3) lookup results and each query's matrix dtype."""
+    x, y = out[:, 1].tolist(), out[:, 2].tolist()
+    dtypes = list(dtypes)
+    if any(np.dtype(dt).kind == "u" for dt in set(dtypes)):   # the raw results hold the values' bits
+        mask = [0xFFFFFFFFFFFFFFFF if np.dtype(dt).kind == "u" else -1 for dt in dtypes]
+        x, y = [a & m for a, m in zip(x, mask)], [b & m for b, m in zip(y, mask)]
+    # the two MSBs (msb() in line)
+    keys = [((a.bit_length() - 1 if a > 1 else 0), (b.bit_length() - 1 if b > 1 else 0)) for a, b in zip(x, y)]
+    names: dict = {}
     res = []
-    for k, dt in enumerate(dtypes):
-        j = int(out[k, 0])
-        if j == -2:
+    for j, key in zip(out[:, 0].tolist(), keys):
+        if j >= 0:
+            name = names.get(key)
+            if name is None:
+                name = names[key] = relationship_name(*key)
+            res.append(Relationship(j, name))
+        elif j == -2:
             raise IndexError("relationship query out of range")
-        if j < 0:
+        else:
             res.append(Relationship(-1, "No Relationship"))
-            continue
-        bits = out[k, 1:3].astype(np.int64)
-        x, y = (bits.view(np.uint64) if np.dtype(dt).kind == "u" else bits).astype(object)
-        res.append(Relationship(j, relationship_name(msb(x), msb(y))))
     return res
 
 
@@ -86,6 +94,9 @@ def lookup_table(table_dev: torch.Tensor, count: int, stream=None) -> np.ndarray
     return out[:count].cpu().numpy()
 
 
+_LOOKUP_DTYPE = np.dtype(_lib.RbgLookup)     # rbg_lookup_t
+
+
 def lookup_many(queries, stream=None) -> list[Relationship]:
     """Answer many queries ``(W, u, v)`` (W a 2-D device tensor with contiguous rows, u and v two
     of its row indices) with one kernel launch."""
@@ -93,19 +104,29 @@ def lookup_many(queries, stream=None) -> list[Relationship]:
     if not queries:
         return []
     dev = queries[0][0].device
-    table = (_lib.RbgLookup * len(queries))()
-    dtypes = []
-    for k, (W, u, v) in enumerate(queries):
-        if W.ndim != 2 or not W.is_cuda or (W.shape[1] > 1 and W.stride(1) != 1):
-            raise ValueError("queries take 2-D CUDA matrices with contiguous rows")
-        if not (0 <= int(u) < W.shape[0] and 0 <= int(v) < W.shape[0]):
-            raise IndexError(f"vertices ({u}, {v}) outside a matrix of {W.shape[0]} rows")
-        dt = numpy_dtype(W.dtype)
-        dtypes.append(dt)
-        table[k] = _lib.RbgLookup(W.data_ptr(), W.stride(0), W.shape[0], W.shape[1], int(u), int(v),
-                                  _lib.dtype_code(dt), 0)
-    raw = np.frombuffer(table, dtype=np.uint8).copy()
-    return decode(lookup_table(to_device(raw, dev), len(queries), stream), dtypes)
+    # the fields of each distinct matrix once (`queries` holds the tensors), the vertices as columns
+    mats, dts, seen = [], [], {}
+    which, us, vs = [], [], []
+    for W, u, v in queries:
+        k = seen.get(id(W))
+        if k is None:
+            if W.ndim != 2 or not W.is_cuda or (W.shape[1] > 1 and W.stride(1) != 1):
+                raise ValueError("queries take 2-D CUDA matrices with contiguous rows")
+            dt = numpy_dtype(W.dtype)
+            k = seen[id(W)] = len(mats)
+            mats.append((W.data_ptr(), W.stride(0), W.shape[0], W.shape[1], 0, 0, _lib.dtype_code(dt), 0))
+            dts.append(dt)
+        rows, u, v = mats[k][2], int(u), int(v)
+        if not (0 <= u < rows and 0 <= v < rows):
+            raise IndexError(f"vertices ({u}, {v}) outside a matrix of {rows} rows")
+        which.append(k)
+        us.append(u)
+        vs.append(v)
+    table = np.array(mats, dtype=_LOOKUP_DTYPE)[which]
+    table["u"] = us
+    table["v"] = vs
+    return decode(lookup_table(to_device(table.view(np.uint8), dev), len(queries), stream),
+                  [dts[k] for k in which])
 
 
 def calculate_relationship(a: Sequence[int], b: Sequence[int]) -> Relationship:

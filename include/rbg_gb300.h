@@ -362,6 +362,16 @@ int32_t rbg_dag_closure(const rbg_csr_t *A, void *workspace, int64_t workspace_b
 /* Scratch bytes rbg_dag_gather needs. */
 int32_t rbg_dag_gather_workspace_bytes(int64_t n, int64_t *bytes);
 
+/* rbg_dag_closure with mode bits.  Without them, pieces of up to 64 consecutive vertices that no edge
+ * leaves (the families of a forest) are closed on their own first, and only the rest by levels.
+ * RBG_DAG_NO_TILES skips that look for pieces: for callers that know most vertices lie in larger
+ * ones (a few passes over A saved).  The closure, *max_abs and *levels are the same. */
+#define RBG_DAG_NO_TILES 1u
+int32_t rbg_dag_closure_mode(const rbg_csr_t *A, uint32_t mode, void *workspace, int64_t workspace_bytes,
+                             int32_t *pool_cols, int32_t *pool_vals, int64_t pool_capacity, int64_t *row_off,
+                             int32_t *row_len, int64_t *nnz, int64_t *max_abs, int64_t *levels,
+                             rbg_stream_t stream);
+
 /* The pooled rows of rbg_dag_closure as CSR: indptr (n + 1, int64), indices and data (int32).
  * Ordered on `stream`. */
 int32_t rbg_dag_gather(int64_t n, const int32_t *pool_cols, const int32_t *pool_vals, const int64_t *row_off,

@@ -39,6 +39,8 @@ MODE_TILE_NARROW = 32
 MODE_AUTOTUNE = 64
 MODE_NO_DAG = 128
 
+DAG_NO_TILES = 1
+
 PATH_BLOCKED32, PATH_BLOCKED64, PATH_EXACT, PATH_DAG = 1, 2, 3, 4
 
 NOALLOC_MAX_N = 1024   # include/rbg_gb300.h RBG_NOALLOC_MAX_N
@@ -148,6 +150,8 @@ SIGNATURES = [
     ("rbg_dag_workspace_bytes", _I32, [_I64, _I64, ctypes.POINTER(_I64)]),
     ("rbg_dag_closure", _I32, [ctypes.POINTER(RbgCsr), _P, _I64, _P, _P, _I64, _P, _P, ctypes.POINTER(_I64),
                                ctypes.POINTER(_I64), ctypes.POINTER(_I64), _P]),
+    ("rbg_dag_closure_mode", _I32, [ctypes.POINTER(RbgCsr), ctypes.c_uint32, _P, _I64, _P, _P, _I64, _P, _P,
+                                    ctypes.POINTER(_I64), ctypes.POINTER(_I64), ctypes.POINTER(_I64), _P]),
     ("rbg_dag_gather_workspace_bytes", _I32, [_I64, ctypes.POINTER(_I64)]),
     ("rbg_dag_gather", _I32, [_I64, _P, _P, _P, _P, _P, _I64, _P, _P, _P, _P]),
     ("rbg_dag_candidate_max", _I32, [ctypes.POINTER(RbgCsr), ctypes.POINTER(RbgCsr), _P, _I64,

@@ -146,6 +146,7 @@ def _msb(v: int) -> int:
 
 
 DAG_MAX_N = 8192          # rows of a component the DAG path takes (include/rbg_gb300.h)
+DAG_TILE_ROWS = 64        # vertices of a piece closed without levels (rbg_dag_closure_mode)
 _UNCLEAN, _BELOW, _ABOVE = 1, 2, 4
 
 
@@ -184,8 +185,12 @@ def dag_component_closure(indptr: torch.Tensor, indices: torch.Tensor, data: tor
     _lib.check(L.rbg_cc_dag_edges(n, ip, ij, iv, eptr.data_ptr(), ecol.data_ptr(), evals.data_ptr(), sh),
                "cc_dag_edges")
     E = DeviceCSR(eptr, ecol[:ne.value], evals[:ne.value], (n, n))
+    # the look for small pieces pays when half of the vertices lie in components a tile can hold (a
+    # forest of 2,000,000 vertices in families of 64: 3.15 to 0.92 ms; one of 300 pedigrees of up to
+    # 4096 vertices: 2.01 to 2.12 ms with it)
+    tiles = 2 * int(comps.sizes[comps.sizes <= DAG_TILE_ROWS].sum()) >= n
     try:
-        C, _, _ = dag_closure_device(E, stream, gather=False)    # the row pool, read in place
+        C, _, _ = dag_closure_device(E, stream, gather=False, tiles=tiles)    # the row pool, read in place
     except RowTooWide:
         return None
     top = torch.empty(k, dtype=torch.int32, device=dev)

@@ -237,12 +237,15 @@ struct CcWs {
 };
 
 size_t cc_tmp_bytes(int64_t n) {
-    const int m = (int)std::max<int64_t>(n + 1, 1);
-    size_t a = 0, b = 0, c = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, a, (int *)nullptr, (int *)nullptr, m);
-    cub::DeviceScan::ExclusiveSum(nullptr, b, (int64_t *)nullptr, (int64_t *)nullptr, m);
-    cub::DeviceRadixSort::SortPairs(nullptr, c, (int *)nullptr, (int *)nullptr, (int *)nullptr, (int *)nullptr, m);
-    return std::max(a, std::max(b, c));
+    static thread_local LastSize last;
+    return last.get(n, [n] {
+        const int m = (int)std::max<int64_t>(n + 1, 1);
+        size_t a = 0, b = 0, c = 0;
+        cub::DeviceScan::ExclusiveSum(nullptr, a, (int *)nullptr, (int *)nullptr, m);
+        cub::DeviceScan::ExclusiveSum(nullptr, b, (int64_t *)nullptr, (int64_t *)nullptr, m);
+        cub::DeviceRadixSort::SortPairs(nullptr, c, (int *)nullptr, (int *)nullptr, (int *)nullptr, (int *)nullptr, m);
+        return std::max(a, std::max(b, c));
+    });
 }
 
 size_t cc_layout(int64_t n, unsigned char *base, CcWs *w) {

@@ -6,7 +6,9 @@
 // (+) A[v][w] (x) C[w][.] over v's parents w != v, with the Cython int32 product and sum; the
 // diameter source is the largest magnitude of any stored entry or candidate.
 //
-// Design.  Vertices are put in topological levels on the device (Kahn's algorithm): a vertex
+// Design.  Pieces of a few consecutive vertices that no edge leaves (the families of a forest) are
+// closed first, a warp per tile of them with its rows in shared memory (the tiles, below).  The
+// other vertices are put in topological levels on the device (Kahn's algorithm): a vertex
 // joins the next level when its last parent's row is done.  The kernel that discovers a vertex
 // also bounds its row (stored entries + the lengths of its parents' rows) and reserves that many
 // slots of a caller-provided row pool (one atomic per warp), so each level then needs a single
@@ -435,8 +437,15 @@ __device__ __forceinline__ long long dag_bound(const DagArgs &a, int c, int64_t 
     return ub;
 }
 
-__global__ void dag_indeg_kernel(int64_t n, const int64_t *ap, const int *aj, int *remaining, int *ccount) {
+// Rows that are closed already (row_len >= 0: by a tile) stay out of the levels; no edge joins them
+// to the others.
+__global__ void dag_indeg_kernel(int64_t n, const int64_t *ap, const int *aj, const int *row_len, int *remaining,
+                                 int *ccount) {
     for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
+        if (row_len[v] >= 0) {
+            remaining[v] = -1;
+            continue;
+        }
         int c = 0;
         for (int64_t e = ap[v]; e < ap[v + 1]; ++e) {
             const int w = aj[e];
@@ -449,9 +458,10 @@ __global__ void dag_indeg_kernel(int64_t n, const int64_t *ap, const int *aj, in
     }
 }
 
-__global__ void dag_children_kernel(int64_t n, const int64_t *ap, const int *aj, const int64_t *coff, int *cursor,
-                                    int *children) {
+__global__ void dag_children_kernel(int64_t n, const int64_t *ap, const int *aj, const int *row_len,
+                                    const int64_t *coff, int *cursor, int *children) {
     for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
+        if (row_len[v] >= 0) continue;
         for (int64_t e = ap[v]; e < ap[v + 1]; ++e) {
             const int w = aj[e];
             if (w != (int)v && w >= 0 && w < n) children[coff[w] + atomicAdd(&cursor[w], 1)] = (int)v;
@@ -796,20 +806,235 @@ __global__ void __launch_bounds__(DG_BTHREADS) dag_fill_block_kernel(DagArgs a, 
     if ((threadIdx.x & 31) == 0 && best > 0) atomicMax(a.max_abs, (unsigned long long)best);
 }
 
-// ----------------------------------------------------------------------------- pool -> CSR
-// Eight lanes per row.
-__global__ void dag_gather_rows_kernel(int64_t n, const int64_t *row_off, const int *pcols, const int *pvals,
-                                       const int64_t *indptr, int *cj, int *cx) {
-    const int sub = threadIdx.x & 7;
-    const int64_t groups = (int64_t)gridDim.x * (blockDim.x >> 3);
-    for (int64_t v = (int64_t)blockIdx.x * (blockDim.x >> 3) + (threadIdx.x >> 3); v < n; v += groups) {
-        const int64_t dst = indptr[v], len = indptr[v + 1] - dst;
-        if (len == 0) continue;
-        const int64_t src = row_off[v];
-        for (int64_t e = sub; e < len; e += 8) {
-            cj[dst + e] = pcols[src + e];
-            cx[dst + e] = pvals[src + e];
+// ----------------------------------------------------------------------------- tiles
+// A forest stored family by family falls apart at the positions no edge crosses.  Pieces of up to
+// DT_ROWS consecutive vertices whose entries all lie on one side of the diagonal need no levels: a
+// warp closes them row by row in their own order, the closed rows kept dense in shared memory
+// (packed: row l holds columns below l), two columns per lane in registers.  Pieces next to each
+// other share a tile while they fit.  Values are plain ones (2 .. 2^31 - 1, products below bit 31;
+// the diagonal -1 or 1): there a row is the minimum over its entries and over each parent's row
+// times the entry, and the parent's diagonal adds nothing to it.  Anything else, and every larger
+// piece, is left to the levels (row_len stays -1).
+//
+// Bound by issue and by the chain of a warp's rows.  A forest of 2,000,000 vertices in families of 64
+// takes 0.92 ms with its pool gathered into a CSR, 3.15 ms by levels; 20,011 vertices 163 us, 887 us
+// by levels.
+constexpr int DT_ROWS = 64;
+constexpr int DT_WARPS = 4;             // warps (tiles) per CTA
+constexpr int DT_ENTRIES = 384;         // stored entries a tile may hold
+constexpr int DT_NONE = 0x7fffffff;
+struct DagTile {
+    int cell[DT_ROWS * (DT_ROWS - 1) / 2];   // row l, column c < l: cell[l (l - 1) / 2 + c]; 0: none
+    int val[DT_ENTRIES];
+    unsigned char col[DT_ENTRIES];
+    unsigned short ptr[DT_ROWS + 1];
+    unsigned char len[DT_ROWS], level[DT_ROWS];
+    signed char diag[DT_ROWS];               // the stored diagonal, 0 if none
+};
+
+// furthest[p]: the largest end of the edges (and vertices) whose lower end is p
+__global__ void dag_span_kernel(int64_t n, const int64_t *ap, const int *aj, int *furthest) {
+    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
+        int lo = (int)v, hi = (int)v;
+        for (int64_t e = ap[v]; e < ap[v + 1]; ++e) {
+            const int w = aj[e];
+            if (w >= 0 && w < n) {
+                lo = min(lo, w);
+                hi = max(hi, w);
+            }
         }
+        atomicMax(furthest + lo, hi);
+    }
+}
+
+// The tile [p, p + len): returns whether it was closed.
+__device__ __forceinline__ bool dag_tile(const DagArgs &a, DagTile &S, int64_t p, int len, int lane, int &best,
+                                         unsigned long long &written, int &levels) {
+    const int64_t e0 = a.ap[p], ne64 = a.ap[p + len] - e0;
+    if (ne64 > DT_ENTRIES) return false;                     // warp-uniform
+    const int ne = (int)ne64;
+    __syncwarp();                                            // the previous tile's reads come first
+    for (int q = lane; q <= len; q += 32) S.ptr[q] = (unsigned short)(a.ap[p + q] - e0);
+    // stage the entries; which side of the diagonal they lie on
+    __syncwarp();
+    bool bad = false, below = false, above = false;
+    for (int q = lane; q < ne; q += 32) {
+        int r = 0;                                           // the entry's row
+#pragma unroll
+        for (int st = DT_ROWS / 2; st > 0; st >>= 1)
+            if (r + st < len && S.ptr[r + st] <= q) r += st;
+        const int c = a.aj[e0 + q] - (int)p, v = a.av[e0 + q];
+        const bool diag = c == r;
+        below |= c < r;
+        above |= c > r;
+        bad |= (unsigned)c >= (unsigned)len || (diag ? v != 1 && v != -1 : v < 2);
+        S.col[q] = (unsigned char)c;
+        S.val[q] = v;
+    }
+    below = __any_sync(FULL, below);
+    const bool flip = __any_sync(FULL, above);               // rows from the last to the first
+    if (__any_sync(FULL, bad) || (below && flip)) return false;
+    __syncwarp();
+    int top = -1, most = 0, total = 0;
+    for (int l = 0; l < len; ++l) {
+        const int r = flip ? len - 1 - l : l;
+        const int q1 = S.ptr[r + 1];
+        int x0 = DT_NONE, x1 = DT_NONE, dg = 0, lev = 0;
+        for (int q = S.ptr[r]; q < q1; ++q) {                // warp-uniform
+            const int v = S.val[q], c = flip ? len - 1 - S.col[q] : S.col[q];
+            most = max(most, v < 0 ? 1 : v);
+            if (c == l) {
+                dg = v;
+                continue;
+            }
+            lev = max(lev, S.level[c] + 1);
+            if (lane == c) x0 = min(x0, v);
+            if (lane + 32 == c) x1 = min(x1, v);
+            const int base = c * (c - 1) / 2, mv = 31 - __clz(v);
+            const int y0 = lane < c ? S.cell[base + lane] : 0, y1 = lane + 32 < c ? S.cell[base + lane + 32] : 0;
+            if (y0 != 0) {
+                const int s = 31 - __clz(y0), pr = (v << s) | (y0 ^ (1 << s));
+                top = max(top, mv + s);
+                x0 = min(x0, pr);
+                most = max(most, pr);
+            }
+            if (y1 != 0) {
+                const int s = 31 - __clz(y1), pr = (v << s) | (y1 ^ (1 << s));
+                top = max(top, mv + s);
+                x1 = min(x1, pr);
+                most = max(most, pr);
+            }
+        }
+        const int base = l * (l - 1) / 2;
+        const bool h0 = x0 != DT_NONE, h1 = x1 != DT_NONE;
+        if (lane < l) S.cell[base + lane] = h0 ? x0 : 0;
+        if (lane + 32 < l) S.cell[base + lane + 32] = h1 ? x1 : 0;
+        const int m = __popc(__ballot_sync(FULL, h0)) + __popc(__ballot_sync(FULL, h1)) + (dg != 0);
+        total += m;
+        if (lane == 0) {
+            S.len[l] = (unsigned char)m;
+            S.level[l] = (unsigned char)lev;
+            S.diag[l] = (signed char)dg;
+        }
+        levels = max(levels, lev + 1);
+        __syncwarp();
+    }
+    if (__any_sync(FULL, top >= 31)) return false;           // a product may wrap
+    unsigned long long at = 0;
+    if (lane == 0) at = atomicAdd(a.base, (unsigned long long)total);
+    at = __shfl_sync(FULL, at, 0);
+    const bool room = (int64_t)at + total <= a.capacity;
+    if (!room && lane == 0) atomicOr(a.flags, 1);            // the call asks for a larger pool
+    const unsigned lt = (1u << lane) - 1u;
+    int64_t off = (int64_t)at;
+    for (int r = 0; r < len; ++r) {                          // in vertex order
+        const int l = flip ? len - 1 - r : r, base = l * (l - 1) / 2, m = S.len[l];
+        if (room) {
+            const int x0 = lane < l ? S.cell[base + lane] : 0, x1 = lane + 32 < l ? S.cell[base + lane + 32] : 0;
+            const unsigned b0 = __ballot_sync(FULL, x0 != 0), b1 = __ballot_sync(FULL, x1 != 0);
+            const int k0 = __popc(b0 & lt), k1 = __popc(b0) + __popc(b1 & lt);
+            if (x0 != 0) {
+                const int64_t k = off + (flip ? m - 1 - k0 : k0);
+                a.pcols[k] = (int)p + (flip ? len - 1 - lane : lane);
+                a.pvals[k] = x0;
+            }
+            if (x1 != 0) {
+                const int64_t k = off + (flip ? m - 1 - k1 : k1);
+                a.pcols[k] = (int)p + (flip ? len - 33 - lane : lane + 32);
+                a.pvals[k] = x1;
+            }
+            if (lane == 0 && S.diag[l] != 0) {               // column r: the last one, or the first when flipped
+                const int64_t k = off + (flip ? 0 : m - 1);
+                a.pcols[k] = (int)p + r;
+                a.pvals[k] = S.diag[l];
+            }
+        }
+        if (lane == 0) {
+            a.row_off[p + r] = room ? off : -1;
+            a.row_len[p + r] = room ? m : 0;
+        }
+        off += m;
+    }
+    best = max(best, most);
+    written += (unsigned long long)total;
+    return true;
+}
+
+// One warp per DT_ROWS positions: the pieces that start there.  reach[p]: the furthest end of any
+// edge that starts at or before p, so a piece starts at p when reach[p - 1] < p.
+__global__ void __launch_bounds__(DT_WARPS * 32)
+dag_tile_kernel(DagArgs a, const int *reach, int *tile_rows, int *tile_levels) {
+    extern __shared__ __align__(16) unsigned char dg_smem[];
+    DagTile &S = reinterpret_cast<DagTile *>(dg_smem)[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const int64_t b = ((int64_t)blockIdx.x * DT_WARPS + (threadIdx.x >> 5)) * DT_ROWS;
+    if (b >= a.n) return;
+    auto starts = [&](int64_t first) -> unsigned long long {
+        unsigned long long f = 0;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int64_t q = first + 32 * h + lane;
+            const bool s = q == 0 || (q <= a.n && reach[q - 1] < q);
+            f |= (unsigned long long)__ballot_sync(FULL, s) << (32 * h);
+        }
+        return f;
+    };
+    const unsigned long long f0 = starts(b), f1 = starts(b + DT_ROWS);   // pieces end at the next start, or at n
+    int best = 0, levels = 0, rows = 0;
+    unsigned long long written = 0;
+    int cur = 0;
+    while (cur < DT_ROWS) {                      // warp-uniform
+        const unsigned long long rest = f0 & (~0ull << cur);
+        if (!rest) break;
+        const int s = __ffsll((long long)rest) - 1;
+        if (b + s >= a.n) break;
+        // ends within DT_ROWS of s: the later starts of this chunk, and the first one past it
+        const unsigned long long past = f1 & (0ull - f1);
+        unsigned long long ends = s == 63 ? past : (f0 >> (s + 1)) | (past << (63 - s));
+        if (!ends) {                             // longer than a tile
+            cur = s + 1;
+            continue;
+        }
+        const int len = 64 - __clzll((long long)ends);   // the furthest of them
+        if (dag_tile(a, S, b + s, len, lane, best, written, levels)) rows += len;
+        cur = s + len;
+    }
+    best = __reduce_max_sync(FULL, best);
+    if (lane == 0) {
+        if (best > 0) atomicMax(a.max_abs, (unsigned long long)best);
+        if (written) atomicAdd(a.total, written);
+        if (rows) {
+            atomicAdd(tile_rows, rows);
+            atomicMax(tile_levels, levels);
+        }
+    }
+}
+
+// ----------------------------------------------------------------------------- pool -> CSR
+// Eight lanes per row, four entries each in flight.
+__global__ void dag_gather_rows_kernel(int64_t n, const int64_t *__restrict__ row_off, const int *__restrict__ pcols,
+                                       const int *__restrict__ pvals, const int64_t *__restrict__ indptr,
+                                       int *__restrict__ cj, int *__restrict__ cx) {
+    const int sub = threadIdx.x & 7;
+    const int64_t v = (int64_t)blockIdx.x * (blockDim.x >> 3) + (threadIdx.x >> 3);
+    if (v >= n) return;
+    const int64_t dst = indptr[v], len = indptr[v + 1] - dst;
+    if (len == 0) return;
+    const int64_t src = row_off[v];
+    for (int64_t e = sub; e < len; e += 32) {
+        int c[4], x[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (e + 8 * u < len) {
+                c[u] = pcols[src + e + 8 * u];
+                x[u] = pvals[src + e + 8 * u];
+            }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (e + 8 * u < len) {
+                cj[dst + e + 8 * u] = c[u];
+                cx[dst + e + 8 * u] = x[u];
+            }
     }
 }
 
@@ -843,31 +1068,50 @@ struct DagWs {
     size_t tmp_bytes;
 };
 
+struct IntMax {
+    __host__ __device__ __forceinline__ int operator()(int a, int b) const { return a > b ? a : b; }
+};
+
 size_t dag_tmp_bytes(int64_t n) {
-    size_t a = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, a, (int *)nullptr, (int64_t *)nullptr, (int)std::max<int64_t>(n + 1, 1));
-    return a;
+    static thread_local LastSize last;
+    return last.get(n, [n] {
+        size_t a = 0, b = 0;
+        cub::DeviceScan::ExclusiveSum(nullptr, a, (int *)nullptr, (int64_t *)nullptr, (int)std::max<int64_t>(n + 1, 1));
+        cub::DeviceScan::InclusiveScan(nullptr, b, (int *)nullptr, (int *)nullptr, IntMax(),
+                                       (int)std::max<int64_t>(n, 1));
+        return std::max(a, b);
+    });
 }
 
+size_t gather_tmp_bytes(int64_t n) {
+    static thread_local LastSize last;
+    return last.get(n, [n] {
+        size_t b = 0;
+        cub::DeviceScan::ExclusiveSum(nullptr, b, (int64_t *)nullptr, (int64_t *)nullptr, (int)(n + 1));
+        return b;
+    });
+}
+
+// What depends on nnz comes last: the rest is in place before nnz is known.
 size_t dag_layout(int64_t n, int64_t nnz, unsigned char *base, DagWs *w) {
     size_t o = 0;
     auto take = [&](size_t bytes) { size_t at = o; o = align_up(o + bytes, 256); return base ? base + at : nullptr; };
     const size_t ni = (size_t)(n + 1) * 4, nl = (size_t)(n + 2) * 8;
     unsigned char *p;
+    p = take(sizeof(DagCounters)); if (w) w->cnt = (DagCounters *)p;
     p = take(ni); if (w) w->remaining = (int *)p;
     p = take(ni); if (w) w->ccount = (int *)p;
     p = take(ni); if (w) w->cursor = (int *)p;
-    p = take((size_t)std::max<int64_t>(nnz, 1) * 4); if (w) w->children = (int *)p;
     p = take(ni); if (w) w->order = (int *)p;
     p = take((size_t)(n + 1) * sizeof(DagRec)); if (w) w->rec = (DagRec *)p;
-    p = take((size_t)std::max<int64_t>(nnz, 1) * 8); if (w) w->desc = (unsigned long long *)p;
     p = take(ni); if (w) w->wide = (int *)p;
     p = take(nl); if (w) w->coff = (int64_t *)p;
     p = take(nl); if (w) w->lb = (int64_t *)p;
     p = take(nl); if (w) w->wlb = (int64_t *)p;
-    p = take(sizeof(DagCounters)); if (w) w->cnt = (DagCounters *)p;   // zeroed together
     const size_t tb = dag_tmp_bytes(n);
     p = take(tb); if (w) { w->tmp = p; w->tmp_bytes = tb; }
+    p = take((size_t)std::max<int64_t>(nnz, 1) * 4); if (w) w->children = (int *)p;
+    p = take((size_t)std::max<int64_t>(nnz, 1) * 8); if (w) w->desc = (unsigned long long *)p;
     return o;
 }
 
@@ -879,6 +1123,8 @@ int dag_configure() {
                                           (int)(sizeof(DagTable<DG_WSLOTS>) * DG_WARPS)));
         RBG_CUDA_TRY(cudaFuncSetAttribute(dag_fill_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)sizeof(DagTable<DG_BSLOTS>)));
+        RBG_CUDA_TRY(cudaFuncSetAttribute(dag_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)(sizeof(DagTile) * DT_WARPS)));
         return (int)RBG_OK;
     });
 }
@@ -903,14 +1149,13 @@ int dag_front(const DagArgs &a, const DagWs &w, cudaStream_t s) {
     const int g = grid_for(n, 256);
     RBG_CUDA_TRY(cudaMemsetAsync(w.ccount, 0, (size_t)(n + 1) * 4, s));
     RBG_CUDA_TRY(cudaMemsetAsync(w.cursor, 0, (size_t)(n + 1) * 4, s));
-    RBG_CUDA_TRY(cudaMemsetAsync(w.cnt, 0, sizeof(DagCounters), s));
     RBG_CUDA_TRY(cudaMemsetAsync(w.lb, 0, 8, s));
     RBG_CUDA_TRY(cudaMemsetAsync(w.wlb, 0, 8, s));
     note_launches(4);
-    dag_indeg_kernel<<<g, 256, 0, s>>>(n, a.ap, a.aj, w.remaining, w.ccount);
+    dag_indeg_kernel<<<g, 256, 0, s>>>(n, a.ap, a.aj, a.row_len, w.remaining, w.ccount);
     size_t tb = w.tmp_bytes;
     RBG_CUDA_TRY(cub::DeviceScan::ExclusiveSum(w.tmp, tb, w.ccount, w.coff, (int)(n + 1), s));
-    dag_children_kernel<<<g, 256, 0, s>>>(n, a.ap, a.aj, w.coff, w.cursor, w.children);
+    dag_children_kernel<<<g, 256, 0, s>>>(n, a.ap, a.aj, a.row_len, w.coff, w.cursor, w.children);
     dag_roots_kernel<<<g, 256, 0, s>>>(a);
     RBG_CUDA_TRY(cudaGetLastError());
     return RBG_OK;
@@ -1037,6 +1282,8 @@ int dag_enqueue(const rbg_csr_t *A, int64_t nnz_bound, void *workspace, int32_t 
     int rc = dag_configure();
     if (rc) return rc;
     const DagArgs a = dag_args(n, A, w, pool_cols, pool_vals, pool_capacity, row_off, row_len);
+    RBG_CUDA_TRY(cudaMemsetAsync(w.cnt, 0, sizeof(DagCounters), s));
+    RBG_CUDA_TRY(cudaMemsetAsync(row_len, 0xff, (size_t)n * 4, s));   // -1: not closed (never placed, in the end)
     rc = dag_front(a, w, s);
     if (rc) return rc;
     *launches += 4;
@@ -1055,6 +1302,14 @@ extern "C" int32_t rbg_dag_workspace_bytes(int64_t n, int64_t nnz, int64_t *byte
 extern "C" int32_t rbg_dag_closure(const rbg_csr_t *A, void *workspace, int64_t workspace_bytes, int32_t *pool_cols,
                                    int32_t *pool_vals, int64_t pool_capacity, int64_t *row_off, int32_t *row_len,
                                    int64_t *nnz, int64_t *max_abs, int64_t *levels, rbg_stream_t stream) {
+    return rbg_dag_closure_mode(A, 0, workspace, workspace_bytes, pool_cols, pool_vals, pool_capacity, row_off, row_len,
+                                nnz, max_abs, levels, stream);
+}
+
+extern "C" int32_t rbg_dag_closure_mode(const rbg_csr_t *A, uint32_t mode, void *workspace, int64_t workspace_bytes,
+                                        int32_t *pool_cols, int32_t *pool_vals, int64_t pool_capacity,
+                                        int64_t *row_off, int32_t *row_len, int64_t *nnz, int64_t *max_abs,
+                                        int64_t *levels, rbg_stream_t stream) {
     if (!A || !A->indptr || A->n_rows != A->n_cols || A->n_rows < 0 || !workspace || !row_off || !row_len ||
         !nnz || !max_abs || !levels || pool_capacity < 0 || (pool_capacity > 0 && (!pool_cols || !pool_vals)))
         return RBG_ERR_INVALID;
@@ -1063,28 +1318,50 @@ extern "C" int32_t rbg_dag_closure(const rbg_csr_t *A, void *workspace, int64_t 
     if (n == 0) return RBG_OK;
     if (n >= (1ll << 31) - 1) return RBG_ERR_INVALID;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    if (workspace_bytes < (int64_t)dag_layout(n, 0, nullptr, nullptr)) return RBG_ERR_NOMEM;
+    int rc = dag_configure();
+    if (rc) return rc;
+    // the pieces that need no levels; their count and nnz(A) come back together
+    DagWs w;
+    dag_layout(n, 0, reinterpret_cast<unsigned char *>(workspace), &w);
+    DagArgs a = dag_args(n, A, w, pool_cols, pool_vals, pool_capacity, row_off, row_len);
+    RBG_CUDA_TRY(cudaMemsetAsync(w.cnt, 0, sizeof(DagCounters), s));
+    RBG_CUDA_TRY(cudaMemsetAsync(row_len, 0xff, (size_t)n * 4, s));
+    if (!(mode & RBG_DAG_NO_TILES)) {
+        RBG_CUDA_TRY(cudaMemsetAsync(w.ccount, 0xff, (size_t)n * 4, s));
+        note_launches(3);
+        dag_span_kernel<<<grid_for(n, 256), 256, 0, s>>>(n, a.ap, a.aj, w.ccount);
+        size_t tb = w.tmp_bytes;
+        RBG_CUDA_TRY(cub::DeviceScan::InclusiveScan(w.tmp, tb, w.ccount, w.cursor, IntMax(), (int)n, s));
+        const int64_t tiles = (n + DT_ROWS - 1) / DT_ROWS;
+        dag_tile_kernel<<<(unsigned)((tiles + DT_WARPS - 1) / DT_WARPS), DT_WARPS * 32, sizeof(DagTile) * DT_WARPS, s>>>(
+            a, w.cursor, &w.cnt->tile_rows, &w.cnt->tile_levels);
+        RBG_CUDA_TRY(cudaGetLastError());
+    }
     int64_t annz = 0;
+    DagCounters c;
     {
-        HostStaging hs(s, 256);
-        int rc = hs.down(&annz, A->indptr + n, 8);
+        HostStaging hs(s, 512);
+        rc = hs.down(&annz, A->indptr + n, 8);
+        if (!rc) rc = hs.down(&c, w.cnt, sizeof(c));
         if (!rc) rc = hs.finish();
         if (rc) return rc;
     }
     if (workspace_bytes < (int64_t)dag_layout(n, annz, nullptr, nullptr)) return RBG_ERR_NOMEM;
-    DagCounters *dc = nullptr;
-    int64_t launched = 0;
-    int rc = dag_enqueue(A, annz, workspace, pool_cols, pool_vals, pool_capacity, row_off, row_len, s, false, &dc,
-                         nullptr, &launched);
-    if (rc) return rc;
-    DagCounters c;
-    {
+    if (c.tile_rows < n) {                       // the rest by levels
+        dag_layout(n, annz, reinterpret_cast<unsigned char *>(workspace), &w);
+        a = dag_args(n, A, w, pool_cols, pool_vals, pool_capacity, row_off, row_len);
+        rc = dag_front(a, w, s);
+        int64_t launched = 0;
+        if (!rc) rc = dag_levels_host(a, w, s, &launched);
+        if (rc) return rc;
         HostStaging hs(s, 256);
-        rc = hs.down(&c, dc, sizeof(c));
+        rc = hs.down(&c, w.cnt, sizeof(c));
         if (!rc) rc = hs.finish();
         if (rc) return rc;
     }
-    *levels = c.nlevels;
-    if (c.placed < n) return RBG_ERR_CYCLE;      // vertices on (or below) a cycle were never placed
+    *levels = std::max(c.nlevels, c.tile_levels);
+    if (c.placed + c.tile_rows < n) return RBG_ERR_CYCLE;      // vertices on (or below) a cycle were never placed
     if (c.flags & 2) { *nnz = -1; return RBG_ERR_CAPACITY; }
     if (c.flags & 1) {
         const int64_t reserved = (int64_t)c.reserved;
@@ -1101,8 +1378,7 @@ extern "C" int32_t rbg_dag_gather(int64_t n, const int32_t *pool_cols, const int
                                   int64_t workspace_bytes, int64_t *indptr, int32_t *indices, int32_t *data,
                                   rbg_stream_t stream) {
     if (n < 0 || !indptr || !workspace) return RBG_ERR_INVALID;
-    size_t tb = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, tb, (int64_t *)nullptr, (int64_t *)nullptr, (int)(n + 1));
+    size_t tb = gather_tmp_bytes(n);
     const size_t need = align_up((size_t)(n + 1) * 8, 256) + tb;
     if ((size_t)workspace_bytes < need) return RBG_ERR_NOMEM;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
@@ -1112,7 +1388,7 @@ extern "C" int32_t rbg_dag_gather(int64_t n, const int32_t *pool_cols, const int
     dag_len64_kernel<<<grid_for(n + 1, 256), 256, 0, s>>>(n, row_len, len64);
     RBG_CUDA_TRY(cub::DeviceScan::ExclusiveSum(tmp, tb, len64, indptr, (int)(n + 1), s));
     if (n > 0)
-        dag_gather_rows_kernel<<<grid_for(n * 8, 256), 256, 0, s>>>(n, row_off, pool_cols, pool_vals, indptr,
+        dag_gather_rows_kernel<<<(unsigned)((n + 31) / 32), 256, 0, s>>>(n, row_off, pool_cols, pool_vals, indptr,
                                                                     indices, data);
     RBG_CUDA_TRY(cudaGetLastError());
     return RBG_OK;
@@ -1120,8 +1396,7 @@ extern "C" int32_t rbg_dag_gather(int64_t n, const int32_t *pool_cols, const int
 
 extern "C" int32_t rbg_dag_gather_workspace_bytes(int64_t n, int64_t *bytes) {
     if (!bytes || n < 0) return RBG_ERR_INVALID;
-    size_t tb = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, tb, (int64_t *)nullptr, (int64_t *)nullptr, (int)(n + 1));
+    size_t tb = gather_tmp_bytes(n);
     *bytes = (int64_t)(align_up((size_t)(n + 1) * 8, 256) + tb);
     return RBG_OK;
 }

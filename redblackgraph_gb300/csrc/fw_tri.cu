@@ -1220,6 +1220,16 @@ struct TriLayout {
     size_t fixed;                            // bytes before the pool
 };
 
+// Scratch of a scan over NR + 1 words.
+size_t tri_scan_tmp(size_t NR) {
+    static thread_local LastSize last;
+    return last.get((int64_t)NR, [NR] {
+        size_t b = 0;
+        cub::DeviceScan::ExclusiveSum(nullptr, b, (int64_t *)nullptr, (int64_t *)nullptr, (int)(NR + 1));
+        return b;
+    });
+}
+
 void tri_layout(unsigned char *base, size_t ws_bytes, size_t C, size_t NR, bool is_short, TriLayout &L) {
     Carve cv{base};
     L.dc = cv.take<TriComp>(C);
@@ -1249,8 +1259,7 @@ void tri_layout(unsigned char *base, size_t ws_bytes, size_t C, size_t NR, bool 
         L.kid_cnt = cv.take<int32_t>(NR);
         L.children = cv.take<int32_t>(NR * TRI_CAP);
     } else {
-        L.scan_tmp = 0;
-        cub::DeviceScan::ExclusiveSum(nullptr, L.scan_tmp, (int64_t *)nullptr, (int64_t *)nullptr, (int)(NR + 1));
+        L.scan_tmp = tri_scan_tmp(NR);
         L.indptr = cv.take<int64_t>(NR + 1);
         L.tmp = cv.take<unsigned char>(L.scan_tmp);
         L.a_col = cv.take<int32_t>(NR * TRI_CAP);
@@ -1321,7 +1330,6 @@ int tri_enqueue(const TriShape &sh, const TriLayout &L, const T *in, T *out, cud
     RBG_CUDA_TRY(cudaGetLastError());
     *launches += 5;
     rbg_csr_t A{R, R, L.indptr, L.a_col, L.a_val};
-    RBG_CUDA_TRY(cudaMemsetAsync(L.row_len, 0xff, (size_t)R * 4, s));   // -1: never placed
     DagChildren kids;
     int rc = dag_enqueue(&A, R * TRI_CAP, L.dag_ws, L.p_col, L.p_val, L.pool, L.row_off, L.row_len, s, captured,
                          dcount, &kids, launches);

@@ -36,6 +36,20 @@ inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
         if (_e != cudaSuccess) return RBG_ERR_CUDA;          \
     } while (0)
 
+// The last answer of a size query that takes microseconds of host time (static thread_local at the
+// place of the query, whose answer depends on n alone).
+struct LastSize {
+    int64_t n = -1;
+    size_t bytes = 0;
+    template <typename F> size_t get(int64_t m, F &&query) {
+        if (m != n) {
+            bytes = query();
+            n = m;
+        }
+        return bytes;
+    }
+};
+
 // grid size for grid-stride loops: a multiple of the SM count
 int grid_for(int64_t work, int threads);
 
@@ -136,6 +150,7 @@ struct DagCounters {
     int placed, nwide, flags, nlevels;       // flags: 1 pool too small, 2 row past the block table
     unsigned long long reserved, max_abs, total;
     long long level;                         // the graph loop's level counter
+    int tile_rows, tile_levels;              // rows closed without levels, and their deepest level + 1
 };
 struct DagChildren {         // children lists of the levels' graph, kept in the workspace
     const int64_t *coff;

@@ -7,7 +7,7 @@
 //
 // One CTA of 128 threads per query: the threads stride the two rows with 16-byte loads where both
 // rows allow it (a warp per query with 4-byte loads took 28 us for 256 queries on n = 4096
-// closures; LOOKUPTIME), keep the smallest (sum, j) and meet in a shuffle and shared-memory
+// closures, 7 us now), keep the smallest (sum, j) and meet in a shuffle and shared-memory
 // reduction: the smallest sum, ties to the smallest j.  The sum wraps in the matrix's own type, as
 // numpy scalar arithmetic does on the reference's rows (for unsigned types the red one, the type's
 // maximum, plus y gives y - 1).  Types of up to 4 bytes pack (sum in the type's order, j) into one

@@ -1151,9 +1151,13 @@ struct Head {   // workspace that lives from rbg_spgemm_count to rbg_spgemm_gath
 };
 
 size_t scan_bytes(int64_t n) {
-    size_t b = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, b, (int64_t *)nullptr, (int64_t *)nullptr, (int)std::max<int64_t>(n + 1, 1));
-    return b;
+    static thread_local LastSize last;
+    return last.get(n, [n] {
+        size_t b = 0;
+        cub::DeviceScan::ExclusiveSum(nullptr, b, (int64_t *)nullptr, (int64_t *)nullptr,
+                                      (int)std::max<int64_t>(n + 1, 1));
+        return b;
+    });
 }
 
 size_t head_layout(int64_t n, unsigned char *base, Head *h) {

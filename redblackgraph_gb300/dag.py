@@ -35,12 +35,13 @@ class DagRows:
     nnz: int
 
 
-def dag_closure_device(A: DeviceCSR, stream=None, pool_factor: int = 16, gather: bool = True):
+def dag_closure_device(A: DeviceCSR, stream=None, pool_factor: int = 16, gather: bool = True, tiles: bool = True):
     """Closure of the DAG ``A`` (int32 values).  Returns ``(C, max_abs, levels)``: the closure as
     a DeviceCSR (int64 row pointers, int32 indices and values, rows sorted) -- or, with
     ``gather=False``, as the row pool itself (``DagRows``) -- the largest magnitude among A's
     entries and all candidates (the reference's diameter source) and the number of topological
-    levels.  Raises CycleError on a cycle and RowTooWide for rows past 8192 columns."""
+    levels.  ``tiles``: look for pieces of a few consecutive vertices that need no levels first (the
+    result is the same).  Raises CycleError on a cycle and RowTooWide for rows past 8192 columns."""
     from .dense import CycleError
     if A.data.dtype != torch.int32:
         raise TypeError("the DAG closure takes int32 values")
@@ -63,9 +64,9 @@ def dag_closure_device(A: DeviceCSR, stream=None, pool_factor: int = 16, gather:
         cols = torch.empty(cap, dtype=torch.int32, device=dev)
         vals = torch.empty(cap, dtype=torch.int32, device=dev)
         nnz, mx, lv = ctypes.c_int64(0), ctypes.c_int64(0), ctypes.c_int64(0)
-        rc = L.rbg_dag_closure(ctypes.byref(ca), ws.data_ptr(), ws.numel(), cols.data_ptr(), vals.data_ptr(), cap,
-                               row_off.data_ptr(), row_len.data_ptr(), ctypes.byref(nnz), ctypes.byref(mx),
-                               ctypes.byref(lv), sh)
+        rc = L.rbg_dag_closure_mode(ctypes.byref(ca), 0 if tiles else _lib.DAG_NO_TILES, ws.data_ptr(), ws.numel(),
+                                    cols.data_ptr(), vals.data_ptr(), cap, row_off.data_ptr(), row_len.data_ptr(),
+                                    ctypes.byref(nnz), ctypes.byref(mx), ctypes.byref(lv), sh)
         if rc == _lib.RBG_ERR_CYCLE:
             raise CycleError("transitive_closure_dag_sparse requires a DAG (no cycles)", vertex=-1)
         if rc == _lib.RBG_ERR_CAPACITY:

@@ -381,11 +381,11 @@ __device__ __forceinline__ void bulk_to_smem(uint32_t dst, const void *src, uint
                  : "memory");
 }
 
-template <typename U, int BN> struct TileSmem {
-    U CPt[FW_B][FW_P];       // CPt[q][i] = d_{t-1}(i, t) for the q-th active step t
+template <typename U, int BM, int BN> struct TileSmem {
+    U CPt[FW_B][BM];         // CPt[q][i] = d_{t-1}(i, t) for the q-th active step t
     U RPm[FW_B][BN];         // 2^msb(d_{t-1}(t, j)) (0 for zero), q-th active step
     U RPl[FW_B][BN];         // d_{t-1}(t, j) - 2^msb   (inf for zero), q-th active step
-    unsigned long long maskC[FW_P];   // bit t: CP(i, t) valid
+    unsigned long long maskC[BM];     // bit t: CP(i, t) valid
     unsigned long long maskR[BN];     // bit t: RP(t, j) valid
     int active[FW_B];                 // active[q] = t
     int qof[FW_B];                    // qof[t] = q (or -1)
@@ -402,14 +402,13 @@ template <typename U, int BN> struct TileSmem {
 // group's snapshot row t is written only when bit t of its group mask is set.
 // Returns false when the snapshot copies did not complete within the bounded wait (the item's
 // component is then marked RBG_EV_TIMEOUT and the CTA stops taking items).
-template <typename U, int BN, int TM, int TN>
-__device__ __forceinline__ bool tile_item(TileSmem<U, BN> &S, int ci, int64_t local, U *__restrict__ work_base,
+template <typename U, int BM, int BN, int TM, int TN>
+__device__ __forceinline__ bool tile_item(TileSmem<U, BM, BN> &S, int ci, int64_t local, U *__restrict__ work_base,
                                           const unsigned long long *__restrict__ mask_base,
                                           unsigned char *__restrict__ occ_base,
                                           const FwComp *__restrict__ comps, int64_t K0, int lbits,
                                           DevStatus *st_base, uint32_t bar, uint32_t &parity) {
     typedef lane<U> L;
-    constexpr int BM = FW_P;
     constexpr int TX = BN / TN;           // threads along columns
     constexpr int TY = BM / TM;           // threads along rows
     static_assert(TX * TY == FW_THREADS, "micro-tile layout must use 256 threads");
@@ -507,10 +506,10 @@ __device__ __forceinline__ bool tile_item(TileSmem<U, BN> &S, int ci, int64_t lo
     {
         constexpr int PC = BM / FW_B, PR = BN / FW_B, PP = PC + PR;   // pieces per active step
         constexpr uint32_t PIECE = FW_B * sizeof(U);                   // bytes per piece
-        static_assert(PC == 2, "a tile is two 64-row groups high");
-        const unsigned long long cg0 = gmC[I0 / FW_B], cg1 = gmC[I0 / FW_B + 1];
+        static_assert(PC == 1 || PC == 2, "a tile is one or two 64-row groups high");
+        const unsigned long long cg0 = gmC[I0 / FW_B], cg1 = PC == 2 ? gmC[I0 / FW_B + 1] : 0ull;
         auto live = [&](int p, int t) -> bool {
-            const unsigned long long g = p == 0 ? cg0 : p == 1 ? cg1 : gmR[J0 / FW_B + (p - PC)];
+            const unsigned long long g = p == 0 ? cg0 : p < PC ? cg1 : gmR[J0 / FW_B + (p - PC)];
             return (g >> t) & 1ull;
         };
         if (tid < 32) {
@@ -574,24 +573,36 @@ __device__ __forceinline__ bool tile_item(TileSmem<U, BN> &S, int ci, int64_t lo
         if (mc >= 0 && mr >= 0 && mc + mr >= lbits - 1) risk = true;
     }
 
+    // small micro-tiles take two steps at a time, so that one step's loads cover the other's latency
+    constexpr int STEPS = TM * TN * sizeof(U) <= 64 ? 2 : 1;
     unsigned steps_done = 0;
-    for (int q = 0; q < na; ++q) {
-        U x[TM], m[TN], l[TN];
+    for (int q0 = 0; q0 < na; q0 += STEPS) {
+        U x[STEPS][TM], m[STEPS][TN], l[STEPS][TN];
         bool anyx = false;
 #pragma unroll
-        for (int r = 0; r < TM; ++r) {
-            x[r] = S.CPt[q][r0 + r];
-            anyx |= L::valid(x[r]);
+        for (int u = 0; u < STEPS; ++u) {
+            const int q = q0 + u;
+#pragma unroll
+            for (int r = 0; r < TM; ++r) {
+                x[u][r] = STEPS == 1 || q < na ? S.CPt[q][r0 + r] : L::inf;
+                anyx |= L::valid(x[u][r]);
+            }
         }
         // the warp's rows all zero at this step: every product is zero
         if (!__any_sync(0xffffffffu, anyx)) continue;
-        ++steps_done;
+        steps_done += STEPS == 1 || q0 + 1 < na ? STEPS : 1;
 #pragma unroll
-        for (int c = 0; c < TN; ++c) { m[c] = S.RPm[q][cidx[c]]; l[c] = S.RPl[q][cidx[c]]; }
+        for (int u = 0; u < STEPS; ++u) {
+            const int q = STEPS == 1 || q0 + u < na ? q0 + u : q0;
 #pragma unroll
-        for (int r = 0; r < TM; ++r)
+            for (int c = 0; c < TN; ++c) { m[u][c] = S.RPm[q][cidx[c]]; l[u][c] = S.RPl[q][cidx[c]]; }
+        }
 #pragma unroll
-            for (int c = 0; c < TN; ++c) acc[r][c] = umin(acc[r][c], x[r] * m[c] + l[c]);
+        for (int u = 0; u < STEPS; ++u)
+#pragma unroll
+            for (int r = 0; r < TM; ++r)
+#pragma unroll
+                for (int c = 0; c < TN; ++c) acc[r][c] = umin(acc[r][c], x[u][r] * m[u][c] + l[u][c]);
     }
     if (lane_id == 0 && steps_done)
         atomicAdd(&st->executed, (unsigned long long)steps_done * 32 * TM * TN);
@@ -641,7 +652,7 @@ __device__ __forceinline__ bool tile_item(TileSmem<U, BN> &S, int ci, int64_t lo
 // Tile worklist: candidate tile (I, J) of this round is an item when some step t has a nonzero
 // column-panel snapshot in one of its rows and a nonzero row-panel snapshot in one of its
 // columns (the OR of the 64-line group masks of both sides intersect).
-template <int BN>
+template <int BM, int BN>
 __global__ void fw_tile_list_kernel(const FwComp *__restrict__ comps, const int64_t *__restrict__ prefix,
                                     int count, const unsigned long long *__restrict__ mask_base,
                                     int2 *__restrict__ list, int *__restrict__ counters) {
@@ -659,19 +670,20 @@ __global__ void fw_tile_list_kernel(const FwComp *__restrict__ comps, const int6
     unsigned long long r = 0;
 #pragma unroll
     for (int gq = 0; gq < GC; ++gq) r |= gmR[tJ * GC + gq];
-    if ((r & (gmC[2 * tI] | gmC[2 * tI + 1])) == 0) return;
+    constexpr int GR = BM / FW_B;
+    if ((r & (gmC[GR * tI] | gmC[GR * tI + GR - 1])) == 0) return;
     const int slot = atomicAdd(&counters[CNT_TILE], 1);
     list[slot] = make_int2(ci, (int)local);
 }
 
-template <typename U, int BN, int TM, int TN>
+template <typename U, int BM, int BN, int TM, int TN>
 __global__ void __launch_bounds__(FW_THREADS, (TM * TN * sizeof(U) <= 128) ? 3 : 2)
 fw_tile_kernel(U *__restrict__ work_base, const unsigned long long *__restrict__ any_base,
                unsigned char *__restrict__ occ_base,
                const FwComp *__restrict__ comps, const int2 *__restrict__ list, int *__restrict__ counters,
                int64_t K0, int lbits, DevStatus *st_base) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    TileSmem<U, BN> &S = *reinterpret_cast<TileSmem<U, BN> *>(smem_raw);
+    TileSmem<U, BM, BN> &S = *reinterpret_cast<TileSmem<U, BM, BN> *>(smem_raw);
     __shared__ int s_item;
     __shared__ __align__(8) unsigned long long s_bar;   // completion of the snapshot copies
     const uint32_t bar = smem_u32(&s_bar);
@@ -690,7 +702,7 @@ fw_tile_kernel(U *__restrict__ work_base, const unsigned long long *__restrict__
         int nxt = 0;
         if (threadIdx.x == 0) nxt = atomicAdd(&counters[CUR_TILE], 1);
         const int2 e = list[i];
-        const bool ok = tile_item<U, BN, TM, TN>(S, e.x, e.y, work_base, any_base, occ_base, comps, K0, lbits,
+        const bool ok = tile_item<U, BM, BN, TM, TN>(S, e.x, e.y, work_base, any_base, occ_base, comps, K0, lbits,
                                                  st_base, bar, parity);
         if (!ok) {   // uniform: the CTA stops; the item it had claimed next is marked as well
             if (threadIdx.x == 0 && nxt < total)
@@ -953,16 +965,20 @@ static int run_exact(const T *in, int64_t ld_in, T *out, int64_t ld_out, int64_t
 // ------------------------------------------------------------------------------------------
 // host driver
 // ------------------------------------------------------------------------------------------
-// Phase-3 tile shapes: BM = 128 rows always; 32-bit lanes have a wide (128 columns, 8 x 8 cells
-// per thread) and a narrow (64 columns, 4 x 8 cells) shape, chosen per round (RBG_MODE_TILE_NARROW
-// or the autotuner); 64-bit lanes use 64 columns, 8 x 4 cells.
+// Phase-3 tile shapes, chosen per round (rule in round_shape, RBG_MODE_TILE_NARROW or the
+// autotuner): wide 128 x 128 (8 x 8 cells per thread), narrow 128 x 64 (4 x 8) and small 64 x 64
+// (2 x 8); 64-bit lanes use 128 x 64 (8 x 4) for the first two and 64 x 64 (4 x 4).
 template <typename U> struct TileCfg;
-template <> struct TileCfg<uint32_t> { static const int BN = 128, TM = 8, TN = 8; };
-template <> struct TileCfg<uint64_t> { static const int BN = 64, TM = 8, TN = 4; };
+template <> struct TileCfg<uint32_t> { static const int BM = 128, BN = 128, TM = 8, TN = 8; };
+template <> struct TileCfg<uint64_t> { static const int BM = 128, BN = 64, TM = 8, TN = 4; };
 template <typename U> struct TileNarrow;
-template <> struct TileNarrow<uint32_t> { static const int BN = 64, TM = 4, TN = 8; };
-template <> struct TileNarrow<uint64_t> { static const int BN = 64, TM = 8, TN = 4; };
-
+template <> struct TileNarrow<uint32_t> { static const int BM = 128, BN = 64, TM = 4, TN = 8; };
+template <> struct TileNarrow<uint64_t> { static const int BM = 128, BN = 64, TM = 8, TN = 4; };
+template <typename U> struct TileSmall;
+template <> struct TileSmall<uint32_t> { static const int BM = 64, BN = 64, TM = 2, TN = 8; };
+template <> struct TileSmall<uint64_t> { static const int BM = 64, BN = 64, TM = 4, TN = 4; };
+constexpr int64_t SMALL_TILES = 4096;      // small tiles of a round, at most
+constexpr unsigned char SHAPE_WIDE = 0, SHAPE_NARROW = 1, SHAPE_SMALL = 2;
 
 // Everything a (batched) blocked run needs on the host: the component table (sorted by size,
 // descending), the per-kernel CTA prefix sums, the per-round active counts and the workspace
@@ -970,9 +986,9 @@ template <> struct TileNarrow<uint64_t> { static const int BN = 64, TM = 8, TN =
 struct FwPlan {
     int count = 0;
     std::vector<FwComp> comps;
-    std::vector<int64_t> pre_conv, pre_panel, pre_tile, pre_tile_n;   // _n: narrow tiles
+    std::vector<int64_t> pre_conv, pre_panel, pre_tile, pre_tile_n, pre_tile_s;   // _n: narrow, _s: small tiles
     std::vector<int> active;                // active[r] = components with n > 64 r
-    size_t off_status = 0, off_comps = 0, off_pconv = 0, off_ppanel = 0, off_ptile = 0, off_ptile_n = 0;
+    size_t off_status = 0, off_comps = 0, off_pconv = 0, off_ppanel = 0, off_ptile = 0, off_ptile_n = 0, off_ptile_s = 0;
     size_t off_rb = 0, off_any = 0, off_lanes = 0, off_exact = 0, total = 0;
     size_t off_occ = 0, occ_bytes = 0, off_plist = 0, off_tlist = 0, off_counters = 0;
 };
@@ -990,6 +1006,7 @@ static void build_plan(FwPlan &P, int64_t count, const int64_t *sizes, const int
     P.pre_panel.assign((size_t)count + 1, 0);
     P.pre_tile.assign((size_t)count + 1, 0);
     P.pre_tile_n.assign((size_t)count + 1, 0);
+    P.pre_tile_s.assign((size_t)count + 1, 0);
     int64_t lanes = 0, anys = 0, maxn = 0, occs = 0;
     for (int64_t k = 0; k < count; ++k) {
         const int i = order[(size_t)k];
@@ -1011,10 +1028,11 @@ static void build_plan(FwPlan &P, int64_t count, const int64_t *sizes, const int
         c.orig = orig ? (int32_t)orig[i] : i;
         P.pre_conv[(size_t)k + 1] = P.pre_conv[(size_t)k] + (c.np + CONV_ROWS - 1) / CONV_ROWS;
         const bool big = c.n > FW_B;   // n <= 64: the diagonal tile is the whole matrix
-        P.pre_panel[(size_t)k + 1] = P.pre_panel[(size_t)k] + (big ? 2 * (c.np / PN_LINES) : 0);
+        P.pre_panel[(size_t)k + 1] = P.pre_panel[(size_t)k] + (big ? 2 * (c.np / FW_B) : 0);
         P.pre_tile[(size_t)k + 1] = P.pre_tile[(size_t)k] + (big ? (c.np / tile_bn) * (c.np / FW_P) : 0);
         P.pre_tile_n[(size_t)k + 1] =
             P.pre_tile_n[(size_t)k] + (big ? (c.np / tile_bn_narrow) * (c.np / FW_P) : 0);
+        P.pre_tile_s[(size_t)k + 1] = P.pre_tile_s[(size_t)k] + (big ? (c.np / FW_B) * (c.np / FW_B) : 0);
         maxn = std::max(maxn, c.n);
     }
     const int rounds = (int)((maxn + FW_B - 1) / FW_B);
@@ -1031,13 +1049,16 @@ static void build_plan(FwPlan &P, int64_t count, const int64_t *sizes, const int
     P.off_ppanel = o; o = align_up(o + ((size_t)count + 1) * 8, 256);
     P.off_ptile = o; o = align_up(o + ((size_t)count + 1) * 8, 256);
     P.off_ptile_n = o; o = align_up(o + ((size_t)count + 1) * 8, 256);
+    P.off_ptile_s = o; o = align_up(o + ((size_t)count + 1) * 8, 256);
     P.off_rb = o; o = align_up(o + (size_t)count * (lane == 8 ? sizeof(RoundBuf<uint64_t>) : sizeof(RoundBuf<uint32_t>)), 256);
     P.off_any = o; o = align_up(o + (size_t)anys * 8, 256);
     P.off_occ = o; P.occ_bytes = (size_t)occs; o = align_up(o + (size_t)occs, 256);
     const int a0 = rounds > 0 ? P.active[0] : 0;
-    P.off_plist = o; o = align_up(o + (size_t)std::max<int64_t>(P.pre_panel[(size_t)a0], 1) * 8, 256);
+    P.off_plist = o; o = align_up(o + (size_t)std::max<int64_t>(2 * P.pre_panel[(size_t)a0], 1) * 8, 256);
     P.off_tlist = o;
-    o = align_up(o + (size_t)std::max<int64_t>(std::max(P.pre_tile[(size_t)a0], P.pre_tile_n[(size_t)a0]), 1) * 8,
+    // (small tiles only run in rounds of at most SMALL_TILES of them)
+    o = align_up(o + (size_t)std::max<int64_t>({P.pre_tile[(size_t)a0], P.pre_tile_n[(size_t)a0],
+                                                std::min<int64_t>(P.pre_tile_s[(size_t)a0], SMALL_TILES), 1}) * 8,
                  256);
     P.off_counters = o; o = align_up(o + 64, 256);
     P.off_lanes = o; o = align_up(o + (size_t)lanes * lane, 256);
@@ -1056,18 +1077,21 @@ template <typename U>
 static int configure_kernels() {
     static PerDeviceOnce once;   // one per lane type, for every device
     return once.run([] {
-    typedef TileCfg<U> C;
-    RBG_CUDA_TRY(cudaFuncSetAttribute(fw_panel_kernel<U>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)sizeof(PanelSmem<U>)));
+    RBG_CUDA_TRY(cudaFuncSetAttribute(fw_panel_kernel<U, 64, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sizeof(PanelSmem<U, 64>)));
+    RBG_CUDA_TRY(cudaFuncSetAttribute(fw_panel_kernel<U, 32, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sizeof(PanelSmem<U, 32>)));
     RBG_CUDA_TRY(cudaFuncSetAttribute(fw_diag_kernel<U>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)sizeof(DiagSmem<U>)));
-    RBG_CUDA_TRY(cudaFuncSetAttribute(fw_tile_kernel<U, C::BN, C::TM, C::TN>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)sizeof(TileSmem<U, C::BN>)));
-    typedef TileNarrow<U> N;
-    RBG_CUDA_TRY(cudaFuncSetAttribute(fw_tile_kernel<U, N::BN, N::TM, N::TN>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)sizeof(TileSmem<U, N::BN>)));
+    auto tile = [](auto shape) {
+        typedef decltype(shape) S;
+        return cudaFuncSetAttribute(fw_tile_kernel<U, S::BM, S::BN, S::TM, S::TN>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)sizeof(TileSmem<U, S::BM, S::BN>));
+    };
+    RBG_CUDA_TRY(tile(TileCfg<U>()));
+    RBG_CUDA_TRY(tile(TileNarrow<U>()));
+    RBG_CUDA_TRY(tile(TileSmall<U>()));
     return (int)RBG_OK;
     });
 }
@@ -1075,14 +1099,25 @@ static int configure_kernels() {
 // Upload the plan's tables into the workspace.
 static int upload_plan(const FwPlan &P, unsigned char *ws, cudaStream_t stream) {
     const size_t b0 = P.comps.size() * sizeof(FwComp), b1 = P.pre_conv.size() * 8, b2 = P.pre_panel.size() * 8,
-                 b3 = P.pre_tile.size() * 8, b4 = P.pre_tile_n.size() * 8;
-    HostStaging hs(stream, b0 + b1 + b2 + b3 + b4 + 5 * 64);
+                 b3 = P.pre_tile.size() * 8, b4 = P.pre_tile_n.size() * 8, b5 = P.pre_tile_s.size() * 8;
+    HostStaging hs(stream, b0 + b1 + b2 + b3 + b4 + b5 + 6 * 64);
     int rc = hs.up(ws + P.off_comps, P.comps.data(), b0);
     if (!rc) rc = hs.up(ws + P.off_pconv, P.pre_conv.data(), b1);
     if (!rc) rc = hs.up(ws + P.off_ppanel, P.pre_panel.data(), b2);
     if (!rc) rc = hs.up(ws + P.off_ptile, P.pre_tile.data(), b3);
     if (!rc) rc = hs.up(ws + P.off_ptile_n, P.pre_tile_n.data(), b4);
+    if (!rc) rc = hs.up(ws + P.off_ptile_s, P.pre_tile_s.data(), b5);
     return rc;
+}
+
+// The tile shape of a round with `a` matrices active, when nobody asked for one.  A round runs as
+// many tiles as the matrix has live blocks, a quarter of all when it is numbered in a topological
+// order, so wide tiles leave SMs idle up to a few thousand rows: 46 us of
+// wide tiles a round, 30 us of small ones for n = 2048 (the closure: 3.48 ms, 2.22 ms with the
+// narrower panels); n = 4096: 6.8 ms, 6.4 ms with narrow ones.
+static unsigned char round_shape(const FwPlan &P, int a, int sms) {
+    if (P.pre_tile_s[(size_t)a] <= std::min<int64_t>(SMALL_TILES, 16 * (int64_t)sms)) return SHAPE_SMALL;
+    return P.pre_tile_n[(size_t)a] <= 16 * (int64_t)sms ? SHAPE_NARROW : SHAPE_WIDE;
 }
 
 // Launch the whole blocked closure of a plan (conversion, every round, finalization) on
@@ -1092,7 +1127,6 @@ template <typename T, typename U>
 static int launch_blocked(const FwPlan &P, const T *in, T *out, unsigned char *ws, cudaStream_t stream,
                           bool stop_after_convert, DevStatus *h_status, const unsigned char *shapes = nullptr,
                           cudaEvent_t *round_events = nullptr, const RowStats &rs = RowStats()) {
-    typedef TileCfg<U> C;
     const int configured = configure_kernels<U>();   // once per device
     if (configured) return configured;
     const int cnt = P.count;
@@ -1102,7 +1136,7 @@ static int launch_blocked(const FwPlan &P, const T *in, T *out, unsigned char *w
     const int64_t *ppanel = reinterpret_cast<const int64_t *>(ws + P.off_ppanel);
     const int64_t *ptile = reinterpret_cast<const int64_t *>(ws + P.off_ptile);
     const int64_t *ptile_n = reinterpret_cast<const int64_t *>(ws + P.off_ptile_n);
-    typedef TileNarrow<U> N;
+    const int64_t *ptile_s = reinterpret_cast<const int64_t *>(ws + P.off_ptile_s);
     RoundBuf<U> *rbs = reinterpret_cast<RoundBuf<U> *>(ws + P.off_rb);
     unsigned long long *any = reinterpret_cast<unsigned long long *>(ws + P.off_any);
     U *lanes = reinterpret_cast<U *>(ws + P.off_lanes);
@@ -1134,8 +1168,10 @@ static int launch_blocked(const FwPlan &P, const T *in, T *out, unsigned char *w
     for (size_t r = 0; r < P.active.size(); ++r) {
         const int a = P.active[r];
         const int64_t K0 = (int64_t)r * FW_B;
-        const bool narrow = shapes && shapes[r];
-        const int64_t np_ = P.pre_panel[(size_t)a], nt_ = narrow ? P.pre_tile_n[(size_t)a] : P.pre_tile[(size_t)a];
+        const unsigned char shape = shapes ? shapes[r] : round_shape(P, a, sms);
+        const int64_t np_ = P.pre_panel[(size_t)a];
+        const int64_t nt_ = shape == SHAPE_SMALL    ? P.pre_tile_s[(size_t)a]
+                            : shape == SHAPE_NARROW ? P.pre_tile_n[(size_t)a] : P.pre_tile[(size_t)a];
         note_launches(1 + (np_ > 0 ? 2 : 0) + (nt_ > 0 ? 2 : 0));
         cudaEvent_t td = timer_begin(2, stream);
         fw_diag_kernel<U><<<a, DG_THREADS, sizeof(DiagSmem<U>), stream>>>(lanes, any, rbs, comps, counters,
@@ -1143,28 +1179,37 @@ static int launch_blocked(const FwPlan &P, const T *in, T *out, unsigned char *w
         timer_end(2, td, stream);
         if (np_ > 0) {
             cudaEvent_t t0 = timer_begin(1, stream);
-            fw_panel_list_kernel<<<(unsigned)((np_ + 255) / 256), 256, 0, stream>>>(comps, ppanel, a, K0, occ,
-                                                                                    plist, counters);
-            fw_panel_kernel<U><<<(unsigned)std::min<int64_t>(np_, persist), PN_THREADS, sizeof(PanelSmem<U>),
-                                 stream>>>(lanes, any, occ, rbs, comps, plist, counters, K0, lbits, st);
+            // 32 lines per CTA while that still leaves the SMs' two CTAs at one item each
+            auto panels = [&](auto lines, auto cells) {
+                constexpr int LINES = decltype(lines)::value, CELLS = decltype(cells)::value;
+                const int64_t items = np_ * (FW_B / LINES);
+                fw_panel_list_kernel<LINES><<<(unsigned)((items + 255) / 256), 256, 0, stream>>>(comps, ppanel, a, K0,
+                                                                                                 occ, plist, counters);
+                fw_panel_kernel<U, LINES, CELLS>
+                    <<<(unsigned)std::min<int64_t>(items, persist), LINES * FW_B / CELLS, sizeof(PanelSmem<U, LINES>),
+                       stream>>>(lanes, any, occ, rbs, comps, plist, counters, K0, lbits, st);
+            };
+            if (2 * np_ <= persist) panels(std::integral_constant<int, 32>(), std::integral_constant<int, 8>());
+            else panels(std::integral_constant<int, 64>(), std::integral_constant<int, 16>());
             timer_end(1, t0, stream);
         }
         if (round_events) RBG_CUDA_TRY(cudaEventRecord(round_events[2 * r], stream));
         if (nt_ > 0) {
             cudaEvent_t t0 = timer_begin(0, stream);
-            const unsigned tl = (unsigned)((nt_ + 255) / 256);
-            // persistent grids: as many CTAs as fit on the SMs (3 per SM for the narrow 32-bit shape)
-            const int per_sm = (N::TM * N::TN * (int)sizeof(U) <= 128) ? 3 : 2;
-            const unsigned tg = (unsigned)std::min<int64_t>(nt_, narrow ? (int64_t)per_sm * sms : persist);
-            if (narrow) {
-                fw_tile_list_kernel<N::BN><<<tl, 256, 0, stream>>>(comps, ptile_n, a, any, tlist, counters);
-                fw_tile_kernel<U, N::BN, N::TM, N::TN><<<tg, FW_THREADS, sizeof(TileSmem<U, N::BN>), stream>>>(
-                    lanes, any, occ, comps, tlist, counters, K0, lbits, st);
-            } else {
-                fw_tile_list_kernel<C::BN><<<tl, 256, 0, stream>>>(comps, ptile, a, any, tlist, counters);
-                fw_tile_kernel<U, C::BN, C::TM, C::TN><<<tg, FW_THREADS, sizeof(TileSmem<U, C::BN>), stream>>>(
-                    lanes, any, occ, comps, tlist, counters, K0, lbits, st);
-            }
+            // persistent grids: as many CTAs as fit on the SMs
+            auto tiles = [&](auto cfg, const int64_t *pre) {
+                typedef decltype(cfg) S;
+                constexpr int per_sm = (S::TM * S::TN * (int)sizeof(U) <= 128) ? 3 : 2;
+                const unsigned tg = (unsigned)std::min<int64_t>(nt_, (int64_t)per_sm * sms);
+                fw_tile_list_kernel<S::BM, S::BN><<<(unsigned)((nt_ + 255) / 256), 256, 0, stream>>>(comps, pre, a, any,
+                                                                                                    tlist, counters);
+                fw_tile_kernel<U, S::BM, S::BN, S::TM, S::TN>
+                    <<<tg, FW_THREADS, sizeof(TileSmem<U, S::BM, S::BN>), stream>>>(lanes, any, occ, comps, tlist,
+                                                                                    counters, K0, lbits, st);
+            };
+            if (shape == SHAPE_SMALL) tiles(TileSmall<U>(), ptile_s);
+            else if (shape == SHAPE_NARROW) tiles(TileNarrow<U>(), ptile_n);
+            else tiles(TileCfg<U>(), ptile);
             timer_end(0, t0, stream);
         }
         if (round_events) RBG_CUDA_TRY(cudaEventRecord(round_events[2 * r + 1], stream));

@@ -6,15 +6,15 @@
 //       cs[t][a] = d_{t-1}(a, t)   (column t as step t reads it)
 //       rs(t, b) = d_{t-1}(t, b)   (row t as step t reads it), stored split as (2^msb, low)
 //   with per-step maxima of msb (for the exact top-bit test) and validity masks.
-// Phase 2 (fw_panel_kernel, 64 panel columns or rows per CTA): each panel column (row panel) or
+// Phase 2 (fw_panel_kernel, 64 or 32 panel columns or rows per CTA): each panel column (row panel) or
 //   row (column panel) is held in registers by PN_LANES lanes and runs its forward substitution
 //       P(a, j) <- P(a, j) (+) cs[t][a] (x) P(t, j)      (row panel, t = K0..K0+63)
 //       P(i, b) <- P(i, b) (+) P(i, t) (x) rs(t, b)      (column panel)
 //   storing the step-t operands P(t, j) / P(i, t) (the phase-3 snapshots) t-major.
 #pragma once
 
-constexpr int DG_THREADS = 256;   // phase 1: 4 threads per column, 16 rows each
-constexpr int DG_ROWS = 16;
+constexpr int DG_THREADS = 512;   // phase 1: 8 threads per column, 8 rows each
+constexpr int DG_ROWS = 8;
 
 // Round buffer (global memory, written by phase 1, read by phase 2).
 template <typename U> struct RoundBuf {
@@ -39,12 +39,12 @@ template <typename U> struct Pad {
     __device__ __forceinline__ static int at(int c) { return c + P * (c >> 4); }
 };
 
-// 16 consecutive lane words from 16-byte aligned shared memory
-template <typename U> __device__ __forceinline__ void load16(const U *p, U (&x)[DG_ROWS]) {
+// N consecutive lane words from 16-byte aligned memory
+template <typename U, int N> __device__ __forceinline__ void loadN(const U *p, U (&x)[N]) {
     const uint4 *q = reinterpret_cast<const uint4 *>(p);
     constexpr int PER = 16 / sizeof(U);
 #pragma unroll
-    for (int i = 0; i < DG_ROWS / PER; ++i) {
+    for (int i = 0; i < N / PER; ++i) {
         uint4 v = q[i];
         const U *w = reinterpret_cast<const U *>(&v);
 #pragma unroll
@@ -57,11 +57,17 @@ template <typename U> struct DiagSmem {
     U CS[FW_B][Pad<U>::LD];           // CS[t][Pad::at(a)]
     U Y[FW_B][FW_B];                  // Y[t][b] = rs(t, b)
     typename signed_of<U>::type colmax[FW_B][DG_THREADS / FW_B];
+    unsigned long long maskC[FW_B], maskR[FW_B];   // as RoundBuf::maskCS, maskRS
 };
 
-// Thread (b = tid % 64, h = tid / 64) holds rows a = 16 h + l (l = 0..15) of column b.  Steps
-// run in blocks of 16, fully unrolled, so the row of step t is the static register R[t % 16]
-// of the threads with h = t / 16.  One barrier per step: step t's writes go to slot t only.
+// Thread (b = tid % 64, h = tid / 64) holds rows a = 8 h + l (l = 0..7) of column b.  Steps
+// run in blocks of 8, fully unrolled, so the row of step t is the static register R[t % 8]
+// of the threads with h = t / 8.  One barrier per step: step t's writes go to slot t only.  A warp
+// (8 rows, 32 columns) skips the update of a step whose column is zero in its rows or whose row is
+// zero in its columns: in a matrix numbered in a topological order half of the tile is.  The running
+// maximum needs each newly valid cell's first valid product only, found from the masks at the end.
+// Bound by the chain of 64 steps: 18 us a round (n = 2048) with 4 threads per column,
+// every update run and every value tracked; 14 us with 8 threads per column.
 template <typename U>
 __global__ void __launch_bounds__(DG_THREADS)
 fw_diag_kernel(U *__restrict__ work_base, unsigned long long *__restrict__ any_base, RoundBuf<U> *__restrict__ rbs,
@@ -85,35 +91,39 @@ fw_diag_kernel(U *__restrict__ work_base, unsigned long long *__restrict__ any_b
 #pragma unroll
     for (int l = 0; l < DG_ROWS; ++l) R[l] = work[(K0 + h * DG_ROWS + l) * np + K0 + b];
     bool risk = false;
-    SU pm[4] = {0, 0, 0, 0};
+    unsigned startInf = 0;                            // bit r: cell r was zero at round start
+#pragma unroll
+    for (int r = 0; r < DG_ROWS; ++r) startInf |= (unsigned)(!L::valid(R[r])) << r;
     for (int T = 0; T < FW_B / DG_ROWS; ++T) {
 #pragma unroll
         for (int l = 0; l < DG_ROWS; ++l) {
             const int t = T * DG_ROWS + l;
             if (b == t) {   // publish column t (invariant during step t)
                 SU cm = -1;
+                constexpr int PER = 16 / sizeof(U);
 #pragma unroll
-                for (int r = 0; r < DG_ROWS; ++r) {
-                    S.CS[t][Pad<U>::at(h * DG_ROWS) + r] = R[r];
-                    cm = max(cm, (SU)R[r]);
+                for (int r = 0; r < DG_ROWS; r += PER) {
+                    U v[PER];
+#pragma unroll
+                    for (int k = 0; k < PER; ++k) {
+                        v[k] = R[r + k];
+                        cm = max(cm, (SU)v[k]);
+                    }
+                    *reinterpret_cast<uint4 *>(&S.CS[t][Pad<U>::at(h * DG_ROWS) + r]) = *reinterpret_cast<const uint4 *>(v);
                 }
                 S.colmax[t][h] = cm;
             }
             if (h == T) S.Y[t][b] = R[l];   // row t (invariant during step t)
             __syncthreads();
             const U y = S.Y[t][b];
+            if (!__any_sync(0xffffffffu, L::valid(y))) continue;   // warp-uniform, as the next test
+            if (S.colmax[t][h] <= 0) continue;
             U m, low;
             L::split(y, m, low);
-            SU cm = max(max(S.colmax[t][0], S.colmax[t][1]), max(S.colmax[t][2], S.colmax[t][3]));
-            if (L::valid(y) && cm > 0 && msb_nz<U>((U)cm) + msb_nz<U>(y) >= lbits - 1) risk = true;
             U x[DG_ROWS];
-            load16<U>(&S.CS[t][Pad<U>::at(h * DG_ROWS)], x);
+            loadN<U, DG_ROWS>(&S.CS[t][Pad<U>::at(h * DG_ROWS)], x);
 #pragma unroll
-            for (int r = 0; r < DG_ROWS; ++r) {
-                const U v = umin(R[r], x[r] * m + low);
-                R[r] = v;
-                pm[r & 3] = max(pm[r & 3], (SU)v);
-            }
+            for (int r = 0; r < DG_ROWS; ++r) R[r] = umin(R[r], x[r] * m + low);
         }
     }
     // end-of-round tile; a valid diagonal cell means a cycle
@@ -141,55 +151,60 @@ fw_diag_kernel(U *__restrict__ work_base, unsigned long long *__restrict__ any_b
     }
     if (tid < FW_B) {
         unsigned long long mc = 0, mr = 0;
-        int bc = -100000, br = -100000;
         for (int t = 0; t < FW_B; ++t) {
-            const U x = S.CS[t][Pad<U>::at(tid)], y = S.Y[t][tid];
-            mc |= (unsigned long long)L::valid(x) << t;
-            mr |= (unsigned long long)L::valid(y) << t;
-            bc = max(bc, msb_or_neg<U>(S.CS[tid][Pad<U>::at(t)]));   // step tid's maximum
-            br = max(br, msb_or_neg<U>(S.Y[tid][t]));
+            mc |= (unsigned long long)L::valid(S.CS[t][Pad<U>::at(tid)]) << t;
+            mr |= (unsigned long long)L::valid(S.Y[t][tid]) << t;
         }
-        rb->maskCS[tid] = mc;
-        rb->maskRS[tid] = mr;
-        rb->msbCS[tid] = bc;
-        rb->msbRS[tid] = br;
+        S.maskC[tid] = rb->maskCS[tid] = mc;
+        S.maskR[tid] = rb->maskRS[tid] = mr;
     }
-    SU smx = max(max(pm[0], pm[1]), max(pm[2], pm[3]));
+    // the largest operands of each step, a warp per step; a product of theirs may reach the top bit
+    for (int t = tid >> 5; t < FW_B; t += DG_THREADS / 32) {
+        const int l = tid & 31;
+        int br = max(msb_or_neg<U>(S.Y[t][l]), msb_or_neg<U>(S.Y[t][l + 32]));
+        int bc = l < DG_THREADS / FW_B && S.colmax[t][l] > 0 ? msb_nz<U>((U)S.colmax[t][l]) : -100000;
+        br = __reduce_max_sync(0xffffffffu, br);
+        bc = __reduce_max_sync(0xffffffffu, bc);
+        if (l == 0) {
+            rb->msbCS[t] = bc;
+            rb->msbRS[t] = br;
+        }
+        risk |= bc + br >= lbits - 1;
+    }
+    __syncthreads();
+    SU smx = 0;
+#pragma unroll
+    for (int r = 0; r < DG_ROWS; ++r) {
+        const int a = h * DG_ROWS + r;
+        if (!L::valid(R[r]) || !((startInf >> r) & 1u)) continue;
+        const int tf = __ffsll((long long)(S.maskC[a] & S.maskR[b])) - 1;
+        U m, low;
+        L::split(S.Y[tf][b], m, low);
+        smx = max(smx, (SU)(S.CS[tf][Pad<U>::at(h * DG_ROWS) + r] * m + low));
+    }
     unsigned flags = (risk ? RBG_EV_RISK : 0u) | (cyc ? RBG_EV_CYCLE : 0u);
     flush_status(st, smx > 0 ? (unsigned long long)smx : 0ull, flags);
 }
 
 // ------------------------------------------------------------------------------ phase 2
-// PN_LANES lanes of a warp share one panel column (row panel) or row (column panel),
-// PN_CELLS cells each.  The step-t operand P(t, j) / P(i, t) lives in lane h = t / PN_CELLS of
+// FW_B / CELLS lanes of a warp share one panel column (row panel) or row (column panel),
+// CELLS cells each.  The step-t operand P(t, j) / P(i, t) lives in lane h = t / CELLS of
 // the group and is broadcast with a shuffle, so the 64 steps need no barrier.  Steps run in
-// fully unrolled blocks of PN_CELLS, keeping every register index static.
-constexpr int PN_LINES = 64;                      // panel columns / rows per CTA
-constexpr int PN_CELLS = 16;                      // cells of a line held by one lane
-constexpr int PN_LANES = FW_B / PN_CELLS;         // lanes per line
-constexpr int PN_THREADS = PN_LINES * PN_LANES;
+// fully unrolled blocks of CELLS, keeping every register index static.
+// A CTA takes LINES columns / rows: 64, or 32 when a round has too few items to fill the GPU (its
+// 64 steps then share the SM with fewer warps: 18 us a round against 20 us, n = 2048).  The group masks and snapshots stay
+// per 64 lines: with LINES 32 the two halves meet in an atomic OR, and each writes its snapshots of
+// all steps, zeros included.
+// CELLS cells of a line are held by one lane: 16, or 8 with LINES 32 (more warps, shorter steps).
 
-// N consecutive lane words from 16-byte aligned memory
-template <typename U, int N> __device__ __forceinline__ void loadN(const U *p, U (&x)[N]) {
-    const uint4 *q = reinterpret_cast<const uint4 *>(p);
-    constexpr int PER = 16 / sizeof(U);
-#pragma unroll
-    for (int i = 0; i < N / PER; ++i) {
-        uint4 v = q[i];
-        const U *w = reinterpret_cast<const U *>(&v);
-#pragma unroll
-        for (int k = 0; k < PER; ++k) x[i * PER + k] = w[k];
-    }
-}
-
-template <typename U> struct PanelSmem {
+template <typename U, int LINES> struct PanelSmem {
     U TA[FW_B][Pad<U>::LD];           // row panel: cs[t][a]; column panel: rsm[t][b] (padded)
     U RSl[FW_B][Pad<U>::LD];          //               rsl[t][b]   (padded)
     unsigned long long maskCS[FW_B];
     unsigned long long maskRS[FW_B];
     int msbCS[FW_B];
     int msbRS[FW_B];
-    U Z[FW_B][PN_LINES];              // Z[t][line]: the line's step-t operand (its snapshot)
+    U Z[FW_B][LINES];                 // Z[t][line]: the line's step-t operand (its snapshot)
     unsigned long long any;           // OR of the item's line masks
 };
 
@@ -201,10 +216,9 @@ template <typename U> __device__ __forceinline__ U shfl_lane(U v, int src) {
     return (U)__shfl_sync(0xffffffffu, (unsigned)v, src);
 }
 
-// One panel item: 64 lines (a 64 x 64 block) of component ci's row panel (local < np / 64)
-// or column panel.
-template <typename U>
-__device__ __forceinline__ void panel_item(PanelSmem<U> &S, int ci, int local, U *__restrict__ work_base,
+// One panel item: LINES lines of component ci's row panel (local < np / LINES) or column panel.
+template <typename U, int LINES, int PN_CELLS>
+__device__ __forceinline__ void panel_item(PanelSmem<U, LINES> &S, int ci, int local, U *__restrict__ work_base,
                                            unsigned long long *__restrict__ any_base,
                                            unsigned char *__restrict__ occ_base,
                                            const RoundBuf<U> *__restrict__ rbs,
@@ -212,6 +226,9 @@ __device__ __forceinline__ void panel_item(PanelSmem<U> &S, int ci, int local, U
                                            DevStatus *st_base) {
     typedef lane<U> L;
     typedef typename signed_of<U>::type SU;
+    constexpr int PN_LANES = FW_B / PN_CELLS;         // lanes per line
+    constexpr int PN_THREADS = LINES * PN_LANES;
+    constexpr int SPLIT = FW_B / LINES;               // items per 64-line group
     const int tid = threadIdx.x;
     const FwComp cmp = comps[ci];
     const int64_t np = cmp.np;
@@ -226,7 +243,7 @@ __device__ __forceinline__ void panel_item(PanelSmem<U> &S, int ci, int local, U
     const int nb = (int)(np / FW_B);
     const RoundBuf<U> *rb = rbs + cmp.rb_index;
     DevStatus *st = st_base + cmp.status_index;
-    const int nct = (int)(np / PN_LINES);             // items per panel
+    const int nct = (int)(np / LINES);                // items per panel
     const bool rowPanel = local < nct;
     const int cta = rowPanel ? local : local - nct;
 
@@ -234,7 +251,7 @@ __device__ __forceinline__ void panel_item(PanelSmem<U> &S, int ci, int local, U
     const int h = lanei & (PN_LANES - 1);             // cells h*PN_CELLS .. of the line
     const int grp = lanei & ~(PN_LANES - 1);          // first lane of this line's group
     const int line = tid / PN_LANES;
-    const int64_t g = (int64_t)cta * PN_LINES + line; // global column / row
+    const int64_t g = (int64_t)cta * LINES + line;    // global column / row
     const bool inK = g >= K0 && g < K0 + FW_B;        // the diagonal tile's own cells
     const int c0 = h * PN_CELLS;
     constexpr unsigned ALL_INF = (1u << PN_CELLS) - 1u;
@@ -277,9 +294,17 @@ __device__ __forceinline__ void panel_item(PanelSmem<U> &S, int ci, int local, U
             if (!rowPanel) vb[i] = tb[tid + i * PN_THREADS];
         }
     }
-    // 64 lines that are all zero stay zero this round: no snapshots, no write-back, and the
-    // group flag stays 0 so the tile kernel reads none of them
-    if (!__syncthreads_or(startInf != ALL_INF)) return;
+    // lines that are all zero stay zero this round: no snapshots, no write-back, and the group flag
+    // stays 0 so the tile kernel reads none of them (unless the group's other lines set it)
+    if (!__syncthreads_or(startInf != ALL_INF)) {
+        if (SPLIT > 1) {
+            U *dst = rowPanel ? rpbuf : cpbuf;
+            for (int e = tid; e < FW_B * LINES; e += PN_THREADS)
+                dst[(int64_t)(e / LINES) * np + (int64_t)cta * LINES + e % LINES] = L::inf;
+            if (h == 0) (rowPanel ? lineRP : lineCP)[g] = 0;
+        }
+        return;
+    }
 
     if (tid == 0) S.any = 0;
     {
@@ -304,7 +329,6 @@ __device__ __forceinline__ void panel_item(PanelSmem<U> &S, int ci, int local, U
     const int pc0 = Pad<U>::at(c0);
     const U *tabA = &S.TA[0][pc0];
     const U *tabB = &S.RSl[0][pc0];
-    bool changed = false;                             // some cell of this thread decreased
     if (__all_sync(0xffffffffu, startInf == ALL_INF)) {
         // the warp's lines are all zero: they stay zero (a line only meets its own cells as
         // step operands), so only their snapshots are written, as zeros
@@ -315,6 +339,7 @@ __device__ __forceinline__ void panel_item(PanelSmem<U> &S, int ci, int local, U
             // the step operands of block T are lane T's cells; if they are all zero for every
             // line of the warp at the block's start, no step of the block updates anything (an
             // update needs a valid step operand), so they stay zero: skip the block
+            unsigned seenT = 0;
             bool mine = false;
             if (h == T) {
 #pragma unroll
@@ -332,7 +357,7 @@ __device__ __forceinline__ void panel_item(PanelSmem<U> &S, int ci, int local, U
                 const int t = T * PN_CELLS + l;
                 const U z = shfl_lane<U>(R[l], grp | T);  // P(t, j) or P(i, t): invariant at step t
                 const bool zv = L::valid(z);
-                seen |= (unsigned long long)zv << t;
+                seenT |= (unsigned)zv << l;
                 if (h == 0) S.Z[t][line] = z;
                 // a zero step operand makes every product of the step a zero: skip the step when
                 // it is zero for the whole warp (closures of family trees are sparse); operands
@@ -344,29 +369,27 @@ __device__ __forceinline__ void panel_item(PanelSmem<U> &S, int ci, int local, U
                 if (rowPanel) {
                     U m, low;
                     L::split(z, m, low);
-                    if (zv && S.msbCS[t] + msb_nz<U>(z) >= lbits - 1) risk = true;
 #pragma unroll
-                    for (int r = 0; r < PN_CELLS; ++r) {
-                        const U v = umin(R[r], xa[r] * m + low);
-                        changed |= v != R[r];
-                        R[r] = v;
-                    }
+                    for (int r = 0; r < PN_CELLS; ++r) R[r] = umin(R[r], xa[r] * m + low);
                 } else {
                     U xb[PN_CELLS];
                     loadN<U, PN_CELLS>(tabB + t * Pad<U>::LD, xb);
-                    if (zv && msb_nz<U>(z) + S.msbRS[t] >= lbits - 1) risk = true;
 #pragma unroll
-                    for (int r = 0; r < PN_CELLS; ++r) {
-                        const U v = umin(R[r], z * xa[r] + xb[r]);
-                        changed |= v != R[r];
-                        R[r] = v;
-                    }
+                    for (int r = 0; r < PN_CELLS; ++r) R[r] = umin(R[r], z * xa[r] + xb[r]);
                 }
             }
+            seen |= (unsigned long long)seenT << (T * PN_CELLS);
         }
     }
     if (seen && h == 0) atomicOr(&S.any, seen);
     __syncthreads();   // the snapshots (written by lane h == 0 of each group) and S.any are visible
+    // a step operand whose product with the step's largest other operand may reach the top bit (the
+    // line's lanes share its steps)
+#pragma unroll
+    for (int l = 0; l < PN_CELLS; ++l) {
+        const U z = S.Z[c0 + l][line];
+        if (L::valid(z) && msb_nz<U>(z) + (rowPanel ? S.msbCS : S.msbRS)[c0 + l] >= lbits - 1) risk = true;
+    }
     const unsigned long long anyMask = S.any;
     {
         // t-major, coalesced over the CTA's lines; only the steps some line of this group has
@@ -374,16 +397,16 @@ __device__ __forceinline__ void panel_item(PanelSmem<U> &S, int ci, int local, U
         // an invalid operand is written as the encoded zero, so that the tile kernel can copy the
         // rows into shared memory as they are
         U *dst = rowPanel ? rpbuf : cpbuf;
-        const int64_t base = (int64_t)cta * PN_LINES;
-        for (int e = tid; e < FW_B * PN_LINES; e += PN_THREADS) {
-            const int t = e / PN_LINES;
-            if ((anyMask >> t) & 1ull) {
-                const U z = S.Z[t][e % PN_LINES];
-                dst[(int64_t)t * np + base + e % PN_LINES] = L::valid(z) ? z : L::inf;
+        const int64_t base = (int64_t)cta * LINES;
+        for (int e = tid; e < FW_B * LINES; e += PN_THREADS) {
+            const int t = e / LINES;
+            if (SPLIT > 1 || ((anyMask >> t) & 1ull)) {
+                const U z = S.Z[t][e % LINES];
+                dst[(int64_t)t * np + base + e % LINES] = L::valid(z) ? z : L::inf;
             }
         }
     }
-    // write back the cells that changed; the running maximum needs each newly valid cell's
+    // write back the cells of warps that ran a step; the running maximum needs each newly valid cell's
     // first valid product
     SU smx = 0;
     bool wrote = false;
@@ -392,7 +415,7 @@ __device__ __forceinline__ void panel_item(PanelSmem<U> &S, int ci, int local, U
         const U v = R[r];
         const bool vv = L::valid(v);
         const int c = c0 + r;
-        if (!inK && changed) {
+        if (!inK && steps_done) {
             if (rowPanel) work[(K0 + c) * np + g] = vv ? v : L::inf;
             else rowp[r] = vv ? v : L::inf;
             wrote |= vv;
@@ -415,10 +438,15 @@ __device__ __forceinline__ void panel_item(PanelSmem<U> &S, int ci, int local, U
     if ((tid & 31) == 0 && steps_done)
         atomicAdd(&st->executed, (unsigned long long)steps_done * 32 * PN_CELLS);
     if (h == 0) (rowPanel ? lineRP : lineCP)[g] = seen;
-    if (tid == 0) (rowPanel ? anyRP : anyCP)[cta] = anyMask;
+    const int grp64 = cta / SPLIT;
+    if (tid == 0) {
+        unsigned long long *gm = (rowPanel ? anyRP : anyCP) + grp64;
+        if (SPLIT > 1) atomicOr(gm, anyMask);         // zeroed by the diagonal kernel
+        else *gm = anyMask;
+    }
     if (wrote) {
         const int kb = (int)(K0 / FW_B);
-        occ[rowPanel ? (int64_t)kb * nb + cta : (int64_t)cta * nb + kb] = 1;
+        occ[rowPanel ? (int64_t)kb * nb + grp64 : (int64_t)grp64 * nb + kb] = 1;
     }
     flush_status(st, smx > 0 ? (unsigned long long)smx : 0ull, risk ? RBG_EV_RISK : 0u);
 }
@@ -429,10 +457,12 @@ constexpr int CNT_PANEL = 0, CUR_PANEL = 1, CNT_TILE = 2, CUR_TILE = 3;
 
 // Panel worklist: candidate c of this round's panel prefix -> item if its 64 x 64 block of the
 // work matrix holds a nonzero (a zero block stays zero and needs no forward substitution).
+template <int LINES>
 __global__ void fw_panel_list_kernel(const FwComp *__restrict__ comps, const int64_t *__restrict__ prefix,
                                      int count, int64_t K0, const unsigned char *__restrict__ occ_base,
                                      int2 *__restrict__ list, int *__restrict__ counters) {
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    constexpr int SPLIT = FW_B / LINES;
+    const int64_t part = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, c = part / SPLIT;
     if (c >= prefix[count]) return;
     const int ci = fw_find(prefix, count, c);
     const FwComp cmp = comps[ci];
@@ -445,19 +475,19 @@ __global__ void fw_panel_list_kernel(const FwComp *__restrict__ comps, const int
     const unsigned char *occ = occ_base + cmp.occ_off;
     if (!occ[rowPanel ? (int64_t)kb * nb + grp : (int64_t)grp * nb + kb]) return;
     const int slot = atomicAdd(&counters[CNT_PANEL], 1);
-    list[slot] = make_int2(ci, local);
+    list[slot] = make_int2(ci, local * SPLIT + (int)(part % SPLIT));
 }
 
 // Persistent panel kernel: CTAs pull items from the worklist until it is exhausted.
-template <typename U>
-__global__ void __launch_bounds__(PN_THREADS, 2)
+template <typename U, int LINES, int CELLS>
+__global__ void __launch_bounds__(LINES * FW_B / CELLS, 2)
 fw_panel_kernel(U *__restrict__ work_base, unsigned long long *__restrict__ any_base,
                 unsigned char *__restrict__ occ_base,
                 const RoundBuf<U> *__restrict__ rbs, const FwComp *__restrict__ comps,
                 const int2 *__restrict__ list, int *__restrict__ counters, int64_t K0, int lbits,
                 DevStatus *st_base) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    PanelSmem<U> &S = *reinterpret_cast<PanelSmem<U> *>(smem_raw);
+    PanelSmem<U, LINES> &S = *reinterpret_cast<PanelSmem<U, LINES> *>(smem_raw);
     __shared__ int s_item;
     const int total = counters[CNT_PANEL];
     if (threadIdx.x == 0) s_item = atomicAdd(&counters[CUR_PANEL], 1);
@@ -469,7 +499,7 @@ fw_panel_kernel(U *__restrict__ work_base, unsigned long long *__restrict__ any_
         int nxt = 0;
         if (threadIdx.x == 0) nxt = atomicAdd(&counters[CUR_PANEL], 1);
         const int2 e = list[i];
-        panel_item<U>(S, e.x, e.y, work_base, any_base, occ_base, rbs, comps, K0, lbits, st_base);
+        panel_item<U, LINES, CELLS>(S, e.x, e.y, work_base, any_base, occ_base, rbs, comps, K0, lbits, st_base);
         if (threadIdx.x == 0) s_item = nxt;
         __syncthreads();
         i = s_item;

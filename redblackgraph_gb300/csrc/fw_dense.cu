@@ -24,6 +24,9 @@
 //    multiply-add x * 2^msb(y) + (y - 2^msb(y)); (+) is an unsigned min with "zero" encoded as
 //    any word with the top bit set.
 //
+//    A matrix numbered in a topological order whose rows are too wide for the DAG path needs none of
+//    those snapshots and takes the block steps of fw_sided.cuh.
+//
 // 2. Exact path: one k per step, all (i, j) in parallel, with the reference's full scalar
 //    semantics (identities, parity filters, wrap, overflow/cycle signalling).  It replays the
 //    in-place order (rows above k see the old row k, rows below see the new one; W(i,k) changes
@@ -988,7 +991,7 @@ struct FwPlan {
     std::vector<FwComp> comps;
     std::vector<int64_t> pre_conv, pre_panel, pre_tile, pre_tile_n, pre_tile_s;   // _n: narrow, _s: small tiles
     std::vector<int> active;                // active[r] = components with n > 64 r
-    size_t off_status = 0, off_comps = 0, off_pconv = 0, off_ppanel = 0, off_ptile = 0, off_ptile_n = 0, off_ptile_s = 0;
+    size_t off_status = 0, off_comps = 0, off_pconv = 0, off_ppanel = 0, off_ptile = 0, off_ptile_n = 0, off_ptile_s = 0, off_sided = 0;
     size_t off_rb = 0, off_any = 0, off_lanes = 0, off_exact = 0, total = 0;
     size_t off_occ = 0, occ_bytes = 0, off_plist = 0, off_tlist = 0, off_counters = 0;
 };
@@ -1062,6 +1065,12 @@ static void build_plan(FwPlan &P, int64_t count, const int64_t *sizes, const int
                  256);
     P.off_counters = o; o = align_up(o + 64, 256);
     P.off_lanes = o; o = align_up(o + (size_t)lanes * lane, 256);
+    // one matrix: the masks of fw_sided.cuh
+    P.off_sided = o;
+    if (count == 1 && lane == 4) {
+        const size_t np = (size_t)P.comps[0].np;
+        o = align_up(o + 2 * np * (np / 64) * 8 + 2 * np * 4, 256);
+    }
     P.off_exact = o; o = align_up(o + 3 * align_up((size_t)maxn, 32) * elem_bytes + 256, 256);
     P.total = o;
 }
@@ -1226,6 +1235,8 @@ static int launch_blocked(const FwPlan &P, const T *in, T *out, unsigned char *w
     return RBG_OK;
 }
 
+#include "fw_sided.cuh"
+
 static void decode_seq(long long seq, int64_t n, rbg_result_t *r) {
     if (seq < 0 || seq == LLONG_MAX) { r->k = r->i = r->j = -1; return; }
     r->j = seq % n;
@@ -1311,8 +1322,8 @@ static bool dag_path_allowed(uint32_t mode) {
     return !(mode & (RBG_MODE_NO_DAG | RBG_MODE_TRIANGULAR | RBG_MODE_FORCE_EXACT | RBG_MODE_FORCE_WIDE));
 }
 
-// Single matrix: the DAG path for int32 / int64 matrices numbered in a topological order, else
-// 32-bit lanes, then 64-bit lanes when 64-bit values need them, then the exact sequential-order
+// Single matrix: the DAG path for int32 / int64 matrices that are acyclic with short rows, the block
+// steps of fw_sided.cuh for ones in a topological order with wide rows, else 32-bit lanes, then 64-bit lanes when 64-bit values need them, then the exact sequential-order
 // kernel for anything outside the clean regime, cycles and top-bit products.  A matrix whose
 // loop the DAG path found to compute a product reaching bit 31 (`top_bit`, from the DAG path of
 // this call or of the batch that hands it over) skips the 32-bit lanes, which could only report
@@ -1325,6 +1336,7 @@ static int fw_dense_t(int64_t n, const T *in, int64_t ld_in, T *out, int64_t ld_
     const int triangular = (mode & RBG_MODE_TRIANGULAR) ? 1 : 0;
     memset(res, 0, sizeof(*res));
     res->k = res->i = res->j = -1;
+    char side = TRI_OPEN;
     if constexpr (std::is_same<T, int32_t>::value || std::is_same<T, int64_t>::value) {
         if (try_dag && dag_path_allowed(mode)) {
             const int64_t zero = 0;
@@ -1334,11 +1346,24 @@ static int fw_dense_t(int64_t n, const T *in, int64_t ld_in, T *out, int64_t ld_
             if (rc) return rc;
             if (closed == TRI_CLOSED) return RBG_OK;
             top_bit = closed == TRI_TOP_BIT;
+            side = closed == TRI_WIDE_BELOW || closed == TRI_WIDE_ABOVE ? closed : TRI_OPEN;
         }
     }
     DevStatus h;
     FwPlan P;
     single_plan<uint32_t>(P, n, ld_in, ld_out, triangular, (int)sizeof(T));
+    if constexpr (std::is_same<T, int32_t>::value || std::is_same<T, int64_t>::value) {
+        if (side != TRI_OPEN) {              // clean, in a topological order, rows too wide for the DAG path
+            int rc = upload_plan(P, ws, stream);
+            if (!rc) rc = launch_sided<T>(P, in, ld_in, out, ws, stream, side == TRI_WIDE_ABOVE);
+            if (!rc) rc = read_status(reinterpret_cast<DevStatus *>(ws + P.off_status), &h, 1, stream);
+            if (rc) return rc;
+            if (!(h.flags & (RBG_EV_UNCLEAN | RBG_EV_CYCLE | RBG_EV_WIDE | RBG_EV_RISK))) {
+                result_from_blocked(h, RBG_PATH_BLOCKED32, res);
+                return RBG_OK;
+            }
+        }
+    }
     if (!(mode & RBG_MODE_FORCE_EXACT) && !(top_bit && sizeof(T) == 4)) {
         bool wide = sizeof(T) == 8 && ((mode & RBG_MODE_FORCE_WIDE) || top_bit);
         if (!wide) {
@@ -1554,8 +1579,8 @@ static int fw_batch_t(int64_t count, const int64_t *sizes, const int64_t *offset
     // components the DAG path found to reach bit 31 skip the batched 32-bit pass
     std::vector<int64_t> idx, top;
     for (int64_t i = 0; i < count; ++i) {
-        if (closed[(size_t)i] == TRI_OPEN) idx.push_back(i);
-        else if (closed[(size_t)i] == TRI_TOP_BIT) top.push_back(i);
+        if (closed[(size_t)i] == TRI_TOP_BIT) top.push_back(i);
+        else if (closed[(size_t)i] != TRI_CLOSED) idx.push_back(i);
     }
     for (int64_t i : top) {
         const int rc = fw_dense_t<T>(sizes[i], in + offsets[i], sizes[i], out + offsets[i], sizes[i], mode, ws,

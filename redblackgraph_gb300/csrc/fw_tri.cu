@@ -69,7 +69,7 @@ constexpr int32_t TRI_PENDING = 3;           // closed by the levels in a second
 
 // Result of one matrix, written on the device and read back once per call.
 struct TriOut {
-    int32_t verdict, diameter;               // verdict: TRI_OPEN, TRI_CLOSED, TRI_TOP_BIT or TRI_PENDING
+    int32_t verdict, diameter;               // verdict: TRI_OPEN .. TRI_WIDE_ABOVE or TRI_PENDING
     unsigned long long executed;
 };
 
@@ -1051,7 +1051,8 @@ tri_write_kernel(const T *__restrict__ in, int64_t ld_in, T *__restrict__ out, i
                  const DagCounters *dc, const unsigned *gflags,
                  const int64_t *__restrict__ row_off, const int32_t *__restrict__ row_len,
                  const int32_t *__restrict__ p_col, const int32_t *__restrict__ p_val, RowStats rs,
-                 const int *__restrict__ cfm, const unsigned long long *__restrict__ cprod, TriOut *__restrict__ res) {
+                 const int *__restrict__ cfm, const unsigned long long *__restrict__ cprod,
+                 const unsigned *__restrict__ cflags, TriOut *__restrict__ res) {
     constexpr int SEG = 2048 / (int)sizeof(T);
     constexpr int E = TriVec<T>::E;
     __shared__ __align__(16) T seg_all[TRI_ROWS][SEG];
@@ -1060,7 +1061,10 @@ tri_write_kernel(const T *__restrict__ in, int64_t ld_in, T *__restrict__ out, i
     if ((int64_t)blockIdx.x == pre[ci] && threadIdx.x == 0) {
         TriOut o;
         o.verdict = accepted ? TRI_CLOSED : tri_top_bit(ci, ckind, cam, cbad, dc, gflags) ? TRI_TOP_BIT
-                    : ckind[ci] == KIND_PENDING ? TRI_PENDING : TRI_OPEN;
+                    : ckind[ci] == KIND_PENDING ? TRI_PENDING
+                    : (cflags[ci] & ~(TF_BELOW | TF_ABOVE)) != TF_WIDE ? TRI_OPEN
+                    : !(cflags[ci] & TF_ABOVE) ? TRI_WIDE_BELOW
+                    : !(cflags[ci] & TF_BELOW) ? TRI_WIDE_ABOVE : TRI_OPEN;
         o.diameter = cfm[ci] > 0 ? cfm[ci] : 0;
         o.executed = cprod[ci];
         res[ci] = o;
@@ -1381,7 +1385,7 @@ int tri_enqueue(const TriShape &sh, const TriLayout &L, const T *in, T *out, cud
         tri_write_kernel<T><<<(unsigned)sh.ctas, TRI_THREADS, 0, s>>>(in, sh.ld_in, out, sh.ld_out, L.dc, L.dpre,
                                                                       count, L.ckind, L.cam, L.cbad, *dcount,
                                                                       L.gflags, L.row_off, L.row_len, L.p_col,
-                                                                      L.p_val, rs, L.cfm, L.cprod, L.res);
+                                                                      L.p_val, rs, L.cfm, L.cprod, L.cflags, L.res);
         RBG_CUDA_TRY(cudaGetLastError());
         timer_end(7, t, s);
     }
@@ -1608,7 +1612,7 @@ template <typename T> int tri_short(TriCall<T> &c, bool second) {
         tri_write_kernel<T><<<(unsigned)c.sh.ctas, TRI_THREADS, 0, s>>>(c.in, c.ld_in, c.out, c.ld_out, L.dc, L.dpre,
                                                                        count, L.ckind, L.cam, L.cbad, L.counters,
                                                                        L.gflags, L.row_off, L.row_len, L.p_col,
-                                                                       L.p_val, c.rs, L.cfm, L.cprod, L.res);
+                                                                       L.p_val, c.rs, L.cfm, L.cprod, L.cflags, L.res);
         timer_end(7, t, s);
     }
     RBG_CUDA_TRY(cudaGetLastError());

@@ -173,7 +173,9 @@ constexpr int DAG_GRAPH_CHUNK = 4;           // levels per iteration of the grap
 // `ws_bytes`); a workspace too small for a closure leaves its components to the other paths.
 // ld_in / ld_out are the row strides of every block (0: each block's own n).  With
 // RBG_MODE_GRAPH in `mode` the whole sequence is replayed from a cached CUDA graph.
-constexpr char TRI_OPEN = 0, TRI_CLOSED = 1, TRI_TOP_BIT = 2;
+// closed[i] = TRI_WIDE_BELOW / TRI_WIDE_ABOVE marks one left alone for rows of more than 16 entries
+// only: clean, every entry on that side of the diagonal.
+constexpr char TRI_OPEN = 0, TRI_CLOSED = 1, TRI_TOP_BIT = 2, TRI_WIDE_BELOW = 4, TRI_WIDE_ABOVE = 5;
 template <typename T>
 int tri_batch(int64_t count, const int64_t *sizes, const int64_t *in_off, const int64_t *out_off, int64_t ld_in,
               int64_t ld_out, const T *in, T *out, rbg_result_t *results, char *closed, unsigned char *ws,

@@ -944,6 +944,7 @@ tri_order_kernel(const TriComp *__restrict__ comps, int32_t *ckind, const int32_
     __syncthreads();                         // (the lists' writes are visible to the CTA)
     // levels: 8 lanes per frontier vertex
     int h = 0, tail = s_tail;
+    __syncthreads();                         // everyone has the first level's end before it moves
     while (h < tail) {                       // block-uniform
         for (int q = h + (tid >> 3); q < tail; q += TRI_ORDER_THREADS / 8) {
             const int v = S.list[q];

@@ -482,16 +482,8 @@ __global__ void dag_roots_kernel(DagArgs a) {
     }
 }
 
-// The level a kernel works on: L itself, or L levels past the device-resident level counter *Lp
-// (the level loop run as a CUDA-graph while node); false past the last possible level.
-__device__ __forceinline__ bool dag_level(const DagArgs &a, int64_t &L, const int64_t *Lp) {
-    if (Lp) L += *Lp;
-    return L < a.n;
-}
-
 // Level L + 1 from level L: every child edge of the level's vertices, flattened over the warp.
-__global__ void dag_discover_kernel(DagArgs a, int64_t L, const int64_t *Lp) {
-    if (!dag_level(a, L, Lp)) return;
+__global__ void dag_discover_kernel(DagArgs a, int64_t L) {
     const int lane = threadIdx.x & 31;
     const int64_t s = a.lb[L], e = a.lb[L + 1];
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -635,8 +627,7 @@ __device__ __forceinline__ DagRec dag_shfl_rec(const DagRec &r, int src) {
 // largest of the four sent three quarters of a pedigree forest's iterations down the slowest
 // path).  Lanes 8i..8i+7 hold row i's record; the next four records are read before the current
 // rows are filled.  Block 0 closes the level's range.
-__global__ void __launch_bounds__(DG_WARPS * 32) dag_fill_kernel(DagArgs a, int64_t L, const int64_t *Lp) {
-    if (!dag_level(a, L, Lp)) return;
+__global__ void __launch_bounds__(DG_WARPS * 32) dag_fill_kernel(DagArgs a, int64_t L) {
     extern __shared__ __align__(16) unsigned char dg_smem[];
     const int wi = threadIdx.x >> 5, lane = threadIdx.x & 31;
     DagTable<DG_WSLOTS> &H = reinterpret_cast<DagTable<DG_WSLOTS> *>(dg_smem)[wi];
@@ -730,8 +721,7 @@ __global__ void __launch_bounds__(DG_WARPS * 32) dag_fill_kernel(DagArgs a, int6
 }
 
 // One 512-thread block per row of level L with more than 256 candidates.
-__global__ void __launch_bounds__(DG_BTHREADS) dag_fill_block_kernel(DagArgs a, int64_t L, const int64_t *Lp) {
-    if (!dag_level(a, L, Lp)) return;
+__global__ void __launch_bounds__(DG_BTHREADS) dag_fill_block_kernel(DagArgs a, int64_t L) {
     extern __shared__ __align__(16) unsigned char dg_smem[];
     DagTable<DG_BSLOTS> &H = *reinterpret_cast<DagTable<DG_BSLOTS> *>(dg_smem);
     __shared__ int s_nd, s_ok;
@@ -1043,15 +1033,6 @@ __global__ void dag_len64_kernel(int64_t n, const int *row_len, int64_t *len64) 
         len64[v] = v < n ? row_len[v] : 0;
 }
 
-// One iteration of the graph's level loop has run DAG_GRAPH_CHUNK levels from *Lp: advance the
-// counter and keep looping while the next level holds a vertex (fill(L - 1) wrote lb[L]).
-__global__ void dag_advance_kernel(DagArgs a, int64_t *Lp, cudaGraphConditionalHandle h) {
-    if (threadIdx.x != 0) return;
-    const int64_t L = *Lp + DAG_GRAPH_CHUNK;
-    *Lp = L;
-    cudaGraphSetConditional(h, (L < a.n && (int64_t)*a.tail > a.lb[L]) ? 1u : 0u);
-}
-
 }  // namespace rbg
 
 using namespace rbg;
@@ -1183,16 +1164,16 @@ LevelLaunch level_launch() {
     return l;
 }
 
-void launch_level(const DagArgs &a, const LevelLaunch &l, int64_t L, const int64_t *Lp, cudaStream_t s) {
-    dag_fill_kernel<<<l.fill_grid, DG_WARPS * 32, l.wsm, s>>>(a, L, Lp);
-    dag_fill_block_kernel<<<l.block_grid, DG_BTHREADS, l.bsm, s>>>(a, L, Lp);
-    dag_discover_kernel<<<l.disc_grid, 256, 0, s>>>(a, L, Lp);
+void launch_level(const DagArgs &a, const LevelLaunch &l, int64_t L, cudaStream_t s) {
+    dag_fill_kernel<<<l.fill_grid, DG_WARPS * 32, l.wsm, s>>>(a, L);
+    dag_fill_block_kernel<<<l.block_grid, DG_BTHREADS, l.bsm, s>>>(a, L);
+    dag_discover_kernel<<<l.disc_grid, 256, 0, s>>>(a, L);
 }
 
 // Levels launched in chunks of 8 without waiting (every kernel reads its level's bounds from
 // device memory and exits at once on an empty level); the host looks at the frontier once per
 // chunk.
-int dag_levels_host(const DagArgs &a, const DagWs &w, cudaStream_t s, int64_t *launches) {
+int dag_levels(const DagArgs &a, const DagWs &w, cudaStream_t s) {
     const LevelLaunch l = level_launch();
     const int64_t chunk = 8;
     int64_t L = 0;
@@ -1200,8 +1181,7 @@ int dag_levels_host(const DagArgs &a, const DagWs &w, cudaStream_t s, int64_t *l
         const int64_t Lend = std::min<int64_t>(L + chunk, a.n);
         for (; L < Lend; ++L) {
             note_launches(3);
-            *launches += 3;
-            launch_level(a, l, L, nullptr, s);
+            launch_level(a, l, L, s);
         }
         RBG_CUDA_TRY(cudaGetLastError());
         // level L is empty when the order has not grown past its start (written by fill(L - 1))
@@ -1214,42 +1194,6 @@ int dag_levels_host(const DagArgs &a, const DagWs &w, cudaStream_t s, int64_t *l
         if (rc) return rc;
         if ((int64_t)tail <= start || L >= a.n) break;
     }
-    return RBG_OK;
-}
-
-// The level loop inside the graph being captured on `s`: a while node whose body runs
-// DAG_GRAPH_CHUNK levels from the device-resident counter and then lets dag_advance_kernel
-// decide whether to go on.  Nothing is read back by the host.
-int dag_levels_graph(const DagArgs &a, const DagWs &w, cudaStream_t s) {
-    const LevelLaunch l = level_launch();
-    int64_t *Lp = reinterpret_cast<int64_t *>(&w.cnt->level);
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    cudaGraph_t g = nullptr;
-    const cudaGraphNode_t *deps = nullptr;
-    size_t ndeps = 0;
-    RBG_CUDA_TRY(cudaStreamGetCaptureInfo(s, &st, nullptr, &g, &deps, nullptr, &ndeps));
-    if (st != cudaStreamCaptureStatusActive || !g) return RBG_ERR_INVALID;
-    cudaGraphConditionalHandle h;
-    RBG_CUDA_TRY(cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault));
-    cudaGraphNodeParams p = {};
-    p.type = cudaGraphNodeTypeConditional;
-    p.conditional.handle = h;
-    p.conditional.type = cudaGraphCondTypeWhile;
-    p.conditional.size = 1;
-    cudaGraphNode_t node;
-    RBG_CUDA_TRY(cudaGraphAddNode(&node, g, deps, nullptr, ndeps, &p));
-    cudaGraph_t body = p.conditional.phGraph_out[0];
-    // the body is recorded from a second stream captured into it
-    static thread_local cudaStream_t side = nullptr;
-    if (!side) RBG_CUDA_TRY(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
-    RBG_CUDA_TRY(cudaStreamBeginCaptureToGraph(side, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    for (int t = 0; t < DAG_GRAPH_CHUNK; ++t) launch_level(a, l, t, Lp, side);
-    dag_advance_kernel<<<1, 32, 0, side>>>(a, Lp, h);
-    const cudaError_t le = cudaGetLastError();
-    cudaGraph_t got = nullptr;
-    const cudaError_t ee = cudaStreamEndCapture(side, &got);
-    if (le != cudaSuccess || ee != cudaSuccess) return RBG_ERR_CUDA;
-    RBG_CUDA_TRY(cudaStreamUpdateCaptureDependencies(s, &node, nullptr, 1, cudaStreamSetCaptureDependencies));
     return RBG_OK;
 }
 
@@ -1267,28 +1211,6 @@ int sm_count() {
         sms[dev] = v > 0 ? v : 152;   // every thread writes the same value
     }
     return sms[dev];
-}
-
-size_t dag_workspace_for(int64_t n, int64_t nnz_bound) { return dag_layout(n, nnz_bound, nullptr, nullptr); }
-
-int dag_enqueue(const rbg_csr_t *A, int64_t nnz_bound, void *workspace, int32_t *pool_cols, int32_t *pool_vals,
-                int64_t pool_capacity, int64_t *row_off, int32_t *row_len, cudaStream_t s, bool captured,
-                DagCounters **counters, DagChildren *kids, int64_t *launches) {
-    const int64_t n = A->n_rows;
-    DagWs w;
-    dag_layout(n, nnz_bound, reinterpret_cast<unsigned char *>(workspace), &w);
-    *counters = w.cnt;
-    if (kids) *kids = DagChildren{w.coff, w.children};
-    int rc = dag_configure();
-    if (rc) return rc;
-    const DagArgs a = dag_args(n, A, w, pool_cols, pool_vals, pool_capacity, row_off, row_len);
-    RBG_CUDA_TRY(cudaMemsetAsync(w.cnt, 0, sizeof(DagCounters), s));
-    RBG_CUDA_TRY(cudaMemsetAsync(row_len, 0xff, (size_t)n * 4, s));   // -1: not closed (never placed, in the end)
-    rc = dag_front(a, w, s);
-    if (rc) return rc;
-    *launches += 4;
-    if (n == 0) return RBG_OK;
-    return captured ? dag_levels_graph(a, w, s) : dag_levels_host(a, w, s, launches);
 }
 
 }  // namespace rbg
@@ -1352,8 +1274,7 @@ extern "C" int32_t rbg_dag_closure_mode(const rbg_csr_t *A, uint32_t mode, void 
         dag_layout(n, annz, reinterpret_cast<unsigned char *>(workspace), &w);
         a = dag_args(n, A, w, pool_cols, pool_vals, pool_capacity, row_off, row_len);
         rc = dag_front(a, w, s);
-        int64_t launched = 0;
-        if (!rc) rc = dag_levels_host(a, w, s, &launched);
+        if (!rc) rc = dag_levels(a, w, s);
         if (rc) return rc;
         HostStaging hs(s, 256);
         rc = hs.down(&c, w.cnt, sizeof(c));

@@ -140,39 +140,23 @@ struct RowStats {
     }
 };
 
-// dag.cu: the closure by levels as an enqueue-only sequence for callers inside this library.
-// The workspace is laid out for at most `nnz_bound` stored entries of A, so nothing is read back
-// before the levels.  With `captured` the stream is being captured into a CUDA graph and the
-// level loop becomes a while node that the device ends when a level comes out empty (no host
-// synchronisation at all); otherwise the host looks at the frontier once per chunk of levels.
-// The device counters (DagCounters) are left in the workspace for the caller to read later.
+// The device counters of a closure by rows (dag.cu; fw_tri.cu uses reserved and flags).
 struct DagCounters {
     int placed, nwide, flags, nlevels;       // flags: 1 pool too small, 2 row past the block table
     unsigned long long reserved, max_abs, total;
-    long long level;                         // the graph loop's level counter
     int tile_rows, tile_levels;              // rows closed without levels, and their deepest level + 1
 };
-struct DagChildren {         // children lists of the levels' graph, kept in the workspace
-    const int64_t *coff;
-    const int32_t *children;
-};
-size_t dag_workspace_for(int64_t n, int64_t nnz_bound);
-int dag_enqueue(const rbg_csr_t *A, int64_t nnz_bound, void *workspace, int32_t *pool_cols, int32_t *pool_vals,
-                int64_t pool_capacity, int64_t *row_off, int32_t *row_len, cudaStream_t s, bool captured,
-                DagCounters **counters, DagChildren *kids, int64_t *launches);
-constexpr int DAG_GRAPH_CHUNK = 4;           // levels per iteration of the graph's while node
 
 // fw_tri.cu: the components of an int32 or int64 batch that are acyclic and in the clean regime
-// (at most 16 off-diagonal entries per row, at most 8192 rows), closed through the DAG closure by
-// levels (in any numbering: off the topological order, searches from every vertex give
-// the diameter and the overflow decision); sets closed[i] = TRI_CLOSED and results[i] for each
+// (at most 16 off-diagonal entries per row, at most 8192 rows), closed by the DAG recurrence (in any
+// numbering: off the topological order, searches from every vertex give the diameter and the overflow
+// decision); sets closed[i] = TRI_CLOSED and results[i] for each
 // of them and leaves every other component untouched.  closed[i] = TRI_TOP_BIT marks a component
 // the closure went through completely whose loop computes a product reaching bit 31: 32-bit
 // lanes would only report that risk, so the caller goes on with 64-bit lanes (int64) or the
 // exact kernel (int32).  Scratch comes from the caller's workspace (`ws`,
 // `ws_bytes`); a workspace too small for a closure leaves its components to the other paths.
-// ld_in / ld_out are the row strides of every block (0: each block's own n).  With
-// RBG_MODE_GRAPH in `mode` the whole sequence is replayed from a cached CUDA graph.
+// ld_in / ld_out are the row strides of every block (0: each block's own n).
 // closed[i] = TRI_WIDE_BELOW / TRI_WIDE_ABOVE marks one left alone for rows of more than 16 entries
 // only: clean, every entry on that side of the diagonal.
 constexpr char TRI_OPEN = 0, TRI_CLOSED = 1, TRI_TOP_BIT = 2, TRI_WIDE_BELOW = 4, TRI_WIDE_ABOVE = 5;

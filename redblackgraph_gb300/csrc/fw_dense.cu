@@ -996,6 +996,12 @@ struct FwPlan {
     size_t off_occ = 0, occ_bytes = 0, off_plist = 0, off_tlist = 0, off_counters = 0;
 };
 
+// The masks of fw_sided.cuh for a matrix of n rows (any multiple of the block above it).
+inline size_t sided_mask_bytes(int64_t n) {
+    const size_t np = align_up((size_t)n, 64);
+    return 2 * np * (np / 64) * 8 + 2 * np * 4;
+}
+
 // sizes[i], in_off[i], out_off[i] of component i (input order); lane = bytes per lane word
 static void build_plan(FwPlan &P, int64_t count, const int64_t *sizes, const int64_t *in_off,
                        const int64_t *out_off, size_t lane, int triangular, int tile_bn,
@@ -1068,8 +1074,7 @@ static void build_plan(FwPlan &P, int64_t count, const int64_t *sizes, const int
     // one matrix: the masks of fw_sided.cuh
     P.off_sided = o;
     if (count == 1 && lane == 4) {
-        const size_t np = (size_t)P.comps[0].np;
-        o = align_up(o + 2 * np * (np / 64) * 8 + 2 * np * 4, 256);
+        o = align_up(o + sided_mask_bytes(P.comps[0].np), 256);
     }
     P.off_exact = o; o = align_up(o + 3 * align_up((size_t)maxn, 32) * elem_bytes + 256, 256);
     P.total = o;
@@ -1815,7 +1820,8 @@ static size_t batch_workspace_uncached(int32_t dtype, int64_t count, const int64
                TileCfg<uint32_t>::BN, dtype_bytes(dtype));
     int64_t maxn = 0;
     for (int64_t i = 0; i < count; ++i) maxn = std::max(maxn, sizes[i]);
-    return std::max(P.total, single_workspace(maxn, dtype));
+    // a matrix left by the batch is closed by itself in the same scratch, which then also holds its masks
+    return std::max(P.total + sided_mask_bytes(maxn), single_workspace(maxn, dtype));
 }
 
 extern "C" int32_t rbg_fw_batch_workspace_bytes(int32_t dtype, int64_t count, const int64_t *sizes,

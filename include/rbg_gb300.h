@@ -486,8 +486,9 @@ int32_t rbg_cc_compact_fill(int64_t n, const int32_t *label, const int32_t *loca
  * Component-wise closure straight from the CSR graph (no dense blocks) when every component is
  * numbered in a topological order (its off-diagonal entries all below, or all above, the
  * diagonal) and in the clean regime: the DAG path of rbg_fw_batch applied to the graph.  The
- * sequence is rbg_cc_dag_classify -> rbg_cc_dag_edges -> rbg_dag_closure on the edges (its row
- * pool is read as it is) -> rbg_cc_dag_stats -> rbg_cc_dag_merge_count / _fill; values and diameters are
+ * sequence is rbg_cc_dag_classify -> rbg_cc_dag_edges -> rbg_cc_dag_close, or where that does not take
+ * the graph rbg_dag_closure on the edges (its row pool is read as it is) and rbg_cc_dag_stats ->
+ * rbg_cc_dag_merge_count / _fill; values and diameters are
  * those of merge_component_matrices over the reference's per-component closures
  * (redblackgraph/sparse/csgraph/transitive_closure.py:85-195).  Components come from
  * rbg_cc_label; `workspace` is its workspace.
@@ -520,6 +521,20 @@ int32_t rbg_cc_dag_stats(int64_t n, int64_t ncomp, const int32_t *label, const i
                          const rbg_csr_t *edges, const int64_t *row_off, const int32_t *row_len,
                          const int32_t *pool_cols, const int32_t *pool_vals, const int32_t *diag,
                          int32_t *top_msb, int32_t *first_msb, int32_t *comp_max, rbg_stream_t stream);
+
+/* rbg_dag_closure on the edges and rbg_cc_dag_stats in one pass over the rows, without levels: a warp
+ * per row waits for its parents.  *closed = 1 when the rows (row_off, row_len, pool_cols, pool_vals) and
+ * the statistics are complete; 0 when the call is not for this path (a row of more than 16 entries, a
+ * component that spans more than 8192 vertex numbers, entries on the other side of the diagonal than
+ * comp_kind says, or a pool too small): then call the two others.  comp_kind as above, without 0.
+ * Synchronises `stream`. */
+int32_t rbg_cc_dag_close_workspace_bytes(int64_t n, int64_t *bytes);
+int32_t rbg_cc_dag_close(int64_t n, int64_t ncomp, const int32_t *label, const int32_t *local,
+                         const int64_t *start, const int32_t *sorted_vertex, const int32_t *comp_kind,
+                         const rbg_csr_t *edges, const int32_t *diag, void *workspace, int64_t workspace_bytes,
+                         int32_t *pool_cols, int32_t *pool_vals, int64_t pool_capacity, int64_t *row_off,
+                         int32_t *row_len, int32_t *top_msb, int32_t *first_msb, int32_t *comp_max,
+                         int32_t *closed, rbg_stream_t stream);
 
 /* Row pointers (device, n + 1) of the merged matrix: each closure row (row_len from the row
  * pool) plus its diagonal value when nonzero; *nnz (host) its size.  Synchronises `stream`. */

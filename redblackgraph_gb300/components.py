@@ -150,6 +150,30 @@ DAG_TILE_ROWS = 64        # vertices of a piece closed without levels (rbg_dag_c
 _UNCLEAN, _BELOW, _ABOVE = 1, 2, 4
 
 
+def _close_rows(E, comps: Components, kind, diag, top, first, cmax, sh):
+    """The closure rows of the edges ``E`` as DagRows and the components' statistics (rbg_cc_dag_close), or
+    None when the graph is not for that path."""
+    from .dag import DagRows
+    n, dev = comps.n, E.indptr.device
+    L = _lib.load()
+    nb = ctypes.c_int64(0)
+    _lib.check(L.rbg_cc_dag_close_workspace_bytes(n, ctypes.byref(nb)), "cc_dag_close")
+    ws = torch.empty(nb.value, dtype=torch.uint8, device=dev)
+    row_off = torch.empty(n, dtype=torch.int64, device=dev)
+    row_len = torch.empty(n, dtype=torch.int32, device=dev)
+    cap = max(16 * E.nnz + n, 1024)
+    cols = torch.empty(cap, dtype=torch.int32, device=dev)
+    vals = torch.empty(cap, dtype=torch.int32, device=dev)
+    closed = ctypes.c_int32(0)
+    ec = E.cstruct()
+    _lib.check(L.rbg_cc_dag_close(n, comps.count, comps.label.data_ptr(), comps.local.data_ptr(), comps.start.data_ptr(),
+                                  comps.sorted_vertex.data_ptr(), kind.data_ptr(), ctypes.byref(ec), diag.data_ptr(),
+                                  ws.data_ptr(), ws.numel(), cols.data_ptr(), vals.data_ptr(), cap, row_off.data_ptr(),
+                                  row_len.data_ptr(), top.data_ptr(), first.data_ptr(), cmax.data_ptr(),
+                                  ctypes.byref(closed), sh), "cc_dag_close")
+    return DagRows(cols, vals, row_off, row_len, -1) if closed.value else None
+
+
 def dag_component_closure(indptr: torch.Tensor, indices: torch.Tensor, data: torch.Tensor, n: int,
                           comps: Components, method: str, densify_threshold: int, stream=None):
     """Component-wise closure straight from the CSR graph when every component is numbered in a
@@ -185,23 +209,28 @@ def dag_component_closure(indptr: torch.Tensor, indices: torch.Tensor, data: tor
     _lib.check(L.rbg_cc_dag_edges(n, ip, ij, iv, eptr.data_ptr(), ecol.data_ptr(), evals.data_ptr(), sh),
                "cc_dag_edges")
     E = DeviceCSR(eptr, ecol[:ne.value], evals[:ne.value], (n, n))
-    # the look for small pieces pays when half of the vertices lie in components a tile can hold (a
-    # forest of 2,000,000 vertices in families of 64: 3.15 to 0.92 ms; one of 300 pedigrees of up to
-    # 4096 vertices: 2.01 to 2.12 ms with it)
-    tiles = 2 * int(comps.sizes[comps.sizes <= DAG_TILE_ROWS].sum()) >= n
-    try:
-        C, _, _ = dag_closure_device(E, stream, gather=False, tiles=tiles)    # the row pool, read in place
-    except RowTooWide:
-        return None
     top = torch.empty(k, dtype=torch.int32, device=dev)
     first = torch.empty(k, dtype=torch.int32, device=dev)
     cmax = torch.empty(k, dtype=torch.int32, device=dev)
     ec = E.cstruct()
+    # the look for small pieces pays when half of the vertices lie in components a tile can hold (a
+    # forest of 2,000,000 vertices in families of 64: 3.15 to 0.92 ms); for larger components rows that
+    # wait for their parents beat levels (1024 pedigrees of up to 4096 vertices: 0.99 to 0.78 ms
+    # with the statistics)
+    tiles = 2 * int(comps.sizes[comps.sizes <= DAG_TILE_ROWS].sum()) >= n
+    C = None if tiles else _close_rows(E, comps, kind, diag, top, first, cmax, sh)
+    closed = C is not None
+    if not closed:
+        try:
+            C, _, _ = dag_closure_device(E, stream, gather=False, tiles=tiles)    # the row pool, read in place
+        except RowTooWide:
+            return None
     pool = (C.row_off.data_ptr(), C.row_len.data_ptr(), C.cols.data_ptr(), C.vals.data_ptr())
-    _lib.check(L.rbg_cc_dag_stats(n, k, comps.label.data_ptr(), comps.local.data_ptr(), comps.start.data_ptr(),
-                                  comps.sorted_vertex.data_ptr(), kind.data_ptr(), ctypes.byref(ec), *pool,
-                                  diag.data_ptr(), top.data_ptr(), first.data_ptr(), cmax.data_ptr(), sh),
-               "cc_dag_stats")
+    if not closed:
+        _lib.check(L.rbg_cc_dag_stats(n, k, comps.label.data_ptr(), comps.local.data_ptr(), comps.start.data_ptr(),
+                                      comps.sorted_vertex.data_ptr(), kind.data_ptr(), ctypes.byref(ec), *pool,
+                                      diag.data_ptr(), top.data_ptr(), first.data_ptr(), cmax.data_ptr(), sh),
+                   "cc_dag_stats")
     st = torch.stack([top, first, cmax]).cpu().numpy()
     if (st[0] >= 31).any():
         return None

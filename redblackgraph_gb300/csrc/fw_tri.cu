@@ -38,6 +38,7 @@
 // them with the same kernel, runs the searches and writes them.  Every accept / reject decision is
 // made on the device; scratch is carved from the caller's workspace.
 #include <cuda_runtime.h>
+#include <cub/cub.cuh>
 #include <string.h>
 #include <algorithm>
 #include <vector>
@@ -630,15 +631,86 @@ struct TriTickets {
     int nq, places, batch, block;
 };
 
+// A row to close: its matrix, the kind, vertices and first row of that, the row, its number of entries and
+// (TriCsrRows) their first position.
+struct TriPlace {
+    int ci, kind, n, base, g, cnt, e0;
+};
+
+// The rows of a batch of dense matrices: the scan's slots.
+struct TriSlotRows {
+    static constexpr bool CSR = false;
+    TriTickets tk;
+    const TriComp *comps;
+    const unsigned *cflags, *cbad;
+    int32_t *ckind;
+    const int32_t *order, *col, *val, *cnt;
+    __device__ __forceinline__ TriPlace at(int p) const {
+        int2 pl;
+        if (tk.place) {
+            pl = tk.place[p];
+        } else {
+            pl.y = tk.nq == tk.places ? p : tri_place_row(tk.qstart, tk.nq, p);   // one matrix: its rows
+            pl.x = tk.tmat[p - tk.qstart[pl.y]];
+        }
+        TriPlace m{pl.x, KIND_NONE, (int)comps[pl.x].n, (int)comps[pl.x].row_base, 0, 0, 0};
+        const unsigned f = cflags[m.ci];
+        if (order) {                         // the matrices in any numbering (tri_order_kernel)
+            m.kind = cbad[m.ci] ? KIND_NONE : ckind[m.ci];
+        } else {
+            m.kind = (f & (TF_UNCLEAN | TF_WIDE)) ? KIND_NONE
+                     : ((f & TF_BELOW) && (f & TF_ABOVE)) ? KIND_PENDING
+                     : (f & TF_ABOVE) ? KIND_ABOVE : KIND_BELOW;
+            if (pl.y == 0) ckind[m.ci] = m.kind;
+        }
+        if (m.kind > KIND_NONE) {
+            // a matrix with entries above the diagonal goes from its last row to its first
+            m.g = order ? order[m.base + pl.y] : m.base + (m.kind == KIND_ABOVE ? m.n - 1 - pl.y : pl.y);
+            m.cnt = cnt[m.g];                // at most TRI_CAP
+        }
+        return m;
+    }
+    __device__ __forceinline__ int64_t begin(int64_t g, int) const { return g * TRI_CAP; }
+    __device__ __forceinline__ int64_t row(int64_t g, int &n) const {
+        n = cnt[g];
+        return g * TRI_CAP;
+    }
+    __device__ __forceinline__ int column(int64_t e, int) const { return col[e]; }
+};
+
+// The components of a graph (CSR, the off-diagonal entries): the vertices in the order `order`, by their
+// place among their component's (from the last for entries above the diagonal); a component is the
+// matrix of its lowest to its highest vertex.
+struct TriCsrRows {
+    static constexpr bool CSR = true;
+    TriTickets tk;
+    const int32_t *order, *label, *kind, *sorted_vertex;
+    const int64_t *start, *ptr;
+    const int32_t *col, *val;
+    const int32_t *diag;
+    int *cmax;                               // per component, the largest value of its rows
+    __device__ __forceinline__ TriPlace at(int p) const {
+        const int v = order[p], c = label[v];
+        const int64_t e0 = ptr[v], s0 = start[c], s1 = start[c + 1];
+        const int lo = sorted_vertex[s0];
+        return TriPlace{c, kind[c], sorted_vertex[s1 - 1] - lo + 1, lo, v, (int)(ptr[v + 1] - e0), (int)e0};
+    }
+    __device__ __forceinline__ int64_t begin(int64_t, int e0) const { return e0; }
+    __device__ __forceinline__ int64_t row(int64_t g, int &n) const {
+        const int64_t e0 = ptr[g];
+        n = (int)(ptr[g + 1] - e0);
+        return e0;
+    }
+    __device__ __forceinline__ int column(int64_t e, int base) const { return col[e] - base; }
+};
+
+template <typename Rows>
 __global__ void __launch_bounds__(32 * TRI_PULL_WARPS, TRI_PULL_CTAS)
-tri_pull_kernel(TriTickets tk, const TriComp *__restrict__ comps,
-                const unsigned *__restrict__ cflags, const int32_t *__restrict__ slot_col,
-                const int32_t *__restrict__ slot_val, const int32_t *__restrict__ row_cnt,
-                unsigned long long *state, int64_t *__restrict__ row_off, int32_t *__restrict__ row_len,
+tri_pull_kernel(Rows A, unsigned long long *state, int64_t *__restrict__ row_off, int32_t *__restrict__ row_len,
                 int32_t *p_col, int32_t *p_val, int64_t capacity, DagCounters *dc, int *ticket,
-                int32_t *__restrict__ ckind, int *__restrict__ cam, int *__restrict__ cfm,
-                int32_t *__restrict__ row_prods, const int32_t *__restrict__ order,
-                const unsigned *__restrict__ cbad) {
+                int *__restrict__ cam, int *__restrict__ cfm, int32_t *__restrict__ row_prods) {
+    const TriTickets &tk = A.tk;
+    if (Rows::CSR && (dc->flags & TRI_BAD_ROW)) return;   // set before the launch
     __shared__ TriPullWarp warps[TRI_PULL_WARPS];
     TriPullWarp &S = warps[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
@@ -652,43 +724,17 @@ tri_pull_kernel(TriTickets tk, const TriComp *__restrict__ comps,
         if ((int64_t)t * tk.batch >= tk.places) return;
         // lane u: the ticket's place u
         const int here = min(tk.batch, tk.places - t * tk.batch);
-        int m_ci = 0, m_kind = KIND_NONE, m_n = 0, m_base = 0, m_g = 0, m_cnt = 0;
-        if (lane < here) {
-            const int p = t * tk.batch + lane;
-            int2 pl;
-            if (tk.place) {
-                pl = tk.place[p];
-            } else {
-                pl.y = tk.nq == tk.places ? p : tri_place_row(tk.qstart, tk.nq, p);   // one matrix: its rows
-                pl.x = tk.tmat[p - tk.qstart[pl.y]];
-            }
-            m_ci = pl.x;
-            const unsigned f = cflags[m_ci];
-            m_n = (int)comps[m_ci].n;
-            m_base = (int)comps[m_ci].row_base;
-            if (order) {                     // the matrices in any numbering (tri_order_kernel)
-                m_kind = cbad[m_ci] ? KIND_NONE : ckind[m_ci];
-            } else {
-                m_kind = (f & (TF_UNCLEAN | TF_WIDE)) ? KIND_NONE
-                         : ((f & TF_BELOW) && (f & TF_ABOVE)) ? KIND_PENDING
-                         : (f & TF_ABOVE) ? KIND_ABOVE : KIND_BELOW;
-                if (pl.y == 0) ckind[m_ci] = m_kind;
-            }
-            if (m_kind > KIND_NONE) {
-                // a matrix with entries above the diagonal goes from its last row to its first
-                m_g = order ? order[m_base + pl.y] : m_base + (m_kind == KIND_ABOVE ? m_n - 1 - pl.y : pl.y);
-                m_cnt = row_cnt[m_g];        // at most TRI_CAP
-            }
-        }
-        int m_am = -1, m_fm = -1, m_prods = 0;   // lane u: the statistics of place u
+        TriPlace m{0, KIND_NONE, 0, 0, 0, 0, 0};
+        if (lane < here) m = A.at(t * tk.batch + lane);
+        int m_am = -1, m_fm = -1, m_prods = 0, m_mx = 0;   // lane u: the statistics of place u
         unsigned long long m_pub = 0;        // and its state, while it is not published yet
         // the closed rows' states, all with one fence (which a row otherwise waits for in every case)
         auto publish = [&]() {
             __syncwarp();
             if (m_pub) {
-                tri_release(state + m_g, m_pub);
-                row_off[m_g] = (int64_t)(m_pub >> TRI_STATE_LEN_BITS) - 1;
-                row_len[m_g] = (int)(m_pub & ((1u << TRI_STATE_LEN_BITS) - 1u));
+                tri_release(state + m.g, m_pub);
+                row_off[m.g] = (int64_t)(m_pub >> TRI_STATE_LEN_BITS) - 1;
+                row_len[m.g] = (int)(m_pub & ((1u << TRI_STATE_LEN_BITS) - 1u));
             }
             m_pub = 0;
             __syncwarp();
@@ -696,16 +742,17 @@ tri_pull_kernel(TriTickets tk, const TriComp *__restrict__ comps,
         int w_next = -1, v_next = 0;         // the next row's slots and its parents' states
         unsigned long long st_next = 0;
         {
-            const int g0 = __shfl_sync(0xffffffffu, m_g, 0);
-            if (lane < __shfl_sync(0xffffffffu, m_cnt, 0)) {
-                w_next = slot_col[(int64_t)g0 * TRI_CAP + lane];
-                v_next = slot_val[(int64_t)g0 * TRI_CAP + lane];
+            const int64_t e0 = A.begin(__shfl_sync(0xffffffffu, m.g, 0), __shfl_sync(0xffffffffu, m.e0, 0));
+            const int base0 = __shfl_sync(0xffffffffu, m.base, 0);
+            if (lane < __shfl_sync(0xffffffffu, m.cnt, 0)) {
+                w_next = A.column(e0 + lane, base0);
+                v_next = A.val[e0 + lane];
             }
         }
         for (int u = 0; u < here; ++u) {
-            const int kind = __shfl_sync(0xffffffffu, m_kind, u);   // warp-uniform
-            const int g = __shfl_sync(0xffffffffu, m_g, u), cnt = __shfl_sync(0xffffffffu, m_cnt, u);
-            const int n = __shfl_sync(0xffffffffu, m_n, u), base = __shfl_sync(0xffffffffu, m_base, u);
+            const int kind = __shfl_sync(0xffffffffu, m.kind, u);   // warp-uniform
+            const int g = __shfl_sync(0xffffffffu, m.g, u), cnt = __shfl_sync(0xffffffffu, m.cnt, u);
+            const int n = __shfl_sync(0xffffffffu, m.n, u), base = __shfl_sync(0xffffffffu, m.base, u);
             const int words = (n + 31) >> 5;
             int w = w_next, v = v_next, len = 0;
             int64_t off = 0;
@@ -713,15 +760,16 @@ tri_pull_kernel(TriTickets tk, const TriComp *__restrict__ comps,
             // the next row's slots, while this row is closed
             {
                 const int u1 = min(u + 1, here - 1);
-                const int g1 = __shfl_sync(0xffffffffu, m_g, u1), cnt1 = __shfl_sync(0xffffffffu, m_cnt, u1);
+                const int64_t e1 = A.begin(__shfl_sync(0xffffffffu, m.g, u1), __shfl_sync(0xffffffffu, m.e0, u1));
+                const int cnt1 = __shfl_sync(0xffffffffu, m.cnt, u1), base1 = __shfl_sync(0xffffffffu, m.base, u1);
                 st_next = 0;
                 if (u1 > u && lane < cnt1) {
-                    w_next = slot_col[(int64_t)g1 * TRI_CAP + lane];
-                    v_next = slot_val[(int64_t)g1 * TRI_CAP + lane];
+                    w_next = A.column(e1 + lane, base1);
+                    v_next = A.val[e1 + lane];
                 }
             }
             if (kind <= KIND_NONE) continue;
-            int am = -1, fm = lane < cnt ? dag_row_msb(v) : -1;
+            int am = -1, fm = lane < cnt ? dag_row_msb(v) : -1, mx = 0;
             int prods = 0;
             auto mark = [&]() {                  // the bitmap, with the row's own columns
                 for (int q = lane; q < words; q += 32) S.bm[q] = 0;
@@ -808,6 +856,7 @@ tri_pull_kernel(TriTickets tk, const TriComp *__restrict__ comps,
                 if (room && lead) {
                     p_col[at + rank] = base + cc;
                     p_val[at + rank] = vv;
+                    if (Rows::CSR) mx = vv;
                     if (kind == KIND_ABOVE) S.col[rank] = base + cc, S.val[rank] = vv;
                 }
                 __syncwarp();
@@ -878,10 +927,12 @@ tri_pull_kernel(TriTickets tk, const TriComp *__restrict__ comps,
                             p_col[at + q] = S.col[q];
                             p_val[at + q] = S.val[q];
                         }
+                    if (Rows::CSR)
+                        for (int q = lane; q < nd; q += 32) mx = max(mx, wide ? __ldcg(p_val + at + q) : S.val[q]);
                 }
             }
             if (u + 1 < here) {              // the next row's parents, while this row is stored
-                const int cnt1 = __shfl_sync(0xffffffffu, m_cnt, u + 1), base1 = __shfl_sync(0xffffffffu, m_base, u + 1);
+                const int cnt1 = __shfl_sync(0xffffffffu, m.cnt, u + 1), base1 = __shfl_sync(0xffffffffu, m.base, u + 1);
                 if (lane < cnt1) st_next = tri_acquire(state + base1 + w_next);
             }
             if (lane == 0 && !room) atomicOr(&dc->flags, 1);
@@ -901,9 +952,11 @@ tri_pull_kernel(TriTickets tk, const TriComp *__restrict__ comps,
                     if (q + half < nd) {
                         const int64_t k = wide ? (int64_t)__ldcg(p_col + at + q + half) : (int64_t)S.col[q + half];
                         const int kvv = wide ? __ldcg(p_val + at + q + half) : S.val[q + half];
-                        if (e < row_cnt[k]) {
-                            j = slot_col[k * TRI_CAP + e];
-                            pm = dag_row_msb(kvv) + dag_row_msb(slot_val[k * TRI_CAP + e]);
+                        int kn;
+                        const int64_t k0 = A.row(k, kn);
+                        if (e < kn) {
+                            j = A.column(k0 + e, base);
+                            pm = dag_row_msb(kvv) + dag_row_msb(A.val[k0 + e]);
                         }
                     }
                     am = max(am, pm);
@@ -919,14 +972,23 @@ tri_pull_kernel(TriTickets tk, const TriComp *__restrict__ comps,
             am = __reduce_max_sync(0xffffffffu, am);
             fm = __reduce_max_sync(0xffffffffu, fm);
             if (lane == u) m_am = am, m_fm = fm, m_prods = prods;
+            if (Rows::CSR) {
+                mx = __reduce_max_sync(0xffffffffu, mx);
+                if (lane == u) m_mx = mx;
+            }
         }
         publish();
         // a matrix's maxima rarely grow: an atomic per row on one word would be the kernel's bound
         // (any numbering: the searches take the statistics)
-        if (m_kind == KIND_BELOW || m_kind == KIND_ABOVE) {
-            row_prods[m_g] = m_prods;
-            if (m_am > __ldcg(cam + m_ci)) atomicMax(cam + m_ci, m_am);
-            if (m_fm > __ldcg(cfm + m_ci)) atomicMax(cfm + m_ci, m_fm);
+        if (m.kind == KIND_BELOW || m.kind == KIND_ABOVE) {
+            if constexpr (Rows::CSR) {
+                m_mx = max(m_mx, A.diag[m.g]);
+                if (m_mx > 0 && m_mx > __ldcg(A.cmax + m.ci)) atomicMax(A.cmax + m.ci, m_mx);
+            } else {
+                row_prods[m.g] = m_prods;
+            }
+            if (m_am > __ldcg(cam + m.ci)) atomicMax(cam + m.ci, m_am);
+            if (m_fm > __ldcg(cfm + m.ci)) atomicMax(cfm + m.ci, m_fm);
         }
     }
 }
@@ -1381,6 +1443,22 @@ template <typename T> struct TriCall {
     }
 };
 
+// Rows far more than resident warps: several rows per ticket (fewer fences and atomics on one word) while
+// the tickets in flight stay a small part of the rows, so that parents are seldom among them.  411 000
+// rows: 454 us with one row, 349 with three, 382 with five, 540 with eight; 227 000 rows: 266 us with one,
+// 212 with two, 247 with five.  And pool entries for some rows at once (the warps' rests together at most
+// a 16th of the pool).
+inline TriTickets tri_tickets(int64_t rows, int64_t pool, TriTickets t) {
+    const int64_t warps = (int64_t)TRI_PULL_CTAS * sm_count() * TRI_PULL_WARPS, part = TRI_PULL_PART * warps;
+    t.places = (int)rows;
+    t.batch = (int)std::min<int64_t>(TRI_PULL_BATCH, std::max<int64_t>(1, (rows + part / 2) / part));
+    t.block = rows >= 4 * warps ? (int)std::min<int64_t>(TRI_PULL_BLOCK, pool / (16 * warps)) : 0;
+    return t;
+}
+inline unsigned tri_pull_grid(int64_t rows) {
+    return (unsigned)std::min<int64_t>((rows + TRI_PULL_WARPS - 1) / TRI_PULL_WARPS, (int64_t)TRI_PULL_CTAS * sm_count());
+}
+
 // First pass: scan, closure kernel, write.  Second pass, over the same scratch, for the matrices the
 // first one left pending: their order, closure kernel, searches, write.
 template <typename T> int tri_pass(TriCall<T> &c, bool second) {
@@ -1411,20 +1489,12 @@ template <typename T> int tri_pass(TriCall<T> &c, bool second) {
             tri_order_kernel<<<(unsigned)count, fat ? 256 : TRI_ORDER_THREADS, tri_order_smem_bytes(c.sh.max_n), s>>>(
                 L.dc, L.ckind, L.slot_col, L.row_cnt, L.order, L.coff, L.kid_cnt, L.children, L.cbad, L.ticket,
                 L.gflags + 1, c.sh.max_n);
-        // rows far more than resident warps: several rows per ticket (fewer fences and atomics on one word)
-        // while the tickets in flight stay a small part of the rows, so that parents are seldom among
-        // them.  411 000 rows: 454 us with one row, 349 with three, 382 with five, 540 with eight; 227 000
-        // rows: 266 us with one, 212 with two, 247 with five.  And pool entries for some rows at once
-        // (the warps' rests together at most a 16th of the pool).
-        const int64_t most = (int64_t)TRI_PULL_CTAS * sm_count(), warps = most * TRI_PULL_WARPS;
-        const int batch = (int)std::min<int64_t>(TRI_PULL_BATCH, std::max<int64_t>(1, (c.sh.R + TRI_PULL_PART / 2 * warps) / (TRI_PULL_PART * warps)));
-        const int block = c.sh.R >= 4 * warps ? (int)std::min<int64_t>(TRI_PULL_BLOCK, L.pool / (16 * warps)) : 0;
-        const int64_t need = (c.sh.R + TRI_PULL_WARPS - 1) / TRI_PULL_WARPS;
-        tri_pull_kernel<<<(unsigned)std::min<int64_t>(need, most), 32 * TRI_PULL_WARPS, 0, s>>>(
-            TriTickets{fat ? L.place : nullptr, L.qstart, L.tmat, c.sh.nq, (int)c.sh.R, batch, block}, L.dc, L.cflags, L.slot_col, L.slot_val, L.row_cnt, L.state,
-            L.row_off, L.row_len, L.p_col, L.p_val, L.pool, L.counters, L.ticket, L.ckind, L.cam, L.cfm,
-            second ? nullptr : L.row_prods,
-            second ? L.order : nullptr, L.cbad);
+        const TriSlotRows rows{tri_tickets(c.sh.R, L.pool, TriTickets{fat ? L.place : nullptr, L.qstart, L.tmat, c.sh.nq}),
+                               L.dc, L.cflags, L.cbad, L.ckind, second ? L.order : nullptr, L.slot_col, L.slot_val,
+                               L.row_cnt};
+        tri_pull_kernel<<<tri_pull_grid(c.sh.R), 32 * TRI_PULL_WARPS, 0, s>>>(
+            rows, L.state, L.row_off, L.row_len, L.p_col, L.p_val, L.pool, L.counters, L.ticket, L.cam, L.cfm,
+            L.row_prods);
         timer_end(5, t, s);
     }
     if (second) {
@@ -1498,6 +1568,124 @@ template int tri_batch<int64_t>(int64_t, const int64_t *, const int64_t *, const
                                 cudaStream_t, const RowStats &);
 
 }  // namespace rbg
+
+// ------------------------------------------------------------------------------------------
+// The components of a graph
+// ------------------------------------------------------------------------------------------
+namespace rbg {
+namespace {
+
+struct CcWork {
+    int32_t *order, *vertex;                 // vertices by key; all vertices
+    unsigned short *key, *key_out;
+    unsigned long long *state;
+    DagCounters *counters;
+    int *ticket;
+    unsigned char *tmp;
+    size_t tmp_bytes, bytes;
+};
+
+void cc_work(unsigned char *base, int64_t n, CcWork &W) {
+    static thread_local LastSize size;
+    W.tmp_bytes = size.get(n, [&] {
+        size_t t = 0;
+        cub::DeviceRadixSort::SortPairs(nullptr, t, (unsigned short *)nullptr, (unsigned short *)nullptr,
+                                        (int32_t *)nullptr, (int32_t *)nullptr, (int)n, 0, 13);
+        return t;
+    });
+    const size_t N = (size_t)n;
+    Carve cv{base};
+    W.counters = cv.take<DagCounters>(1);
+    W.ticket = cv.take<int>(1);
+    W.state = cv.take<unsigned long long>(N);
+    W.order = cv.take<int32_t>(N);
+    W.vertex = cv.take<int32_t>(N);
+    W.key = cv.take<unsigned short>(N);
+    W.key_out = cv.take<unsigned short>(N);
+    W.tmp = cv.take<unsigned char>(W.tmp_bytes);
+    W.bytes = cv.off;
+}
+
+// A vertex's key is its place among its component's vertices, from the last where the entries lie above
+// the diagonal.  A row of more than TRI_CAP entries, or a component that spans more numbers than a
+// bitmap has bits, keeps the call off the path.
+__global__ void cc_key_kernel(int64_t n, const int32_t *__restrict__ label, const int32_t *__restrict__ local,
+                              const int64_t *__restrict__ start, const int32_t *__restrict__ sorted_vertex,
+                              const int32_t *__restrict__ kind, const int64_t *__restrict__ ptr,
+                              const int32_t *__restrict__ col, unsigned short *__restrict__ key, int32_t *__restrict__ vertex,
+                              unsigned long long *__restrict__ state, DagCounters *dc) {
+    bool off = false;
+    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
+        const int c = label[v];
+        const int64_t s0 = start[c], s1 = start[c + 1];
+        const int k = local[v];
+        const int64_t e0 = ptr[v], e1 = ptr[v + 1];
+        bool bad = e1 - e0 > TRI_CAP || e1 > INT32_MAX || sorted_vertex[s1 - 1] - sorted_vertex[s0] >= TRI_MAX_N;
+        for (int64_t e = e0; e < e1 && !bad; ++e) {
+            const int w = col[e];
+            bad = w < 0 || w >= n || label[w] != c || (kind[c] == KIND_ABOVE ? w <= v : w >= v);
+        }
+        off |= bad;
+        key[v] = (unsigned short)(kind[c] == KIND_ABOVE ? (int)(s1 - s0) - 1 - k : k);
+        vertex[v] = (int32_t)v;
+        state[v] = 0;
+    }
+    if (off) atomicOr(&dc->flags, TRI_BAD_ROW);
+}
+
+}  // namespace
+}  // namespace rbg
+
+extern "C" int32_t rbg_cc_dag_close_workspace_bytes(int64_t n, int64_t *bytes) {
+    if (n < 0 || n > INT32_MAX || !bytes) return RBG_ERR_INVALID;
+    rbg::CcWork W;
+    rbg::cc_work(nullptr, n, W);
+    *bytes = (int64_t)W.bytes + 256;
+    return RBG_OK;
+}
+
+extern "C" int32_t rbg_cc_dag_close(int64_t n, int64_t ncomp, const int32_t *label, const int32_t *local,
+                                    const int64_t *start, const int32_t *sorted_vertex, const int32_t *comp_kind,
+                                    const rbg_csr_t *edges, const int32_t *diag, void *workspace,
+                                    int64_t workspace_bytes, int32_t *pool_cols, int32_t *pool_vals,
+                                    int64_t pool_capacity, int64_t *row_off, int32_t *row_len, int32_t *top_msb,
+                                    int32_t *first_msb, int32_t *comp_max, int32_t *closed, rbg_stream_t stream) {
+    using namespace rbg;
+    if (n < 0 || n > INT32_MAX || ncomp < 0 || ncomp > n || !edges || !closed) return RBG_ERR_INVALID;
+    *closed = 1;
+    if (n == 0) return RBG_OK;
+    if (!label || !local || !start || !sorted_vertex || !comp_kind || !diag || !workspace || !row_off || !row_len ||
+        !top_msb || !first_msb || !comp_max || !edges->indptr ||
+        !edges->indices || !edges->data || !pool_cols || !pool_vals || edges->n_rows != n)
+        return RBG_ERR_INVALID;
+    CcWork W;
+    cc_work(reinterpret_cast<unsigned char *>(workspace), n, W);
+    if (workspace_bytes < (int64_t)W.bytes) return RBG_ERR_NOMEM;
+    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    *closed = 0;
+    if (n > (int64_t)1 << 27) return RBG_OK;
+    RBG_CUDA_TRY(cudaMemsetAsync(W.counters, 0, (size_t)((unsigned char *)W.state - (unsigned char *)W.counters), s));
+    RBG_CUDA_TRY(cudaMemsetAsync(top_msb, 0xff, (size_t)ncomp * 4, s));
+    RBG_CUDA_TRY(cudaMemsetAsync(first_msb, 0xff, (size_t)ncomp * 4, s));
+    RBG_CUDA_TRY(cudaMemsetAsync(comp_max, 0, (size_t)ncomp * 4, s));
+    note_launches(2);
+    cc_key_kernel<<<grid_for(n, 256), 256, 0, s>>>(n, label, local, start, sorted_vertex, comp_kind, edges->indptr,
+                                                  edges->indices, W.key, W.vertex, W.state, W.counters);
+    RBG_CUDA_TRY(cub::DeviceRadixSort::SortPairs(W.tmp, W.tmp_bytes, W.key, W.key_out, W.vertex, W.order, (int)n, 0, 13, s));
+    const TriCsrRows rows{tri_tickets(n, pool_capacity, TriTickets{}), W.order, label, comp_kind, sorted_vertex, start,
+                          edges->indptr, edges->indices, static_cast<const int32_t *>(edges->data), diag, comp_max};
+    tri_pull_kernel<<<tri_pull_grid(n), 32 * TRI_PULL_WARPS, 0, s>>>(rows, W.state, row_off, row_len, pool_cols, pool_vals,
+                                                                    pool_capacity, W.counters, W.ticket, top_msb,
+                                                                    first_msb, nullptr);
+    RBG_CUDA_TRY(cudaGetLastError());
+    DagCounters hd;
+    HostStaging hs(s, sizeof(hd) + 128);
+    int rc = hs.down(&hd, W.counters, sizeof(hd));
+    if (!rc) rc = hs.finish();
+    if (rc) return rc;
+    *closed = hd.flags == 0;
+    return RBG_OK;
+}
 
 // The DAG path keeps nothing between calls.
 extern "C" int32_t rbg_release_scratch(void) { return RBG_OK; }

@@ -504,20 +504,26 @@ __device__ __forceinline__ bool sp_small(const void *x, int64_t i, int &v) {
 // ----------------------------------------------------------------------------- tile rows
 // A squaring step over SP_TROWS consecutive rows whose entries, and whose entries' rows, lie in one
 // window of SP_TROWS columns (the families of a forest): the window's rows become a dense tile in
-// shared memory, each value split into (2^msb, rest), and a warp per row adds entry after entry,
-// every lane two columns in registers -- one 16-byte load, two multiply-adds and two mins per
-// entry instead of a walk over its row.  The same value rules as the group kernel's (SQUARE); a row
+// shared memory, each value split into (2^msb, rest).  A warp takes eight rows at once: their entries
+// become a dense 64 x 8 block, and for every column k that one of them holds the lanes read row k of the
+// tile once, two columns each, and add it to the rows that have an entry there -- two multiply-adds and
+// two mins per row and k, predicated.  The same value rules as the group kernel's (SQUARE); a row
 // that meets anything else goes to the warp kernel, a block whose window is wider to the group
 // kernel.
 //
-// Issue bound.  On family trees the tile is a third full, and still a row of 21 entries and 260
-// products takes about 500 instructions, against 850 in the group
-// kernel; the squaring of a 1,000,000-vertex forest takes 4.2 ms with it, 5.8 ms without.
+// Issue bound (65 to 70%; about 440 instructions per row of 15 entries, a third of the products in
+// rows without the entry).  A warp per row, every entry 512 bytes of the tile and two shuffles for
+// itself, was bound by shared memory: the five steps of a 1,000,000-vertex forest took 2.30 ms in this
+// kernel that way, 2.03 so (group kernel alone: 3.9).  Leaving out the empty halves of the tile's rows
+// saved instructions but no time.
 constexpr int SP_TROWS = 64;          // rows of a block and columns of a tile
 constexpr int SP_TWARPS = 8;
+constexpr int SP_TWROWS = SP_TROWS / SP_TWARPS;   // rows of a warp
 struct SpTile {
     uint2 cell[SP_TROWS][SP_TROWS];   // (2^msb, rest) of R(k, j); (0, all ones): none, or the diagonal's identity
-    int own[SP_TWARPS][SP_TROWS];     // a warp's row of R
+    int x[SP_TWARPS][SP_TROWS][SP_TWROWS];  // the entries of a warp's rows by column (the red one as 1)
+    unsigned red[SP_TWARPS][SP_TROWS];      // rows whose entry there is the red one
+    unsigned bad[SP_TWARPS];                // rows for the warp kernel
     int ptr[SP_TROWS + 1];            // first entry of each tile row, from the first one's
     int msb[SP_TROWS];                // largest MSB of a tile row
     int odd[SP_TROWS];                // 1: the row holds a value the tile cannot
@@ -584,61 +590,112 @@ sp_tile_kernel(SpArgs a) {
         }
     }
     __syncthreads();
-    unsigned ev = 0;
-    for (int r = w; r < SP_TROWS; r += SP_TWARPS) {
-        const int64_t i = r0 + r;
-        if (i >= a.n_rows) break;
-        const int64_t e0 = a.ap[i];
-        const int ne = (int)min((int64_t)INT_MAX, a.ap[i + 1] - e0);
-        *reinterpret_cast<int2 *>(&S.own[w][2 * lane]) = make_int2(0, 0);
-        __syncwarp();
-        unsigned s0 = ~0u, s1 = ~0u;
-        bool bad = ne > SP_TROWS;
-        for (int b = 0; b < ne && b < SP_TROWS; b += 32) {
-            int k = 0, x = 0;
-            if (b + lane < ne) {
-                k = a.aj[e0 + b + lane] - lo;
-                const bool in = sp_small<BYTES>(a.ax, e0 + b + lane, x) && x != 0 && (unsigned)k < (unsigned)SP_TROWS;
-                if (in) S.own[w][k] = x;
-                if (!in) k = 0;
-                if (x == -1) x = 1;                  // as a left operand (the splice then gives the right one)
-                bad |= !in || S.odd[k] != 0 || (31 - __clz(x | 1)) + S.msb[k] >= 31;
+    // the warp's rows into x: their entries are one run of the CSR arrays
+    const int64_t i0 = r0 + w * SP_TWROWS;
+    if (i0 >= a.n_rows) return;
+    const int nr = (int)min((int64_t)SP_TWROWS, a.n_rows - i0);
+    auto &X = S.x[w];
+    for (int q = lane; q < SP_TROWS * SP_TWROWS / 4; q += 32) reinterpret_cast<int4 *>(&X[0][0])[q] = make_int4(0, 0, 0, 0);
+    for (int q = lane; q < SP_TROWS; q += 32) S.red[w][q] = 0;
+    if (lane == 0) S.bad[w] = 0;
+    const int64_t e0 = a.ap[i0];
+    const int64_t far = a.ap[i0 + min(lane + 1, nr)] - e0;   // lane r: the end of row r
+    const int end = (int)min(far, (int64_t)INT_MAX);
+    const int ne = __shfl_sync(ALL, end, SP_TWROWS - 1);
+    __syncwarp();
+    for (int b = 0; b < min(ne, SP_TROWS * SP_TWROWS); b += 32) {
+        const int e = b + lane;
+        int r = 0;                                   // rows that end at or before e
+#pragma unroll
+        for (int q = 0; q < SP_TWROWS - 1; ++q) r += __shfl_sync(ALL, end, q) <= e;
+        if (e < ne) {
+            int x = 0;
+            const int k = a.aj[e0 + e] - lo;
+            bool bad = !sp_small<BYTES>(a.ax, e0 + e, x) || x == 0 || (unsigned)k >= (unsigned)SP_TROWS;
+            if (!bad) {
+                if (x == -1) {
+                    x = 1;                           // as a left operand (the splice then gives the right one)
+                    atomicOr(&S.red[w][k], 1u << r);
+                }
+                bad = S.odd[k] != 0 || (31 - __clz(x | 1)) + S.msb[k] >= 31;
+                bad |= atomicExch(&X[k][r], x) != 0; // a column twice
             }
-            const int m = min(32, ne - b);
-            for (int t = 0; t < m; ++t) {
-                const unsigned xt = (unsigned)__shfl_sync(ALL, x, t);
-                const uint4 c = *reinterpret_cast<const uint4 *>(&S.cell[__shfl_sync(ALL, k, t)][2 * lane]);
-                s0 = min(s0, xt * c.x + c.y);
-                s1 = min(s1, xt * c.z + c.w);
-            }
+            if (bad) atomicOr(&S.bad[w], 1u << r);
         }
-        __syncwarp();
-        if (__any_sync(ALL, bad)) {                  // warp-uniform
+    }
+    __syncwarp();
+    // columns 32 h + lane of the rows: R's own entries there, and which columns any row holds
+    int own[2][SP_TWROWS];
+    unsigned held[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        int any = 0;
+#pragma unroll
+        for (int q = 0; q < SP_TWROWS; q += 4) {
+            const int4 v = *reinterpret_cast<const int4 *>(&X[32 * h + lane][q]);
+            any |= v.x | v.y | v.z | v.w;
+        }
+        held[h] = __ballot_sync(ALL, any != 0);
+    }
+    unsigned sum[2][SP_TWROWS];
+#pragma unroll
+    for (int r = 0; r < SP_TWROWS; ++r) sum[0][r] = sum[1][r] = ~0u;
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+        for (unsigned left = held[h]; left; left &= left - 1) {
+            const int k = 32 * h + __ffs(left) - 1;
+            const uint2 c0 = S.cell[k][lane], c1 = S.cell[k][32 + lane];
+            unsigned x[SP_TWROWS];
+#pragma unroll
+            for (int q = 0; q < SP_TWROWS; q += 4) *reinterpret_cast<uint4 *>(&x[q]) = *reinterpret_cast<const uint4 *>(&X[k][q]);
+#pragma unroll
+            for (int r = 0; r < SP_TWROWS; ++r)
+                if (x[r]) {
+                    sum[0][r] = min(sum[0][r], x[r] * c0.x + c0.y);
+                    sum[1][r] = min(sum[1][r], x[r] * c1.x + c1.y);
+                }
+        }
+    unsigned red[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        red[h] = S.red[w][32 * h + lane];
+#pragma unroll
+        for (int q = 0; q < SP_TWROWS; q += 4) {
+            const int4 v = *reinterpret_cast<const int4 *>(&X[32 * h + lane][q]);
+            own[h][q] = v.x; own[h][q + 1] = v.y; own[h][q + 2] = v.z; own[h][q + 3] = v.w;
+        }
+    }
+    const unsigned badrows = ne > SP_TROWS * SP_TWROWS ? ALL : S.bad[w];
+    unsigned ev = 0;
+#pragma unroll
+    for (int r = 0; r < SP_TWROWS; ++r) {
+        if (r >= nr) break;
+        const int64_t i = i0 + r;
+        if ((badrows >> r) & 1u) {                   // warp-uniform
             if (lane == 0) a.warp_rows[atomicAdd(a.warp_count, 1)] = (int)i;
             continue;
         }
-        const int j0 = lo + 2 * lane;
-        if ((j0 == i && s0 != ~0u) || (j0 + 1 == i && s1 != ~0u)) ev |= RBG_EV_CYCLE;   // a vertex reaches itself
-        const int2 own = *reinterpret_cast<const int2 *>(&S.own[w][2 * lane]);
-        auto merged = [&](unsigned sum, int mine, int j) -> int {
-            const int sv = sum == ~0u || (a.upper && j < i) ? 0 : (int)sum;
-            return mine == 0 ? sv : sv == 0 ? mine : sp_minabs_small<UNS>(mine, sv);
-        };
-        const int v0 = merged(s0, own.x, j0), v1 = merged(s1, own.y, j0 + 1);
-        const unsigned b0 = __ballot_sync(ALL, v0 != 0), b1 = __ballot_sync(ALL, v1 != 0);
+        int v[2];
+        unsigned has[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int j = lo + 32 * h + lane;
+            if (j == i && sum[h][r] != ~0u) ev |= RBG_EV_CYCLE;   // a vertex reaches itself
+            const int mine = (red[h] >> r) & 1u ? -1 : own[h][r];
+            const int sv = sum[h][r] == ~0u || (a.upper && j < i) ? 0 : (int)sum[h][r];
+            v[h] = mine == 0 ? sv : sv == 0 ? mine : sp_minabs_small<UNS>(mine, sv);
+            has[h] = __ballot_sync(ALL, v[h] != 0);
+        }
         const unsigned before = (1u << lane) - 1u;
-        int64_t at = a.cand_off[i] + __popc(b0 & before) + __popc(b1 & before);
-        if (v0 != 0) {
-            a.ocol[at] = j0;
-            a.oval[at] = v0;
-            ++at;
-        }
-        if (v1 != 0) {
-            a.ocol[at] = j0 + 1;
-            a.oval[at] = v1;
-        }
-        if (lane == 0) a.rownnz[i] = __popc(b0) + __popc(b1);
-        __syncwarp();                                // before the next row clears its own entries
+        const int64_t at = a.cand_off[i];
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            if (v[h] != 0) {
+                const int64_t o = at + (h ? __popc(has[0]) : 0) + __popc(has[h] & before);
+                a.ocol[o] = lo + 32 * h + lane;
+                a.oval[o] = v[h];
+            }
+        if (lane == 0) a.rownnz[i] = __popc(has[0]) + __popc(has[1]);
     }
     ev = __reduce_or_sync(ALL, ev);
     if (lane == 0 && ev) atomicOr(a.flags, ev);

@@ -92,3 +92,17 @@ def test_squaring_step_reports_a_cycle(native):
             D = DeviceCSR.from_scipy(A.tocsr())
             assert spgemm(D, D, R=D, sem=sem)[2] & _lib.EV_CYCLE
             assert spgemm(D, D, sem=sem)[2] & _lib.EV_CYCLE
+
+
+@pytest.mark.parametrize("n, per_row", [(65, 3), (71, 64), (64, 400), (129, 400), (8, 30)])
+def test_tiles_of_full_and_few_rows(native, n, per_row):
+    """Rows that fill their tile below the diagonal (up to 63 entries, eight rows at a time), and last
+    blocks of fewer than eight rows."""
+    from redblackgraph_gb300.spgemm import DeviceCSR, spgemm
+    A = _random(n, 64, per_row, n, np.int64, "plain")
+    A.data[A.data > 3] = 3                                   # products of two small values: no overflow
+    S, fl = O.rb_matmul_csr(A, A)
+    D = DeviceCSR.from_scipy(A)
+    C, rc, _ = spgemm(D, D, R=D)
+    assert not fl & 7 and rc == 0
+    assert _cells(C.to_scipy()) == _merged(A, S, np.int64)

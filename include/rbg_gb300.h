@@ -71,11 +71,11 @@ typedef void *rbg_stream_t; /* a cudaStream_t */
 #define RBG_MODE_TRIANGULAR 2u  /* assume_upper_triangular loop (_shortest_path.pyx:365) */
 #define RBG_MODE_FORCE_EXACT 4u /* always run the sequential-order kernel                */
 #define RBG_MODE_FORCE_WIDE 8u  /* 64-bit storage: skip the 32-bit lane attempt          */
-#define RBG_MODE_GRAPH 16u      /* rbg_fw_batch, rbg_fw_dense: record the launch sequence as
-                                   a CUDA graph and replay it on later calls with the same
-                                   sizes, offsets, buffers and workspace (small LRU cache);
-                                   the DAG path's level loop is a while node the device ends,
-                                   so a call is one graph launch and one read of results   */
+#define RBG_MODE_GRAPH 16u      /* rbg_fw_batch, rbg_fw_dense: record the launch sequence of
+                                   the blocked kernels as a CUDA graph and replay it on later
+                                   calls with the same sizes, offsets, buffers and workspace
+                                   (small LRU cache); the DAG path is a few launches and
+                                   needs no graph                                          */
 #define RBG_MODE_TILE_NARROW 32u /* rbg_fw_batch: 128 x 64 phase-3 tiles in every round   */
 #define RBG_MODE_AUTOTUNE 64u   /* rbg_fw_batch: per-round tile shape chosen by timing both
                                    shapes on the first call for a batch layout (the first
@@ -87,8 +87,8 @@ typedef void *rbg_stream_t; /* a cudaStream_t */
 #define RBG_PATH_BLOCKED32 1
 #define RBG_PATH_BLOCKED64 2
 #define RBG_PATH_EXACT 3
-#define RBG_PATH_DAG 4   /* int32 / int64 acyclic matrix in the clean regime, closed by the
-                            DAG closure by levels                                          */
+#define RBG_PATH_DAG 4   /* int32 / int64 acyclic matrix in the clean regime, closed row by
+                            row, a row's parents first                                     */
 
 typedef struct rbg_result {
     int32_t status;   /* RBG_OK or RBG_ERR_*                                         */
@@ -116,8 +116,8 @@ int32_t rbg_profile_begin(void);
 int32_t rbg_profile_end(double *ms, int64_t *launches);
 
 /* rbg_profile_end for the first `slots` (1..9) timer slots: 0-3 as above, then the DAG path of
- * rbg_fw_batch / rbg_fw_dense: 4 scan, 5 closure by levels (with its CSR), 6 statistics, 7 write,
- * 8 the searches of matrices in any numbering. */
+ * rbg_fw_batch / rbg_fw_dense: 4 scan, 5 closure rows with their statistics, 6 nothing, 7 write, 8 the
+ * searches of matrices in any numbering. */
 int32_t rbg_profile_end_slots(double *ms, int64_t *launches, int32_t slots);
 
 /* Scratch bytes rbg_fw_dense needs for an n x n matrix of `dtype` under `mode`. */
@@ -182,7 +182,7 @@ int32_t rbg_fw_batch(int32_t dtype, int64_t count, const int64_t *sizes, const i
  * RBG_MODE_NO_DAG, RBG_MODE_TRIANGULAR, RBG_MODE_FORCE_EXACT or RBG_MODE_FORCE_WIDE is given): a
  * matrix in the clean regime (off-diagonal values 0 or in [2, 2^31), diagonal in {-1, 0, 1}),
  * with at most 16 off-diagonal entries per row and at most 8192 rows, whose graph is acyclic, is
- * closed through the DAG closure by levels.  With its vertices in a topological order (every
+ * closed row by row, a row's parents first.  With its vertices in a topological order (every
  * off-diagonal entry below, or every one above, the diagonal) the sequential loop's step k only
  * pushes row k into the rows of k's children (below) or pulls k's parents into the rows that
  * reach k (above), so the values are the DAG recurrence's and the diameter comes from each
@@ -190,14 +190,13 @@ int32_t rbg_fw_batch(int32_t dtype, int64_t count, const int64_t *sizes, const i
  * every vertex k, through the vertices below k, give the products of the loop's step k, hence the
  * same diameter and overflow decision.  A matrix whose loop computes a product
  * reaching bit 31 continues without the 32-bit lanes: on 64-bit lanes (int64) or on the exact
- * kernel (int32).  The path's scratch (row slots, the candidates' CSR, the closure's row pool,
- * the searches' cells) is carved from `workspace`; a closure that does not fit
+ * kernel (int32).  The path's scratch (row slots, orders, the closure's row pool, the searches' cells) is carved from `workspace`; a closure that does not fit
  * leaves its matrices to the blocked kernels.  Every accept / reject decision is made on the
  * device and the results are read back once per call.
  */
 
-/* Destroy the CUDA graphs RBG_MODE_GRAPH keeps for the DAG path (waits for the device first);
- * the next call in that mode records again.  No reference counterpart. */
+/* Frees what the DAG path keeps between calls, which is nothing (kept for callers that call it).  No
+ * reference counterpart. */
 int32_t rbg_release_scratch(void);
 
 /*
@@ -353,7 +352,7 @@ int32_t rbg_dag_workspace_bytes(int64_t n, int64_t nnz, int64_t *bytes);
  * stored entry or candidate (the reference's diameter source); RBG_ERR_CAPACITY when the pool
  * is too small (*nnz = a size to retry with) or a row has more than 8192 distinct columns
  * (*nnz = -1); RBG_ERR_CYCLE when the graph has a cycle.  *levels (host) = topological
- * levels.  Synchronises `stream` once per eight levels.
+ * levels.  Synchronises `stream` after the look for small pieces and once per eight levels.
  */
 int32_t rbg_dag_closure(const rbg_csr_t *A, void *workspace, int64_t workspace_bytes, int32_t *pool_cols,
                         int32_t *pool_vals, int64_t pool_capacity, int64_t *row_off, int32_t *row_len,

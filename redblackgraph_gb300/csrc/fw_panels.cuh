@@ -64,7 +64,10 @@ template <typename U> struct DiagSmem {
 // run in blocks of 8, fully unrolled, so the row of step t is the static register R[t % 8]
 // of the threads with h = t / 8.  One barrier per step: step t's writes go to slot t only.  A warp
 // (8 rows, 32 columns) skips the update of a step whose column is zero in its rows or whose row is
-// zero in its columns: in a matrix numbered in a topological order half of the tile is.  The running
+// zero in its columns: in a matrix numbered in a topological order half of the tile is.  A cell without
+// a path holds some word with the top bit set (an encoded zero times 2^s); published as a left operand
+// it would be multiplied again along a chain of steps until the top bit is gone, so column t is
+// published with its zeros as all ones, whose product keeps the top bit.  The running
 // maximum needs each newly valid cell's first valid product only, found from the masks at the end.
 // Bound by the chain of 64 steps: 18 us a round (n = 2048) with 4 threads per column,
 // every update run and every value tracked; 14 us with 8 threads per column.
@@ -106,7 +109,7 @@ fw_diag_kernel(U *__restrict__ work_base, unsigned long long *__restrict__ any_b
                     U v[PER];
 #pragma unroll
                     for (int k = 0; k < PER; ++k) {
-                        v[k] = R[r + k];
+                        v[k] = L::valid(R[r + k]) ? R[r + k] : L::inf;
                         cm = max(cm, (SU)v[k]);
                     }
                     *reinterpret_cast<uint4 *>(&S.CS[t][Pad<U>::at(h * DG_ROWS) + r]) = *reinterpret_cast<const uint4 *>(v);
@@ -142,8 +145,7 @@ fw_diag_kernel(U *__restrict__ work_base, unsigned long long *__restrict__ any_b
     // round buffer: snapshots, splits, masks and per-step maxima
     for (int e = tid; e < FW_B * FW_B; e += DG_THREADS) {
         const int t = e / FW_B, c = e % FW_B;
-        const U x = S.CS[t][Pad<U>::at(c)];
-        rb->cs[t][c] = L::valid(x) ? x : L::inf;
+        rb->cs[t][c] = S.CS[t][Pad<U>::at(c)];
         U m, low;
         L::split(S.Y[t][c], m, low);
         rb->rsm[t][c] = m;
@@ -178,6 +180,10 @@ fw_diag_kernel(U *__restrict__ work_base, unsigned long long *__restrict__ any_b
         const int a = h * DG_ROWS + r;
         if (!L::valid(R[r]) || !((startInf >> r) & 1u)) continue;
         const int tf = __ffsll((long long)(S.maskC[a] & S.maskR[b])) - 1;
+        if (tf < 0) {                                 // a value no step gave: inconsistent
+            risk = true;
+            continue;
+        }
         U m, low;
         L::split(S.Y[tf][b], m, low);
         smx = max(smx, (SU)(S.CS[tf][Pad<U>::at(h * DG_ROWS) + r] * m + low));

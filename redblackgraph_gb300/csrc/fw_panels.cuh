@@ -361,8 +361,11 @@ __device__ __forceinline__ void panel_item(PanelSmem<U, LINES> &S, int ci, int l
 #pragma unroll
             for (int l = 0; l < PN_CELLS; ++l) {
                 const int t = T * PN_CELLS + l;
-                const U z = shfl_lane<U>(R[l], grp | T);  // P(t, j) or P(i, t): invariant at step t
+                U z = shfl_lane<U>(R[l], grp | T);    // P(t, j) or P(i, t): invariant at step t
                 const bool zv = L::valid(z);
+                // a zero as all ones: as a left operand its products keep the top bit only so
+                // (phase 1, above)
+                if (!zv) z = L::inf;
                 seenT |= (unsigned)zv << l;
                 if (h == 0) S.Z[t][line] = z;
                 // a zero step operand makes every product of the step a zero: skip the step when
@@ -429,6 +432,10 @@ __device__ __forceinline__ void panel_item(PanelSmem<U, LINES> &S, int ci, int l
         if (vv && ((startInf >> r) & 1u)) {
             const unsigned long long both = seen & (rowPanel ? S.maskCS[c] : S.maskRS[c]);
             const int tf = __ffsll((long long)both) - 1;
+            if (tf < 0) {                             // a value no step gave: inconsistent
+                risk = true;
+                continue;
+            }
             U first;
             const U zf = S.Z[tf][line];
             if (rowPanel) {

@@ -93,3 +93,12 @@ def test_diagonal_block(native, dtype):
     mats += [N for n in (35, 50, 63) for N in numberings(dense_dag(n, n), n)]
     check_batch(mats, dtype, 0)
     check_dense(mats[:30], dtype, _lib.MODE_NO_DAG)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_panels(native, dtype):
+    """Several blocks: rows outside a block whose few entries meet the chains inside it."""
+    from redblackgraph_gb300 import _lib
+    mats = [N for n in (65, 128, 129, 200, 300) for s in range(4) for N in numberings(dense_dag(n, 100 * s + n), n)]
+    check_batch(mats, dtype, 0)                          # panels of 64 lines
+    check_dense(mats, dtype, _lib.MODE_NO_DAG)           # of 32 lines

@@ -54,8 +54,9 @@ template <typename T> __device__ __forceinline__ uint32_t sd_lane(T v, bool off_
 
 // D(I): the diagonal blocks of the lane matrix closed in place, one CTA per block.  Its two 64 x 64
 // halves on the diagonal are closed first, 256 threads each (4 x 4 cells per thread in registers; step
-// t's row and column are published before one barrier); then the remaining quarter X is multiplied by
-// the halves on both sides, X <- X (+) X (x) P, then X <- X (+) Q (x) X.
+// t's row and column are published before one barrier, the column with its zeros as all ones, whose
+// products keep the top bit: a zero multiplied along a chain of steps would lose it); then the remaining
+// quarter X is multiplied by the halves on both sides, X <- X (+) X (x) P, then X <- X (+) Q (x) X.
 __global__ void __launch_bounds__(SD_THREADS)
 sd_diag_kernel(uint32_t *__restrict__ work, int64_t np, int above, DevStatus *st) {
     constexpr int H = SD_B / 2;
@@ -93,8 +94,9 @@ sd_diag_kernel(uint32_t *__restrict__ work, int64_t np, int above, DevStatus *st
                 int top = -1;
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
-                    s_col[half][b][4 * ty + r] = R[r][u];
-                    if (sd_valid(R[r][u])) top = max(top, 31 - __clz((int)R[r][u]));
+                    const bool on = sd_valid(R[r][u]);
+                    s_col[half][b][4 * ty + r] = on ? R[r][u] : SD_NONE;
+                    if (on) top = max(top, 31 - __clz((int)R[r][u]));
                 }
                 if (top >= 0) atomicMax(&s_cmax[half][t], top);
             }

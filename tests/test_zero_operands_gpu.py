@@ -102,3 +102,17 @@ def test_panels(native, dtype):
     mats = [N for n in (65, 128, 129, 200, 300) for s in range(4) for N in numberings(dense_dag(n, 100 * s + n), n)]
     check_batch(mats, dtype, 0)                          # panels of 64 lines
     check_dense(mats, dtype, _lib.MODE_NO_DAG)           # of 32 lines
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_block_steps(native, dtype):
+    """Through the entry points' own choice of a path: block steps where the entries lie on one side."""
+    from redblackgraph_gb300 import _lib
+    from redblackgraph_gb300.dense import fw_dense
+    from redblackgraph_gb300.device import to_device
+    mats = [N for k, A in enumerate(small_matrices() + tuple(dense_dag(64, s) for s in range(20)))
+            for N in numberings(A, k)]
+    mats += [N for n in (65, 128, 129, 200, 300) for s in range(4) for N in numberings(dense_dag(n, 100 * s + n), n)]
+    check_dense(mats, dtype, 0)
+    for A in small_matrices():                           # (none is left to another path for its zeros)
+        assert fw_dense(to_device(A.astype(dtype)))[1].path == _lib.PATH_BLOCKED32

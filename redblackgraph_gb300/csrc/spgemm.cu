@@ -585,7 +585,9 @@ sp_tile_kernel(SpArgs a) {
             S.odd[k] = 1;
         } else if (y >= 2) {
             const int s = 31 - __clz(y);
-            S.cell[k][c] = make_uint2(1u << s, (unsigned)y ^ (1u << s));
+            // a cell holds one value: a row with a column twice is not for the tile
+            const unsigned long long both = (unsigned long long)((unsigned)y ^ (1u << s)) << 32 | 1u << s;
+            if ((unsigned)atomicExch(reinterpret_cast<unsigned long long *>(&S.cell[k][c]), both)) S.odd[k] = 1;
             if (s > S.msb[k]) atomicMax(&S.msb[k], s);
         }
     }
@@ -665,14 +667,17 @@ sp_tile_kernel(SpArgs a) {
             own[h][q] = v.x; own[h][q + 1] = v.y; own[h][q + 2] = v.z; own[h][q + 3] = v.w;
         }
     }
-    const unsigned badrows = ne > SP_TROWS * SP_TWROWS ? ALL : S.bad[w];
+    // (a row of columns many times over is the dense kernel's)
+    const unsigned dense = __ballot_sync(ALL, lane < nr && a.cand_off[i0 + min(lane, nr - 1) + 1] -
+                                                               a.cand_off[i0 + min(lane, nr - 1)] > SP_BLOCK_CAP);
+    const unsigned badrows = ne > SP_TROWS * SP_TWROWS ? ALL : S.bad[w] | dense;
     unsigned ev = 0;
 #pragma unroll
     for (int r = 0; r < SP_TWROWS; ++r) {
         if (r >= nr) break;
         const int64_t i = i0 + r;
         if ((badrows >> r) & 1u) {                   // warp-uniform
-            if (lane == 0) a.warp_rows[atomicAdd(a.warp_count, 1)] = (int)i;
+            if (lane == 0 && !((dense >> r) & 1u)) a.warp_rows[atomicAdd(a.warp_count, 1)] = (int)i;
             continue;
         }
         int v[2];

@@ -682,14 +682,20 @@ sp_tile_kernel(SpArgs a) {
         }
         int v[2];
         unsigned has[2];
+        bool lost = false;                           // the identity left out would have kept the red one
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int j = lo + 32 * h + lane;
             if (j == i && sum[h][r] != ~0u) ev |= RBG_EV_CYCLE;   // a vertex reaches itself
             const int mine = (red[h] >> r) & 1u ? -1 : own[h][r];
             const int sv = sum[h][r] == ~0u || (a.upper && j < i) ? 0 : (int)sum[h][r];
+            lost |= UNS && mine == -1 && sv != 0;
             v[h] = mine == 0 ? sv : sv == 0 ? mine : sp_minabs_small<UNS>(mine, sv);
             has[h] = __ballot_sync(ALL, v[h] != 0);
+        }
+        if (UNS && __any_sync(ALL, lost)) {
+            if (lane == 0) a.warp_rows[atomicAdd(a.warp_count, 1)] = (int)i;
+            continue;
         }
         const unsigned before = (1u << lane) - 1u;
         const int64_t at = a.cand_off[i];
@@ -708,7 +714,9 @@ sp_tile_kernel(SpArgs a) {
 
 // SQUARE: a squaring step of one matrix (A = B = R).  Identities on the diagonal are left out as
 // right operands there: R(i, k) (x) R(k, k) is R's own entry (or zero), which the magnitude merge
-// keeps anyway; what meets at (i, i) then are plain products only, each of them a cycle.
+// keeps anyway; what meets at (i, i) then are plain products only, each of them a cycle.  Except for
+// the red one of unsigned values: the sum with it is the red one, but its magnitude is the largest, so
+// the merge would take another product of its column.  A row where the two meet goes to the warp kernel.
 template <bool UNS, int BYTES, bool SQUARE>
 __global__ void __launch_bounds__(SP_GWARPS * 32)
 sp_group_kernel(SpArgs a, int merge) {
@@ -826,6 +834,8 @@ sp_group_kernel(SpArgs a, int merge) {
         }
         if (SQUARE) bad |= low < -1 || top >= 31 || (far >= (unsigned)span && ne > 0);
         __syncwarp();
+        if (SQUARE && UNS)                           // the identity left out would have kept the red one
+            for (int q = gl; q < span; q += SP_GL) bad |= W.own[q] == -1 && W.sum[q] != ~0u;
         bad = (__ballot_sync(ALL, bad) & gmask) != 0;
         if (SQUARE && !bad && gl == 0 && (unsigned long long)(i - jlo) < (unsigned long long)span &&
             W.sum[i - jlo] != ~0u)

@@ -1,6 +1,10 @@
-"""Squaring steps where the tiles' and groups' shortcuts must not show: columns stored twice."""
+"""Squaring steps where the tiles' and groups' shortcuts must not show: columns stored twice, and
+identities that meet other products."""
 import numpy as np
 import pytest
+import scipy.sparse as sp
+
+from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
 
@@ -51,3 +55,41 @@ def test_rows_of_many_candidates_in_one_block(native, dtype):
     A, B = _csr(rows, n, dtype), _csr(once, n, dtype)
     got, want = spgemm(A, A, R=A), spgemm(B, B, R=B)
     assert got[1:] == want[1:] and (got[0].to_scipy().toarray() == want[0].to_scipy().toarray()).all()
+
+
+def _cells(m):
+    m = m.tocoo()
+    return {(r, c): v for r, c, v in zip(m.row.tolist(), m.col.tolist(), m.data.tolist()) if v != 0}
+
+
+def _merged(R, S):
+    """R (+) R^2 by magnitude (R's value on a tie), as int32."""
+    mag = (lambda v: v) if R.dtype.kind == "u" else abs
+    r, s = _cells(R), _cells(S)
+    out = {k: s[k] if k not in r or (k in s and mag(s[k]) < mag(r[k])) else r[k] for k in {**r, **s}}
+    return {k: w for k, w in ((k, int(np.array(v, R.dtype).astype(np.int32))) for k, v in out.items()) if w != 0}
+
+
+@pytest.mark.parametrize("dtype", [np.int32, np.int64, np.uint32, np.uint64])
+@pytest.mark.parametrize("n, family", [(1, 1), (64, 64), (300, 64), (320, 100), (400, 200), (90, 3)])
+def test_identities_that_meet_products(native, dtype, n, family):
+    """Families with entries on both sides of the diagonal (cycles, so that plain products reach the
+    diagonal's identities) and a few identities off it, at columns whose diagonal is the same identity."""
+    from redblackgraph_gb300.spgemm import DeviceCSR, spgemm
+    red = np.array(-1, np.int64).astype(dtype)
+    for seed in range(6):
+        rng = np.random.default_rng([n, family, seed])
+        A = np.zeros((n, n), dtype)
+        r = np.repeat(np.arange(n), 3)
+        f = r // family * family
+        c = f + (rng.random(r.size) * (np.minimum(f + family, n) - f)).astype(int)
+        A[r, c] = rng.integers(2, 9, r.size)
+        k = rng.choice(r.size, max(1, r.size // 10))
+        A[r[k], c[k]] = red if seed % 2 else 1
+        A[np.arange(n), np.arange(n)] = np.where(rng.random(n) < 0.7, red, np.array(seed % 3 != 0, dtype))
+        M = sp.csr_matrix(A)
+        S, fl = O.rb_matmul_csr(M, M)
+        assert not fl & 7
+        D = DeviceCSR.from_scipy(M)
+        C, rc, _ = spgemm(D, D, R=D)
+        assert rc == 0 and _cells(C.to_scipy()) == _merged(M, S), (n, family, seed)

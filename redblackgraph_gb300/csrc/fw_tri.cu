@@ -345,8 +345,11 @@ __device__ __forceinline__ int64_t tri_find_col(const int32_t *__restrict__ p_co
     return -1;
 }
 
-// One warp per candidate row of a general matrix: the cells of A's entries start with key 0 (their
-// first value is A's), the other cells empty.  Cell q of the row is cell[row_off + q].
+// One warp per candidate row of a general matrix: the cells of A's entries start with key 0, the other
+// cells empty.  The loop looks at a value only after it has folded the step's product in, so the first
+// value of such a cell is A's, or the product of step 0 where that is less (A(i, 0) (x) A(0, j); only
+// numberings in which vertex 0 has parents and children hold one).  Cell q of the row is
+// cell[row_off + q].
 __global__ void tri_gen_init_kernel(int64_t R, const int32_t *__restrict__ row_comp, const int32_t *__restrict__ ckind,
                                     const TriComp *__restrict__ comps, TriGraphView G,
                                     const int64_t *__restrict__ row_off,
@@ -364,12 +367,19 @@ __global__ void tri_gen_init_kernel(int64_t R, const int32_t *__restrict__ row_c
         for (int q = lane; q < len; q += 32) cell[o + q] = TRI_EMPTY;
         __syncwarp();
         const int64_t base = comps[ci].row_base;
-        int cnt;
-        const int64_t e0 = G.row(g, cnt);
+        int cnt, cnt0;
+        const int64_t e0 = G.row(g, cnt), z0 = G.row(base, cnt0);
+        const uint32_t x = g != base && cnt > 0 && G.col[e0] == 0 ? (uint32_t)G.val[e0] : 0u;   // A(i, 0)
         for (int64_t e = e0 + lane; e < e0 + cnt; e += 32) {
-            const int64_t q = tri_find_col(p_col, o, len, (int32_t)(base + G.col[e]));
+            const int32_t c = G.col[e];
+            uint32_t v = (uint32_t)G.val[e];             // a clean value: 2 <= v < 2^31
+            for (int64_t z = z0; x != 0 && z < z0 + cnt0; ++z) {
+                const uint32_t y = (uint32_t)G.val[z];
+                if (G.col[z] == c) v = (uint32_t)min((uint64_t)v, ((uint64_t)(x - 1) << msb_u32(y)) + y);
+            }
+            const int64_t q = tri_find_col(p_col, o, len, (int32_t)(base + c));
             if (q < 0) atomicOr(gflags, 2u);
-            else cell[q] = (uint32_t)msb_u32((uint32_t)G.val[e]);   // a clean value: 2 <= v < 2^31
+            else cell[q] = (uint32_t)msb_u32(v);
         }
     }
 }

@@ -815,7 +815,10 @@ tri_pull_kernel(Rows A, unsigned long long *state, int64_t *__restrict__ row_off
                 blk_left = max(bound, tk.block);
                 blk_at = atomicAdd(&dc->reserved, (unsigned long long)blk_left);
             }
-            // candidate idx of the flattened rows: its column and product (0 beyond the end)
+            // candidate idx of the flattened rows: its column and product.  0 beyond the end, and for a product
+            // past 31 bits, which would wrap: it is never a cell's minimum, as a matrix with such a minimum
+            // leaves the path (in any numbering the recurrence forms products that the loop, which has a
+            // shorter path by then, does not)
             auto candidate = [&](int idx, int &col, int &pm) -> int {
                 int lo = 0;
 #pragma unroll
@@ -831,7 +834,7 @@ tri_pull_kernel(Rows A, unsigned long long *state, int64_t *__restrict__ row_off
                 col = __ldcg(p_col + oq + (idx - xq)) - base;
                 const int y = __ldcg(p_val + oq + (idx - xq));
                 pm = dag_row_msb(vq) + dag_row_msb(y);
-                return cy_product(vq, y);
+                return pm >= TRI_TOP ? 0 : cy_product(vq, y);
             };
             int nd = 0;                          // the row's entries
             unsigned long long at = 0;

@@ -812,7 +812,7 @@ __global__ void __launch_bounds__(DG_BTHREADS) dag_fill_block_kernel(DagArgs a, 
 constexpr int DT_ROWS = 64;
 constexpr int DT_WARPS = 4;             // warps (tiles) per CTA
 constexpr int DT_ENTRIES = 384;         // stored entries a tile may hold
-constexpr int DT_NONE = 0x7fffffff;
+constexpr unsigned DT_NONE = ~0u;         // no value yet: above every int32 value, the largest included
 struct DagTile {
     int cell[DT_ROWS * (DT_ROWS - 1) / 2];   // row l, column c < l: cell[l (l - 1) / 2 + c]; 0: none
     int val[DT_ENTRIES];
@@ -869,7 +869,8 @@ __device__ __forceinline__ bool dag_tile(const DagArgs &a, DagTile &S, int64_t p
     for (int l = 0; l < len; ++l) {
         const int r = flip ? len - 1 - l : l;
         const int q1 = S.ptr[r + 1];
-        int x0 = DT_NONE, x1 = DT_NONE, dg = 0, lev = 0;
+        unsigned x0 = DT_NONE, x1 = DT_NONE;
+        int dg = 0, lev = 0;
         for (int q = S.ptr[r]; q < q1; ++q) {                // warp-uniform
             const int v = S.val[q], c = flip ? len - 1 - S.col[q] : S.col[q];
             most = max(most, v < 0 ? 1 : v);
@@ -878,27 +879,27 @@ __device__ __forceinline__ bool dag_tile(const DagArgs &a, DagTile &S, int64_t p
                 continue;
             }
             lev = max(lev, S.level[c] + 1);
-            if (lane == c) x0 = min(x0, v);
-            if (lane + 32 == c) x1 = min(x1, v);
+            if (lane == c) x0 = min(x0, (unsigned)v);
+            if (lane + 32 == c) x1 = min(x1, (unsigned)v);
             const int base = c * (c - 1) / 2, mv = 31 - __clz(v);
             const int y0 = lane < c ? S.cell[base + lane] : 0, y1 = lane + 32 < c ? S.cell[base + lane + 32] : 0;
             if (y0 != 0) {
                 const int s = 31 - __clz(y0), pr = (v << s) | (y0 ^ (1 << s));
                 top = max(top, mv + s);
-                x0 = min(x0, pr);
+                x0 = min(x0, (unsigned)pr);
                 most = max(most, pr);
             }
             if (y1 != 0) {
                 const int s = 31 - __clz(y1), pr = (v << s) | (y1 ^ (1 << s));
                 top = max(top, mv + s);
-                x1 = min(x1, pr);
+                x1 = min(x1, (unsigned)pr);
                 most = max(most, pr);
             }
         }
         const int base = l * (l - 1) / 2;
         const bool h0 = x0 != DT_NONE, h1 = x1 != DT_NONE;
-        if (lane < l) S.cell[base + lane] = h0 ? x0 : 0;
-        if (lane + 32 < l) S.cell[base + lane + 32] = h1 ? x1 : 0;
+        if (lane < l) S.cell[base + lane] = h0 ? (int)x0 : 0;
+        if (lane + 32 < l) S.cell[base + lane + 32] = h1 ? (int)x1 : 0;
         const int m = __popc(__ballot_sync(FULL, h0)) + __popc(__ballot_sync(FULL, h1)) + (dg != 0);
         total += m;
         if (lane == 0) {

@@ -1,0 +1,45 @@
+"""The DAG closure's tiles at the ends of their value range, against the oracle."""
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+TOP = 2 ** 31 - 1
+
+
+def _families(family, count, side, seed):
+    """Families whose entries include 2^31 - 1, and pairs whose product is 2^31 - 1."""
+    rng = np.random.default_rng([family, seed])
+    M = np.zeros((family * count, family * count), np.int64)
+    for f in range(0, family * count, family):
+        for i in range(1, family):
+            to = f + rng.choice(i, min(i, 2), replace=False)
+            M[f + i, to] = rng.integers(2, 4, to.size)
+        leaf = f + family - 1
+        M[leaf] = 0
+        M[leaf, f] = TOP                                         # an edge to a vertex without parents
+        if family > 5:
+            a, b = 1 + rng.integers(0, 14), f + family - 3       # 2^a - 1 and 2^(32 - a) - 1, splices to the top
+            M[b - 2] = M[b - 1] = M[b] = 0
+            M[b, b - 1], M[b - 1, b - 2] = 2 ** (a + 1) - 1, 2 ** (31 - a) - 1
+    np.fill_diagonal(M, rng.choice([-1, 0, 1], M.shape[0]))
+    return sp.csr_matrix((M if side < 0 else M[::-1, ::-1].copy()).astype(np.int32))
+
+
+@pytest.mark.parametrize("side", [-1, 1])
+def test_largest_value(native, side):
+    from redblackgraph_gb300.dag import dag_closure_device
+    from redblackgraph_gb300.spgemm import DeviceCSR
+    for family, count in ((2, 3), (5, 20), (20, 9), (63, 2), (64, 5), (65, 2)):
+        A = _families(family, count, side, count)
+        W = sp.csr_matrix(O.dag_closure(A)[0])
+        W.sort_indices()
+        assert (W.data == TOP).sum() >= count
+        for tiles in (True, False):
+            C, mx, _ = dag_closure_device(DeviceCSR.from_scipy(A), tiles=tiles)
+            got = C.to_scipy()
+            assert mx == TOP and (got.indptr == W.indptr).all()
+            assert (got.indices == W.indices).all() and (got.data == W.data).all(), (family, tiles)

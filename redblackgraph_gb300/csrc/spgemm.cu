@@ -547,8 +547,9 @@ sp_tile_kernel(SpArgs a) {
             const int64_t e0 = a.ap[i], e1 = a.ap[i + 1];
             if (e1 > e0) {                           // (the row's own columns are candidates as well)
                 const int2 wnd = a.win[i];
-                lo = wnd.x;
-                hi = wnd.y;
+                // first column past the last one: the columns do not ascend, and the window is unknown
+                lo = wnd.y < wnd.x ? 0 : wnd.x;
+                hi = wnd.y < wnd.x ? INT_MAX : wnd.y;
             }
         }
         lo = __reduce_min_sync(ALL, lo);

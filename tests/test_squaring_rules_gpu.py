@@ -1,5 +1,5 @@
-"""Squaring steps where the tiles' and groups' shortcuts must not show: columns stored twice, and
-identities that meet other products."""
+"""Squaring steps where the tiles' and groups' shortcuts must not show: columns stored twice,
+identities that meet other products, and columns that do not ascend."""
 import numpy as np
 import pytest
 import scipy.sparse as sp
@@ -93,3 +93,24 @@ def test_identities_that_meet_products(native, dtype, n, family):
         D = DeviceCSR.from_scipy(M)
         C, rc, _ = spgemm(D, D, R=D)
         assert rc == 0 and _cells(C.to_scipy()) == _merged(M, S), (n, family, seed)
+
+
+@pytest.mark.parametrize("dtype", [np.int32, np.int64, np.uint32, np.uint64])
+@pytest.mark.parametrize("n, family", [(2, 2), (64, 64), (65, 64), (300, 50), (256, 100)])
+def test_columns_in_any_order(native, dtype, n, family):
+    """Every row's columns descending, shuffled, or ascending in most rows: the same matrix."""
+    from redblackgraph_gb300.spgemm import spgemm
+    rng = np.random.default_rng([n, family])
+    rows = []
+    for i in range(n):
+        f = i // family * family
+        to = rng.choice(np.arange(f, min(f + family, n)), min(3, min(f + family, n) - f), replace=False)
+        rows.append(sorted({int(c): int(rng.integers(2, 9)) for c in to if c != i}.items() | {(i, 1)}))
+    B = _csr(rows, n, dtype)
+    want = spgemm(B, B, R=B)
+    shuffled = [[r[k] for k in rng.permutation(len(r))] for r in rows]
+    few = [r[::-1] if i % 17 == 1 else r for i, r in enumerate(rows)]
+    for other in ([r[::-1] for r in rows], shuffled, few):
+        A = _csr(other, n, dtype)
+        got = spgemm(A, A, R=A)
+        assert got[1:] == want[1:] and _cells(got[0].to_scipy()) == _cells(want[0].to_scipy())

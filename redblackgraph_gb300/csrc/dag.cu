@@ -870,12 +870,12 @@ __device__ __forceinline__ bool dag_tile(const DagArgs &a, DagTile &S, int64_t p
         const int r = flip ? len - 1 - l : l;
         const int q1 = S.ptr[r + 1];
         unsigned x0 = DT_NONE, x1 = DT_NONE;
-        int dg = 0, lev = 0;
+        int dg = 2, lev = 0;                                 // dg: 2 while there is no diagonal entry
         for (int q = S.ptr[r]; q < q1; ++q) {                // warp-uniform
             const int v = S.val[q], c = flip ? len - 1 - S.col[q] : S.col[q];
             most = max(most, v < 0 ? 1 : v);
             if (c == l) {
-                dg = v;
+                dg = min(dg, v);                             // (stored twice: the (+) of the two)
                 continue;
             }
             lev = max(lev, S.level[c] + 1);
@@ -898,6 +898,7 @@ __device__ __forceinline__ bool dag_tile(const DagArgs &a, DagTile &S, int64_t p
         }
         const int base = l * (l - 1) / 2;
         const bool h0 = x0 != DT_NONE, h1 = x1 != DT_NONE;
+        dg = dg == 2 ? 0 : dg;
         if (lane < l) S.cell[base + lane] = h0 ? (int)x0 : 0;
         if (lane + 32 < l) S.cell[base + lane + 32] = h1 ? (int)x1 : 0;
         const int m = __popc(__ballot_sync(FULL, h0)) + __popc(__ballot_sync(FULL, h1)) + (dg != 0);

@@ -1,4 +1,5 @@
-"""The DAG closure's tiles at the ends of their value range, against the oracle."""
+"""The DAG closure's tiles at the ends of their value range, against the oracle, and with diagonal entries
+stored twice, against the levels."""
 import numpy as np
 import pytest
 import scipy.sparse as sp
@@ -43,3 +44,20 @@ def test_largest_value(native, side):
             got = C.to_scipy()
             assert mx == TOP and (got.indptr == W.indptr).all()
             assert (got.indices == W.indices).all() and (got.data == W.data).all(), (family, tiles)
+
+
+def test_diagonal_stored_twice(native):
+    import torch
+    from redblackgraph_gb300.dag import dag_closure_device
+    from redblackgraph_gb300.device import to_host
+    from redblackgraph_gb300.spgemm import DeviceCSR
+    twice = [(1, -1), (-1, 1), (1, 1), (-1, -1), (1,), (-1,), ()]
+    rows = [[(i - 1, 2)] * (i % 7 > 0) + [(i, v) for v in twice[i % 7]] for i in range(64)]
+    ptr = torch.tensor(np.cumsum([0] + [len(r) for r in rows]), device="cuda")
+    col = torch.tensor([c for r in rows for c, _ in r], dtype=torch.int32, device="cuda")
+    val = torch.tensor([v for r in rows for _, v in r], dtype=torch.int32, device="cuda")
+    got, want = (dag_closure_device(DeviceCSR(ptr, col, val, (64, 64)), tiles=t) for t in (True, False))
+    assert got[1:] == want[1:]
+    for a, b in ((got[0].indptr, want[0].indptr), (got[0].indices, want[0].indices), (got[0].data, want[0].data)):
+        assert (to_host(a) == to_host(b)).all()
+    assert want[0].to_scipy().diagonal().tolist() == [min(twice[i % 7], default=0) for i in range(64)]

@@ -62,8 +62,6 @@ __device__ __forceinline__ void mm_flush_flags(unsigned *dflags, unsigned f) {
 // column of a thread's output c within the tile
 __device__ __forceinline__ int mm_col(int tx, int c) { return (c < 4 ? 0 : 60) + 4 * tx + c; }
 
-constexpr size_t align_up_c(size_t x) { return (x + 15) / 16 * 16; }
-
 // the sum as a minimum: the red one first, "no path" last
 template <typename U> __device__ __forceinline__ U mm_enc(U v) { return v == 0 ? (U)~(U)0 : v == (U)~(U)0 ? (U)0 : v; }
 
@@ -83,50 +81,117 @@ __device__ __forceinline__ void mm_load4(const T *__restrict__ row, bool live, i
     }
 }
 
-// Full scalar semantics for one tile, steps [j0, j1): the outputs of each thread (as in mm_kernel)
-// into `tile`, in the encoding of mm_enc.  Every thread of the CTA calls it; `tile` may overlap
-// the staging buffers.
+// Full scalar semantics for one tile, steps [j0, j1): its outputs into `tile`, in the encoding of
+// mm_enc.  Every thread of the CTA calls it.  The quarters of the tile come one after another (a quarter
+// beyond the matrix not at all), 2 x 4 outputs per thread, so that small products spread over the CTA.
+// Only steps with a negative value in the quarter take every case; the others ask for zeros and
+// identities, and for the top bit where a thread's operands may reach it.  Bound by issue, 64-bit shifts and mins.  int64 operands
+// with a third of their entries up to 2^40, 64 x 64 x 64: 328 us with every case on 32 outputs per thread,
+// 115 so (193 us one 64 x 64 tile per CTA); 1500 x 1500 x 1500: 12.3, 6.3 (9.9) ms.
+constexpr int MM_Q = MM_T / 2;               // quarter edge
+template <typename T> struct MmExact {
+    T as[MM_Q][MM_K + 1];
+    T bs[MM_K][MM_Q + 4];
+    unsigned negative;                       // steps of the chunk with a negative value other than -1
+};
 template <typename T>
 __device__ __noinline__ void mm_exact_tile(int64_t m, int64_t p, int64_t i0, int64_t k0, int64_t j0, int64_t j1,
                                            const T *__restrict__ A, int64_t lda, const T *__restrict__ B, int64_t ldb,
-                                           unsigned char *smem, unsigned *dflags) {
+                                           typename utype<T>::type *tile, MmExact<T> &S, unsigned *dflags) {
     typedef typename utype<T>::type U;
-    T(*as)[MM_K + 1] = reinterpret_cast<T(*)[MM_K + 1]>(smem);
-    T(*bs)[MM_T + 1] = reinterpret_cast<T(*)[MM_T + 1]>(smem + align_up_c(sizeof(T) * MM_T * (MM_K + 1)));
+    constexpr int BITS = (int)sizeof(U) * 8;
+    constexpr U NONE = (U)~(U)0, RED = (U)~(U)0;   // mm_enc of no path; the red one itself
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     unsigned ev = 0;
-    T acc[4][8];
+    __syncthreads();                         // the last chunk's reads of the staging buffers
+    for (int q = 0; q < 4; ++q) {
+        const int64_t iq = i0 + MM_Q * (q >> 1), kq = k0 + MM_Q * (q & 1);
+        if (iq >= m || kq >= p) continue;    // block-uniform
+        U acc[2][4];
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+        for (int r = 0; r < 2; ++r)
 #pragma unroll
-        for (int c = 0; c < 8; ++c) acc[r][c] = 0;
-    for (int64_t j = j0; j < j1; j += MM_K) {
-        __syncthreads();
-        for (int e = tid; e < MM_T * MM_K; e += MM_THREADS) {
-            const int r = e / MM_K, c = e % MM_K, rr = e / MM_T, cc = e % MM_T;
-            as[r][c] = (i0 + r < m && j + c < j1) ? A[(i0 + r) * lda + j + c] : (T)0;
-            bs[rr][cc] = (j + rr < j1 && k0 + cc < p) ? B[(j + rr) * ldb + k0 + cc] : (T)0;
+            for (int c = 0; c < 4; ++c) acc[r][c] = NONE;
+        const bool mine = iq + 2 * ty < m && kq + 4 * tx < p;
+        for (int64_t j = j0; j < j1; j += MM_K) {
+            __syncthreads();
+            if (tid == 0) S.negative = 0;
+            __syncthreads();
+            unsigned neg = 0;
+            auto negative_value = [](T v) { return utype<T>::is_signed && v < 0 && v != (T)-1; };
+            for (int e = tid; e < MM_Q * MM_K; e += MM_THREADS) {
+                const int r = e / MM_K, c = e % MM_K, rr = e / MM_Q, cc = e % MM_Q;
+                const T a = (iq + r < m && j + c < j1) ? A[(iq + r) * lda + j + c] : (T)0;
+                const T b = (j + rr < j1 && kq + cc < p) ? B[(j + rr) * ldb + kq + cc] : (T)0;
+                S.as[r][c] = a;
+                S.bs[rr][cc] = b;
+                neg |= (negative_value(a) ? 1u << c : 0u) | (negative_value(b) ? 1u << rr : 0u);
+            }
+            neg = __reduce_or_sync(0xffffffffu, neg);
+            if ((tid & 31) == 0 && neg) atomicOr(&S.negative, neg);
+            __syncthreads();
+            const int steps = j1 - j < MM_K ? (int)(j1 - j) : MM_K;
+            const unsigned negative = S.negative;
+            for (int t = 0; mine && t < steps; ++t) {
+                const U x[2] = {(U)S.as[2 * ty][t], (U)S.as[2 * ty + 1][t]};
+                if (x[0] == 0 && x[1] == 0) continue;
+                U y[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) y[c] = (U)S.bs[t][4 * tx + c];
+                if ((negative >> t) & 1u) {          // block-uniform
+#pragma unroll
+                    for (int r = 0; r < 2; ++r)
+#pragma unroll
+                        for (int c = 0; c < 4; ++c)
+                            acc[r][c] = min(acc[r][c], mm_enc<U>(avos_product<T>((T)x[r], (T)y[c], ev)));
+                    continue;
+                }
+                U z[2], yo = 0;                      // the left operands, the red one as 1; plain right ones ORed
+#pragma unroll
+                for (int r = 0; r < 2; ++r) z[r] = x[r] == RED ? (U)1 : x[r];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) yo |= (U)(y[c] + 1) <= 2 ? (U)0 : y[c];
+                const int mx[2] = {msb_nz<U>((U)(z[0] | 1)), msb_nz<U>((U)(z[1] | 1))};
+                // may a product of the thread's reach the top bit?
+                const bool top = max(mx[0], mx[1]) + msb_nz<U>((U)(yo | 1)) >= BITS - 1;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    if ((U)(y[c] + 1) <= 2) {        // 0 or an identity: 1 keeps an odd left value, -1 an even one
+                        if (y[c] == 0) continue;
+#pragma unroll
+                        for (int r = 0; r < 2; ++r)
+                            if (x[r] == RED ? y[c] == RED : x[r] != 0 && (x[r] & 1) == (U)(y[c] == 1))
+                                acc[r][c] = min(acc[r][c], mm_enc<U>(x[r]));
+                        continue;
+                    }
+                    const int s = msb_nz<U>(y[c]);
+                    const U low = (U)(y[c] ^ ((U)1 << s));
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) {
+                        if (z[r] == 0) continue;
+                        const U v = (U)((U)(z[r] << s) | low);
+                        if (top) {
+                            if (mx[r] + s >= BITS) ev |= RBG_EV_OVF_SIZE;
+                            if (v == RED) ev |= RBG_EV_OVF_ONES;
+                        }
+                        acc[r][c] = min(acc[r][c], top ? mm_enc<U>(v) : v);
+                    }
+                }
+            }
         }
-        __syncthreads();
-        for (int t = 0; t < MM_K; ++t) {
-            T a[4], b[8];
 #pragma unroll
-            for (int r = 0; r < 4; ++r) a[r] = as[4 * ty + r][t];
+        for (int r = 0; r < 2; ++r)
 #pragma unroll
-            for (int c = 0; c < 8; ++c) b[c] = bs[t][mm_col(tx, c)];
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int c = 0; c < 8; ++c) acc[r][c] = avos_sum<T>(acc[r][c], (T)avos_product<T>(a[r], b[c], ev));
-        }
+            for (int c = 0; c < 4; ++c)
+                tile[(MM_Q * (q >> 1) + 2 * ty + r) * MM_T + MM_Q * (q & 1) + 4 * tx + c] = acc[r][c];
     }
-    __syncthreads();
-    U *tile = reinterpret_cast<U *>(smem);
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int c = 0; c < 8; ++c) tile[(4 * ty + r) * MM_T + mm_col(tx, c)] = mm_enc<U>((U)acc[r][c]);
     mm_flush_flags(dflags, ev);
+}
+
+// Shared memory of a CTA: the lanes' staging buffers, over them the tile when it is shared by a cluster
+// or redone; the exact tile's staging buffers behind the tile.
+template <typename T> constexpr size_t mm_smem_bytes() {
+    return std::max(sizeof(MmSmem), sizeof(T) * MM_T * MM_T + sizeof(MmExact<T>));
 }
 
 // One 128 x 128 tile of C per cluster of `split` CTAs (1, 2, 4 or 8), each taking an equal part of
@@ -285,7 +350,8 @@ mm_kernel(int64_t m, int64_t q, int64_t p, const T *__restrict__ A, int64_t lda,
     auto dec = [](U e) -> T { return (T)mm_enc<U>(e); };   // the encoding is its own inverse
     auto lane_enc = [](uint32_t v) -> U { return (v >> 31) ? (U)~(U)0 : (U)v; };
     if (dirty) {
-        mm_exact_tile<T>(m, p, i0, k0, c0 * MM_K, c1 * MM_K < q ? c1 * MM_K : q, A, lda, B, ldb, mm_smem, dflags);
+        mm_exact_tile<T>(m, p, i0, k0, c0 * MM_K, c1 * MM_K < q ? c1 * MM_K : q, A, lda, B, ldb, tile,
+                         *reinterpret_cast<MmExact<T> *>(mm_smem + sizeof(T) * MM_T * MM_T), dflags);
     } else if (split > 1) {
         __syncthreads();                     // the last chunk's reads of the staging buffers
 #pragma unroll
@@ -339,7 +405,7 @@ static int matmul_t(int64_t m, int64_t q, int64_t p, const T *A, int64_t lda, co
         RBG_CUDA_TRY(cudaMemset2DAsync(C, ldc * sizeof(T), 0, p * sizeof(T), m, s));
         return RBG_OK;
     }
-    constexpr size_t smem = std::max(sizeof(MmSmem), sizeof(T) * MM_T * MM_T);
+    constexpr size_t smem = mm_smem_bytes<T>();
     static PerDeviceOnce once;               // per storage type, for every device
     const int configured = once.run([] {
         RBG_CUDA_TRY(cudaFuncSetAttribute(mm_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

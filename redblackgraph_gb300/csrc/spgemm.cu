@@ -132,7 +132,7 @@ struct SpArgs {
     int *big_rows; int *big_count;                      // rows for the block / dense kernels
     unsigned *flags;
     int2 *win;                                          // per row: first and last column it can reach
-    int *warp_rows; int *warp_count;                    // rows the group kernel leaves to the warp kernel
+    int *warp_rows; int *warp_count;                    // rows left to the warp kernel; [1]: taken by it
     unsigned char *tile_done;                           // squaring: blocks of rows the tile kernel has taken
 };
 
@@ -381,6 +381,7 @@ struct SpWinWarp {
 };
 constexpr size_t SP_WARP_BYTES = sizeof(SpHashWarp) > sizeof(SpWinWarp) ? sizeof(SpHashWarp) : sizeof(SpWinWarp);
 constexpr size_t SP_WARP_SMEM = SP_WARP_BYTES * SP_HWARPS;
+constexpr int SP_WARP_CTAS = 5;       // CTAs per SM (shared memory)
 
 // Slot of column j (inserted if new); -1 when the table is full.
 __device__ __forceinline__ int sp_hash_slot(SpHashWarp &H, unsigned j, int mask) {
@@ -893,9 +894,16 @@ sp_warp_kernel(SpArgs a, int merge) {
     SpHashWarp &H = *reinterpret_cast<SpHashWarp *>(sp_smem + (size_t)w * SP_WARP_BYTES);
     SpWinWarp &Wn = *reinterpret_cast<SpWinWarp *>(sp_smem + (size_t)w * SP_WARP_BYTES);
     unsigned ev = 0;
-    const int64_t warps = (int64_t)gridDim.x * SP_HWARPS;
     const int todo = *a.warp_count;
-    for (int64_t t = (int64_t)blockIdx.x * SP_HWARPS + w; t < todo; t += warps) {
+    // the rows are uneven, so a warp takes a few at a time (about eight times in all)
+    const int few = max(1, min(16, todo / (8 * (int)gridDim.x * SP_HWARPS)));
+    for (int t = 0, end = 0; todo > 0; ++t) {
+        if (t >= end) {
+            if (lane == 0) t = atomicAdd(a.warp_count + 1, few);
+            t = __shfl_sync(0xffffffffu, t, 0);
+            if (t >= todo) break;
+            end = min(t + few, todo);
+        }
         const int64_t i = a.warp_rows[t];            // at most SP_BLOCK_CAP candidates
         const int64_t c = a.cand_off[i + 1] - a.cand_off[i];
         const bool sq = merge && a.rp;
@@ -1221,7 +1229,7 @@ struct Head {   // workspace that lives from rbg_spgemm_count to rbg_spgemm_gath
     int64_t *cand_off;   // n+1
     int2 *win;           // n: each row's column window
     int *big_rows;       // n
-    int *counters;       // [0] big rows, [1] dense rows, [2] flags, [3] rows for the warp kernel
+    int *counters;       // [0] big rows, [1] dense rows, [2] flags, [3] rows for the warp kernel, [4] taken by it
     void *scan_tmp;
     size_t scan_bytes;
 };
@@ -1377,7 +1385,7 @@ int run_numeric(SpArgs &a, int merge, int64_t dense, int64_t nc, cudaStream_t s)
         else sp_group_kernel<UNS, 4, false><<<gg, SP_GWARPS * 32, 0, s>>>(a, merge);
     }
     // the rows left over, usually none: one wave of CTAs
-    const int wg = (int)std::min<int64_t>((n + SP_HWARPS - 1) / SP_HWARPS, 4 * sm_count());
+    const int wg = (int)std::min<int64_t>((n + SP_HWARPS - 1) / SP_HWARPS, SP_WARP_CTAS * sm_count());
     if (a.elem_bytes == 8) sp_warp_kernel<SEM, UNS, 8><<<wg, SP_HWARPS * 32, SP_WARP_SMEM, s>>>(a, merge);
     else sp_warp_kernel<SEM, UNS, 4><<<wg, SP_HWARPS * 32, SP_WARP_SMEM, s>>>(a, merge);
     sp_block_kernel<SEM, UNS><<<2 * sm_count(), SP_BLOCK_THREADS, SP_BLOCK_SMEM, s>>>(a, merge);
@@ -1423,7 +1431,7 @@ extern "C" int32_t rbg_spgemm_numeric(int32_t sem, int32_t dtype, const rbg_csr_
     a.warp_rows = t.warp_rows;
     a.tile_done = t.tile_done;
     a.warp_count = h.counters + 3;
-    RBG_CUDA_TRY(cudaMemsetAsync(h.counters + 2, 0, 8, s));
+    RBG_CUDA_TRY(cudaMemsetAsync(h.counters + 2, 0, 12, s));
     RBG_CUDA_TRY(cudaMemsetAsync(t.rownnz, 0, (size_t)(n + 1) * 8, s));
     const int merge = R != nullptr;
     int rc;

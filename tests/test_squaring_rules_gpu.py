@@ -114,3 +114,23 @@ def test_columns_in_any_order(native, dtype, n, family):
         A = _csr(other, n, dtype)
         got = spgemm(A, A, R=A)
         assert got[1:] == want[1:] and _cells(got[0].to_scipy()) == _cells(want[0].to_scipy())
+
+
+@pytest.mark.parametrize("n", [1, 8, 5000, 130_003])
+def test_rows_left_to_the_warps(native, n):
+    """Values past 32 bits in every row: all rows go to the warp kernel, several at a time when many."""
+    from redblackgraph_gb300.spgemm import DeviceCSR, spgemm
+    rng = np.random.default_rng(n)
+    i = np.arange(n)
+    r = np.repeat(i, 2)
+    c = np.maximum(r - rng.integers(0, 40, r.size), 0)
+    k = np.unique(r * n + c)
+    A = sp.csr_matrix((rng.integers(2, 5, k.size), (k // n, k % n)), shape=(n, n))
+    big = A.copy()
+    big.data = big.data + (1 << 33)
+    S, fl = O.rb_matmul_csr(big, A)
+    S.sort_indices()
+    C, rc, _ = spgemm(DeviceCSR.from_scipy(big), DeviceCSR.from_scipy(A))
+    got = C.to_scipy()
+    assert not fl & 7 and rc == 0 and (got.indptr == S.indptr).all()
+    assert (got.indices == S.indices).all() and (got.data == S.data).all()

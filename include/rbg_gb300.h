@@ -494,7 +494,8 @@ int32_t rbg_cc_compact_fill(int64_t n, const int32_t *label, const int32_t *loca
  * ---------------------------------------------------------------------------------------- */
 
 /* comp_flags[c] (device, ncomp): bit 0 outside the clean regime, bit 1 an entry below the
- * diagonal, bit 2 an entry above it; diag (device, n): each row's diagonal value (0 when not
+ * diagonal, bit 2 an entry above it, bit 3 a row of more than 16 off-diagonal entries or vertices 8192
+ * or more apart (rbg_cc_dag_close does not take such a graph); diag (device, n): each row's diagonal value (0 when not
  * stored); edge_ptr (device, n + 1): row pointers of the off-diagonal nonzeros, *edges (host)
  * their number.  sorted_vertex and start (ncomp + 1 entries, start[ncomp] = n) as rbg_cc_label
  * writes them; a graph of n > 0 vertices without components is RBG_ERR_INVALID.  Synchronises
@@ -534,6 +535,11 @@ int32_t rbg_cc_dag_close(int64_t n, int64_t ncomp, const int32_t *label, const i
                          int32_t *pool_cols, int32_t *pool_vals, int64_t pool_capacity, int64_t *row_off,
                          int32_t *row_len, int32_t *top_msb, int32_t *first_msb, int32_t *comp_max,
                          int32_t *closed, rbg_stream_t stream);
+
+/* After rbg_cc_dag_close left *closed = 0 in `workspace`: *entries (host) = the pool entries its rows asked
+ * for when the pool was all that was too small (rows behind one without room ask for less than they will
+ * need: call again with half as many more at least), 0 otherwise.  Synchronises `stream`. */
+int32_t rbg_cc_dag_close_reserved(const void *workspace, int64_t *entries, rbg_stream_t stream);
 
 /* Row pointers (device, n + 1) of the merged matrix: each closure row (row_len from the row
  * pool) plus its diagonal value when nonzero; *nnz (host) its size.  Synchronises `stream`. */

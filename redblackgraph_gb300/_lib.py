@@ -146,6 +146,7 @@ SIGNATURES = [
     ("rbg_cc_dag_close_workspace_bytes", _I32, [_I64, ctypes.POINTER(_I64)]),
     ("rbg_cc_dag_close", _I32, [_I64, _I64, _P, _P, _P, _P, _P, ctypes.POINTER(RbgCsr), _P, _P, _I64, _P, _P, _I64, _P, _P,
                                 _P, _P, _P, ctypes.POINTER(_I32), _P]),
+    ("rbg_cc_dag_close_reserved", _I32, [_P, ctypes.POINTER(_I64), _P]),
     ("rbg_cc_dag_merge_count", _I32, [_I64, _P, _P, _P, _I64, _P, ctypes.POINTER(_I64), _P]),
     ("rbg_cc_dag_merge_fill", _I32, [_I64, _P, _P, _P, _P, _P, _P, _P, _P, _P]),
     ("rbg_cc_compact_fill", _I32, [_I64, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P]),

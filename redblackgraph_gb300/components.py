@@ -147,13 +147,16 @@ def _msb(v: int) -> int:
 
 DAG_MAX_N = 8192          # rows of a component the DAG path takes (include/rbg_gb300.h)
 DAG_TILE_ROWS = 64        # vertices of a piece closed without levels (rbg_dag_closure_mode)
-_UNCLEAN, _BELOW, _ABOVE = 1, 2, 4
+_UNCLEAN, _BELOW, _ABOVE, _LARGE = 1, 2, 4, 8
 
 
-def _close_rows(E, comps: Components, kind, diag, top, first, cmax, sh):
+def _close_rows(E, comps: Components, kind, diag, top, first, cmax, large, short, sh):
     """The closure rows of the edges ``E`` as DagRows and the components' statistics (rbg_cc_dag_close), or
-    None when the graph is not for that path."""
+    None when the graph is not for that path: ``large`` (known before), or long rows, when the size of
+    a pool to go on with is added to ``short``."""
     from .dag import DagRows
+    if large:
+        return None
     n, dev = comps.n, E.indptr.device
     L = _lib.load()
     nb = ctypes.c_int64(0)
@@ -162,16 +165,30 @@ def _close_rows(E, comps: Components, kind, diag, top, first, cmax, sh):
     row_off = torch.empty(n, dtype=torch.int64, device=dev)
     row_len = torch.empty(n, dtype=torch.int32, device=dev)
     cap = max(16 * E.nnz + n, 1024)
-    cols = torch.empty(cap, dtype=torch.int32, device=dev)
-    vals = torch.empty(cap, dtype=torch.int32, device=dev)
-    closed = ctypes.c_int32(0)
+    closed, reserved = ctypes.c_int32(0), ctypes.c_int64(0)
     ec = E.cstruct()
-    _lib.check(L.rbg_cc_dag_close(n, comps.count, comps.label.data_ptr(), comps.local.data_ptr(), comps.start.data_ptr(),
-                                  comps.sorted_vertex.data_ptr(), kind.data_ptr(), ctypes.byref(ec), diag.data_ptr(),
-                                  ws.data_ptr(), ws.numel(), cols.data_ptr(), vals.data_ptr(), cap, row_off.data_ptr(),
-                                  row_len.data_ptr(), top.data_ptr(), first.data_ptr(), cmax.data_ptr(),
-                                  ctypes.byref(closed), sh), "cc_dag_close")
-    return DagRows(cols, vals, row_off, row_len, -1) if closed.value else None
+    while True:
+        cols = torch.empty(cap, dtype=torch.int32, device=dev)
+        vals = torch.empty(cap, dtype=torch.int32, device=dev)
+        _lib.check(L.rbg_cc_dag_close(n, comps.count, comps.label.data_ptr(), comps.local.data_ptr(),
+                                      comps.start.data_ptr(), comps.sorted_vertex.data_ptr(), kind.data_ptr(),
+                                      ctypes.byref(ec), diag.data_ptr(), ws.data_ptr(), ws.numel(), cols.data_ptr(),
+                                      vals.data_ptr(), cap, row_off.data_ptr(), row_len.data_ptr(), top.data_ptr(),
+                                      first.data_ptr(), cmax.data_ptr(), ctypes.byref(closed), sh), "cc_dag_close")
+        if closed.value:
+            return DagRows(cols, vals, row_off, row_len, -1)
+        _lib.check(L.rbg_cc_dag_close_reserved(ws.data_ptr(), ctypes.byref(reserved), sh), "cc_dag_close")
+        # a pool that nearly sufficed: again with twice as much (once: rows behind one without room ask for
+        # less than they need).  Otherwise the rows are long and the closure by levels is as good; it
+        # reserves the same entries and need not try this pool again
+        if reserved.value == 0:
+            return None
+        near = 4 * reserved.value <= 5 * cap and not short
+        short.append(max(2 * cap, reserved.value + reserved.value // 2))
+        if not near:
+            return None
+        cap = short[0]
+        del cols, vals
 
 
 def dag_component_closure(indptr: torch.Tensor, indices: torch.Tensor, data: torch.Tensor, n: int,
@@ -218,11 +235,14 @@ def dag_component_closure(indptr: torch.Tensor, indices: torch.Tensor, data: tor
     # wait for their parents beat levels (1024 pedigrees of up to 4096 vertices: 0.99 to 0.78 ms
     # with the statistics)
     tiles = 2 * int(comps.sizes[comps.sizes <= DAG_TILE_ROWS].sum()) >= n
-    C = None if tiles else _close_rows(E, comps, kind, diag, top, first, cmax, sh)
+    large = bool(((f & _LARGE) != 0).any())
+    short = []
+    C = None if tiles else _close_rows(E, comps, kind, diag, top, first, cmax, large, short, sh)
     closed = C is not None
     if not closed:
         try:
-            C, _, _ = dag_closure_device(E, stream, gather=False, tiles=tiles)    # the row pool, read in place
+            factor = -(-max(short) // max(E.nnz, 1)) if short else 16
+            C, _, _ = dag_closure_device(E, stream, factor, gather=False, tiles=tiles)    # the row pool, read in place
         except RowTooWide:
             return None
     pool = (C.row_off.data_ptr(), C.row_len.data_ptr(), C.cols.data_ptr(), C.vals.data_ptr())

@@ -434,6 +434,9 @@ extern "C" int32_t rbg_cc_compact_fill(int64_t n, const int32_t *label, const in
 namespace rbg {
 
 constexpr unsigned CCD_UNCLEAN = 1u, CCD_BELOW = 2u, CCD_ABOVE = 4u;
+constexpr unsigned CCD_LARGE = 8u;               // a row or a span that rbg_cc_dag_close does not take
+constexpr int64_t CCD_ROW = 16;                  // (TRI_CAP and TRI_MAX_N of fw_tri.cu)
+constexpr int64_t CCD_SPAN = DAG_MAX_N;
 constexpr int CCD_WARPS = 8;
 
 // one thread per vertex, in the order of the components (position r of sorted_vertex): its row's
@@ -480,6 +483,7 @@ __global__ void __launch_bounds__(256) cc_dag_classify_kernel(int64_t n, int64_t
                     ++k;
                 }
             }
+            if (k > CCD_ROW || u - sorted_vertex[start[c]] >= CCD_SPAN) f |= CCD_LARGE;
             diag[u] = d;
             cnt[u] = k;
         }

@@ -1700,5 +1700,17 @@ extern "C" int32_t rbg_cc_dag_close(int64_t n, int64_t ncomp, const int32_t *lab
     return RBG_OK;
 }
 
+extern "C" int32_t rbg_cc_dag_close_reserved(const void *workspace, int64_t *entries, rbg_stream_t stream) {
+    using namespace rbg;
+    if (!workspace || !entries) return RBG_ERR_INVALID;
+    DagCounters hd;                              // (the workspace starts with them)
+    HostStaging hs(reinterpret_cast<cudaStream_t>(stream), sizeof(hd) + 128);
+    int rc = hs.down(&hd, workspace, sizeof(hd));
+    if (!rc) rc = hs.finish();
+    if (rc) return rc;
+    *entries = hd.flags == 1 ? (int64_t)hd.reserved : 0;
+    return RBG_OK;
+}
+
 // The DAG path keeps nothing between calls.
 extern "C" int32_t rbg_release_scratch(void) { return RBG_OK; }

@@ -952,15 +952,10 @@ __device__ __forceinline__ bool dag_tile(const DagArgs &a, DagTile &S, int64_t p
     return true;
 }
 
-// One warp per DT_ROWS positions: the pieces that start there.  reach[p]: the furthest end of any
-// edge that starts at or before p, so a piece starts at p when reach[p - 1] < p.
-__global__ void __launch_bounds__(DT_WARPS * 32)
-dag_tile_kernel(DagArgs a, const int *reach, int *tile_rows, int *tile_levels) {
-    extern __shared__ __align__(16) unsigned char dg_smem[];
-    DagTile &S = reinterpret_cast<DagTile *>(dg_smem)[threadIdx.x >> 5];
-    const int lane = threadIdx.x & 31;
-    const int64_t b = ((int64_t)blockIdx.x * DT_WARPS + (threadIdx.x >> 5)) * DT_ROWS;
-    if (b >= a.n) return;
+// The tiles that start at the DT_ROWS positions from b on, in turn: tile(start, length).  reach[p]: the
+// furthest end of any edge that starts at or before p, so a piece starts at p when reach[p - 1] < p.
+template <typename F>
+__device__ __forceinline__ void dag_tiles_at(const DagArgs &a, const int *reach, int64_t b, int lane, F &&tile) {
     auto starts = [&](int64_t first) -> unsigned long long {
         unsigned long long f = 0;
 #pragma unroll
@@ -972,8 +967,6 @@ dag_tile_kernel(DagArgs a, const int *reach, int *tile_rows, int *tile_levels) {
         return f;
     };
     const unsigned long long f0 = starts(b), f1 = starts(b + DT_ROWS);   // pieces end at the next start, or at n
-    int best = 0, levels = 0, rows = 0;
-    unsigned long long written = 0;
     int cur = 0;
     while (cur < DT_ROWS) {                      // warp-uniform
         const unsigned long long rest = f0 & (~0ull << cur);
@@ -988,9 +981,44 @@ dag_tile_kernel(DagArgs a, const int *reach, int *tile_rows, int *tile_levels) {
             continue;
         }
         const int len = 64 - __clzll((long long)ends);   // the furthest of them
-        if (dag_tile(a, S, b + s, len, lane, best, written, levels)) rows += len;
+        tile(b + s, len);
         cur = s + len;
     }
+}
+
+// How many of the rows at `looked` evenly spread chunks of positions a tile could hold, a warp per
+// chunk.  A tile takes its warp about 45 us, so a few of them cost more than the levels that the other
+// rows take anyway: fewer than half of the rows, and the tiles are left out (families of 65, 300,000
+// vertices: 1.08 ms by levels, 1.15 with the tiles of a few odd families, 1.10 so).
+constexpr int DT_LOOK = 512;
+__global__ void __launch_bounds__(256)
+dag_look_kernel(DagArgs a, const int *reach, int64_t chunks, int looked, int *room) {
+    const int lane = threadIdx.x & 31;
+    const int64_t w = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    __shared__ int s_rows;
+    if (threadIdx.x == 0) s_rows = 0;
+    __syncthreads();
+    int rows = 0;
+    if (w < looked) dag_tiles_at(a, reach, w * chunks / looked * DT_ROWS, lane, [&](int64_t, int len) { rows += len; });
+    if (lane == 0 && rows) atomicAdd(&s_rows, rows);
+    __syncthreads();
+    if (threadIdx.x == 0 && s_rows) atomicAdd(room, s_rows);
+}
+
+// One warp per DT_ROWS positions: the tiles that start there, if dag_look_kernel found at least `least` rows.
+__global__ void __launch_bounds__(DT_WARPS * 32)
+dag_tile_kernel(DagArgs a, const int *reach, const int *room, int least, int *tile_rows, int *tile_levels) {
+    extern __shared__ __align__(16) unsigned char dg_smem[];
+    DagTile &S = reinterpret_cast<DagTile *>(dg_smem)[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const int64_t b = ((int64_t)blockIdx.x * DT_WARPS + (threadIdx.x >> 5)) * DT_ROWS;
+    if (b >= a.n) return;
+    const bool on = __ldg(room) >= least;        // (asked for below, with the positions on their way)
+    int best = 0, levels = 0, rows = 0;
+    unsigned long long written = 0;
+    dag_tiles_at(a, reach, b, lane, [&](int64_t p, int len) {
+        if (on && dag_tile(a, S, p, len, lane, best, written, levels)) rows += len;
+    });
     best = __reduce_max_sync(FULL, best);
     if (lane == 0) {
         if (best > 0) atomicMax(a.max_abs, (unsigned long long)best);
@@ -1253,13 +1281,16 @@ extern "C" int32_t rbg_dag_closure_mode(const rbg_csr_t *A, uint32_t mode, void 
     RBG_CUDA_TRY(cudaMemsetAsync(row_len, 0xff, (size_t)n * 4, s));
     if (!(mode & RBG_DAG_NO_TILES)) {
         RBG_CUDA_TRY(cudaMemsetAsync(w.ccount, 0xff, (size_t)n * 4, s));
-        note_launches(3);
+        note_launches(4);
         dag_span_kernel<<<grid_for(n, 256), 256, 0, s>>>(n, a.ap, a.aj, w.ccount);
         size_t tb = w.tmp_bytes;
         RBG_CUDA_TRY(cub::DeviceScan::InclusiveScan(w.tmp, tb, w.ccount, w.cursor, IntMax(), (int)n, s));
         const int64_t tiles = (n + DT_ROWS - 1) / DT_ROWS;
+        const int looked = (int)std::min<int64_t>(tiles, DT_LOOK);
+        const int least = (int)(std::min<int64_t>(n, (int64_t)looked * DT_ROWS) / 2);
+        dag_look_kernel<<<(unsigned)((looked + 7) / 8), 256, 0, s>>>(a, w.cursor, tiles, looked, &w.cnt->tile_room);
         dag_tile_kernel<<<(unsigned)((tiles + DT_WARPS - 1) / DT_WARPS), DT_WARPS * 32, sizeof(DagTile) * DT_WARPS, s>>>(
-            a, w.cursor, &w.cnt->tile_rows, &w.cnt->tile_levels);
+            a, w.cursor, &w.cnt->tile_room, least, &w.cnt->tile_rows, &w.cnt->tile_levels);
         RBG_CUDA_TRY(cudaGetLastError());
     }
     int64_t annz = 0;

@@ -145,6 +145,7 @@ struct DagCounters {
     int placed, nwide, flags, nlevels;       // flags: 1 pool too small, 2 row past the block table
     unsigned long long reserved, max_abs, total;
     int tile_rows, tile_levels;              // rows closed without levels, and their deepest level + 1
+    int tile_room;                           // rows of the looked-at positions that a tile could hold
 };
 
 // fw_tri.cu: the components of an int32 or int64 batch that are acyclic and in the clean regime

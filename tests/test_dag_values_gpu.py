@@ -61,3 +61,28 @@ def test_diagonal_stored_twice(native):
     for a, b in ((got[0].indptr, want[0].indptr), (got[0].indices, want[0].indices), (got[0].data, want[0].data)):
         assert (to_host(a) == to_host(b)).all()
     assert want[0].to_scipy().diagonal().tolist() == [min(twice[i % 7], default=0) for i in range(64)]
+
+
+@pytest.mark.parametrize("sizes", [[1], [40], [65] * 4, [64] * 3 + [100] * 2, [100] * 5 + [20],
+                                   [64] * 400 + [70] * 300, [64] * 300 + [70] * 400, [3, 90] * 500])
+def test_pieces_in_any_share(native, sizes):
+    """Pieces a tile holds and larger ones, about half of the rows each, past the positions looked at: with
+    the tiles or without, the same closure."""
+    from redblackgraph_gb300.dag import dag_closure_device
+    from redblackgraph_gb300.device import to_host
+    from redblackgraph_gb300.spgemm import DeviceCSR
+    rng = np.random.default_rng(len(sizes))
+    first = np.repeat(np.concatenate([[0], np.cumsum(sizes)[:-1]]), sizes)
+    n = first.size
+    i = np.arange(n)
+    parent = np.where(i > first, np.maximum(i - rng.integers(1, 12, n), first), -1)
+    other = np.where(i > first + 1, first + 1, -1)
+    r, c = np.concatenate([i, i, i]), np.concatenate([i, parent, other])
+    key = np.unique((r * n + c)[(c >= 0)])
+    r, c = key // n, key % n
+    v = np.where(r == c, rng.choice([-1, 1], key.size), rng.integers(2, 4, key.size)).astype(np.int32)
+    A = DeviceCSR.from_scipy(sp.csr_matrix((v, (r, c)), shape=(n, n)))
+    got, want = dag_closure_device(A), dag_closure_device(A, tiles=False)
+    assert got[1:] == want[1:]
+    for a, b in ((got[0].indptr, want[0].indptr), (got[0].indices, want[0].indices), (got[0].data, want[0].data)):
+        assert (to_host(a) == to_host(b)).all()

@@ -122,11 +122,12 @@ def lookup_many(queries, stream=None) -> list[Relationship]:
         which.append(k)
         us.append(u)
         vs.append(v)
-    table = np.array(mats, dtype=_LOOKUP_DTYPE)[which]
+    table = np.array(mats, dtype=_LOOKUP_DTYPE)
+    if len(mats) < len(which):           # else every query has a matrix of its own, in order
+        table, dts = table[which], [dts[k] for k in which]
     table["u"] = us
     table["v"] = vs
-    return decode(lookup_table(to_device(table.view(np.uint8), dev), len(queries), stream),
-                  [dts[k] for k in which])
+    return decode(lookup_table(to_device(table.view(np.uint8), dev), len(queries), stream), dts)
 
 
 def calculate_relationship(a: Sequence[int], b: Sequence[int]) -> Relationship:

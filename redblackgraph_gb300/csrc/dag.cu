@@ -822,18 +822,21 @@ struct DagTile {
     signed char diag[DT_ROWS];               // the stored diagonal, 0 if none
 };
 
-// furthest[p]: the largest end of the edges (and vertices) whose lower end is p
+// furthest[p]: the largest end of the edges (and vertices) whose lower end is p.  A row that stores its
+// diagonal twice (whose (+) the tiles do not take) reaches past the last vertex: no tile holds it, nor
+// any row behind it.
 __global__ void dag_span_kernel(int64_t n, const int64_t *ap, const int *aj, int *furthest) {
     for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
-        int lo = (int)v, hi = (int)v;
+        int lo = (int)v, hi = (int)v, diag = 0;
         for (int64_t e = ap[v]; e < ap[v + 1]; ++e) {
             const int w = aj[e];
+            diag += w == v;
             if (w >= 0 && w < n) {
                 lo = min(lo, w);
                 hi = max(hi, w);
             }
         }
-        atomicMax(furthest + lo, hi);
+        atomicMax(furthest + lo, diag > 1 ? (int)n : hi);
     }
 }
 
@@ -870,12 +873,12 @@ __device__ __forceinline__ bool dag_tile(const DagArgs &a, DagTile &S, int64_t p
         const int r = flip ? len - 1 - l : l;
         const int q1 = S.ptr[r + 1];
         unsigned x0 = DT_NONE, x1 = DT_NONE;
-        int dg = 2, lev = 0;                                 // dg: 2 while there is no diagonal entry
+        int dg = 0, lev = 0;
         for (int q = S.ptr[r]; q < q1; ++q) {                // warp-uniform
             const int v = S.val[q], c = flip ? len - 1 - S.col[q] : S.col[q];
             most = max(most, v < 0 ? 1 : v);
             if (c == l) {
-                dg = min(dg, v);                             // (stored twice: the (+) of the two)
+                dg = v;
                 continue;
             }
             lev = max(lev, S.level[c] + 1);
@@ -898,7 +901,6 @@ __device__ __forceinline__ bool dag_tile(const DagArgs &a, DagTile &S, int64_t p
         }
         const int base = l * (l - 1) / 2;
         const bool h0 = x0 != DT_NONE, h1 = x1 != DT_NONE;
-        dg = dg == 2 ? 0 : dg;
         if (lane < l) S.cell[base + lane] = h0 ? (int)x0 : 0;
         if (lane + 32 < l) S.cell[base + lane + 32] = h1 ? (int)x1 : 0;
         const int m = __popc(__ballot_sync(FULL, h0)) + __popc(__ballot_sync(FULL, h1)) + (dg != 0);

@@ -593,11 +593,12 @@ def dense_layered_dag(n, layers, p, seed, dtype=np.int32):
 
 
 def run_dense_blocked(n=4096, layers=24, p=0.5, seed=5, steps=5):
-    """The blocked Floyd-Warshall kernels on the workload they exist for: one dense layered DAG
-    (n=4096, int32; every row has hundreds of entries, so the DAG path declines it), whose
-    closure is dense, so nearly every tile item runs all 64 steps of its round.  ALU roofline on
-    the executed relaxations; a 1024-vertex instance of the same generator is checked bit-exact
-    against the oracle's sequential loop."""
+    """One dense layered DAG (n=4096, int32; every row has hundreds of entries, so the DAG path
+    declines it), numbered in a topological order: the one-sided closure's block steps.  ALU roofline
+    of sd_step_kernel on the relaxations of the steps with an entry on both sides (those that a warp
+    then skips included), at the two int32 operations a relaxation takes in the lane encoding
+    (multiply-add and min); a 1024-vertex instance of the same generator is checked bit-exact against
+    the oracle's sequential loop."""
     import torch
     from oracle import oracle as orc
     from redblackgraph_gb300 import _lib
@@ -623,10 +624,13 @@ def run_dense_blocked(n=4096, layers=24, p=0.5, seed=5, steps=5):
     e1.record(stream)
     torch.cuda.synchronize()
     t = e0.elapsed_time(e1) / 1e3 / steps
-    kp = {k: v for k, v in profile_kernels(lambda: fw_dense(d, out=out)).items() if v[1]}
-    phase_ms = sum(kp[k][0] for k in ("fw_tile_kernel", "fw_panel_kernel", "fw_diag_kernel") if k in kp)
+    # the timer slots of the blocked kernels' three phases
+    sided = {"fw_tile_kernel": "sd_step_kernel", "fw_panel_kernel": "sd_mask_kernel + sd_first_kernel",
+             "fw_diag_kernel": "sd_diag_kernel"}
+    kp = {sided.get(k, k): v for k, v in profile_kernels(lambda: fw_dense(d, out=out)).items() if v[1]}
+    step_ms = kp["sd_step_kernel"][0] if "sd_step_kernel" in kp else 0.0
     peak, sms = int32_peak_ops(0, None)
-    alu = res.executed * OPS_PER_RELAXATION / (phase_ms / 1e3) / 1e12 if phase_ms else None
+    alu = res.executed * 2 / (step_ms / 1e3) / 1e12 if step_ms else None
     nnz_out = int(np.count_nonzero(to_host(out)))
     return {"workload": f"one dense layered DAG, n={n}, {layers} layers, link probability {p}, int32 "
                         f"({int(np.count_nonzero(A)) / n:.0f} entries per row, {nnz_out / n / n:.0%} of the "
@@ -635,8 +639,8 @@ def run_dense_blocked(n=4096, layers=24, p=0.5, seed=5, steps=5):
             "diameter": int(res.diameter), "executed_relaxations": int(res.executed),
             "roofline": {"bound": "int32_alu", "unit": "Tops/s", "achieved": alu, "peak": peak / 1e12,
                          "frac": alu / (peak / 1e12) if alu else None,
-                         "kernel": "fw_diag_kernel + fw_panel_kernel + fw_tile_kernel",
-                         "ops_per_relaxation": OPS_PER_RELAXATION,
+                         "kernel": "sd_step_kernel",
+                         "ops_per_relaxation": 2,
                          "peak_source": f"nominal: {sms} SMs x 128 int32 lanes x max SM clock"},
             "kernel_ms": {k: v[0] for k, v in kp.items()},
             "bit_exact_vs_oracle_n1024": exact}

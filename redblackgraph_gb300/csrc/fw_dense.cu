@@ -1346,7 +1346,7 @@ static int fw_dense_t(int64_t n, const T *in, int64_t ld_in, T *out, int64_t ld_
         if (try_dag && dag_path_allowed(mode)) {
             const int64_t zero = 0;
             char closed = TRI_OPEN;
-            const int rc = tri_batch<T>(1, &n, &zero, &zero, ld_in, ld_out, in, out, res, &closed, ws, ws_bytes, mode,
+            const int rc = tri_batch<T>(1, &n, &zero, &zero, ld_in, ld_out, in, out, res, &closed, ws, ws_bytes,
                                         stream, RowStats());
             if (rc) return rc;
             if (closed == TRI_CLOSED) return RBG_OK;
@@ -1577,7 +1577,7 @@ static int fw_batch_t(int64_t count, const int64_t *sizes, const int64_t *offset
     if constexpr (std::is_same<T, int32_t>::value || std::is_same<T, int64_t>::value) {
         if (dag_path_allowed(mode)) {
             const int rc = tri_batch<T>(count, sizes, offsets, offsets, 0, 0, in, out, results, closed.data(), ws,
-                                        ws_bytes, mode, stream, rs);
+                                        ws_bytes, stream, rs);
             if (rc) return rc;
         }
     }

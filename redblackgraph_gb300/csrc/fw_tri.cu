@@ -13,7 +13,8 @@
 //
 // In the clean regime (off-diagonal values 0 or >= 2, diagonal in {-1, 0, 1}) products with the
 // diagonal change nothing and a cell only decreases once it holds a value, so the largest value
-// the loop ever writes -- the diameter's source -- is, per cell, its first value: A(i, j), else
+// the loop ever writes -- the diameter's source -- is, per cell, its first value: A(i, j) (or step 0's
+// product where that is less, as the loop looks at a value after the step: tri_gen_init_kernel), else
 // the product of the first step that reaches the cell.  Below the diagonal that is the smallest
 // parent k of i with j in C(k); above it, the smallest k in C(i) with j a parent of k.  A
 // product whose most significant bit may reach bit 31 sends the matrix to the blocked kernels
@@ -1389,7 +1390,6 @@ template <typename T> struct TriCall {
     T *out;
     unsigned char *ws;
     size_t ws_bytes;
-    uint32_t mode;
     cudaStream_t s;
     const RowStats &rs;
     TriShape sh;
@@ -1557,13 +1557,13 @@ int64_t tri_take_results(const TriCall<T> &c, bool pending, rbg_result_t *result
 template <typename T>
 int tri_batch(int64_t count, const int64_t *sizes, const int64_t *in_off, const int64_t *out_off, int64_t ld_in,
               int64_t ld_out, const T *in, T *out, rbg_result_t *results, char *closed, unsigned char *ws,
-              size_t ws_bytes, uint32_t mode, cudaStream_t s, const RowStats &rs) {
+              size_t ws_bytes, cudaStream_t s, const RowStats &rs) {
     if (count <= 0 || count > INT32_MAX || !ws) return RBG_OK;
     {
         const int rc = tri_configure();     // before any capture: kernel attributes per device
         if (rc) return rc;
     }
-    TriCall<T> c{count, sizes, in_off, out_off, ld_in, ld_out, in, out, ws, ws_bytes, mode, s, rs};
+    TriCall<T> c{count, sizes, in_off, out_off, ld_in, ld_out, in, out, ws, ws_bytes, s, rs};
     if (!c.shape()) return RBG_OK;
     int rc = tri_pass(c, false);
     if (rc) return rc;
@@ -1574,10 +1574,10 @@ int tri_batch(int64_t count, const int64_t *sizes, const int64_t *in_off, const 
 }
 
 template int tri_batch<int32_t>(int64_t, const int64_t *, const int64_t *, const int64_t *, int64_t, int64_t,
-                                const int32_t *, int32_t *, rbg_result_t *, char *, unsigned char *, size_t, uint32_t,
+                                const int32_t *, int32_t *, rbg_result_t *, char *, unsigned char *, size_t,
                                 cudaStream_t, const RowStats &);
 template int tri_batch<int64_t>(int64_t, const int64_t *, const int64_t *, const int64_t *, int64_t, int64_t,
-                                const int64_t *, int64_t *, rbg_result_t *, char *, unsigned char *, size_t, uint32_t,
+                                const int64_t *, int64_t *, rbg_result_t *, char *, unsigned char *, size_t,
                                 cudaStream_t, const RowStats &);
 
 }  // namespace rbg

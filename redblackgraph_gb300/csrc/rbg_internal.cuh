@@ -114,9 +114,9 @@ void launch_recording(bool on);
 
 // Benchmark timer (rbg_profile_begin / rbg_profile_end_slots): CUDA events around the kernels
 // of each slot, recorded on the launching stream while the timer is on.  Slots: 0 phase-3
-// tiles, 1 panels, 2 diagonal tiles, 3 convert + finalize, 4 DAG path scan, 5 DAG path
-// closure by levels (with its CSR), 6 DAG path statistics, 7 DAG path write, 8 DAG path
-// searches of matrices in any numbering.
+// tiles (one-sided closure: block steps), 1 panels (one-sided: masks and first values), 2 diagonal
+// tiles, 3 convert + finalize, 4 DAG path scan, 5 DAG path closure rows with their statistics,
+// 6 nothing, 7 DAG path write, 8 DAG path searches of matrices in any numbering.
 constexpr int TIMER_SLOTS = 9;
 cudaEvent_t timer_begin(int slot, cudaStream_t s);
 void timer_end(int slot, cudaEvent_t start, cudaStream_t s);
@@ -142,7 +142,9 @@ struct RowStats {
 
 // The device counters of a closure by rows (dag.cu; fw_tri.cu uses reserved and flags).
 struct DagCounters {
-    int placed, nwide, flags, nlevels;       // flags: 1 pool too small, 2 row past the block table
+    // flags: 1 pool too small; dag.cu: 2 row past the block table; fw_tri.cu: 4 an inconsistent closure
+    // row, or a graph that is not for the path, 8 a bounded wait ran out
+    int placed, nwide, flags, nlevels;
     unsigned long long reserved, max_abs, total;
     int tile_rows, tile_levels;              // rows closed without levels, and their deepest level + 1
     int tile_room;                           // rows of the looked-at positions that a tile could hold
@@ -164,7 +166,7 @@ constexpr char TRI_OPEN = 0, TRI_CLOSED = 1, TRI_TOP_BIT = 2, TRI_WIDE_BELOW = 4
 template <typename T>
 int tri_batch(int64_t count, const int64_t *sizes, const int64_t *in_off, const int64_t *out_off, int64_t ld_in,
               int64_t ld_out, const T *in, T *out, rbg_result_t *results, char *closed, unsigned char *ws,
-              size_t ws_bytes, uint32_t mode, cudaStream_t stream, const RowStats &rs);
+              size_t ws_bytes, cudaStream_t stream, const RowStats &rs);
 
 template <typename T> struct dtype_of;
 template <> struct dtype_of<int8_t> { static const int value = RBG_DTYPE_INT8; };

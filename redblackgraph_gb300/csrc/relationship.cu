@@ -10,8 +10,7 @@
 // closures, 7 us now), keep the smallest (sum, j) and meet in a shuffle and shared-memory
 // reduction: the smallest sum, ties to the smallest j.  The sum wraps in the matrix's own type, as
 // numpy scalar arithmetic does on the reference's rows (for unsigned types the red one, the type's
-// maximum, plus y gives y - 1).  Types of up to 4 bytes pack (sum in the type's order, j) into one
-// 64-bit key; 8-byte types carry the two words.
+// maximum, plus y gives y - 1).  Every type carries two words, the sum in the type's order and j.
 #include <cuda_runtime.h>
 #include <type_traits>
 #include "rbg_internal.cuh"
